@@ -37,6 +37,11 @@ int hq_query_device(hq_device_info* info);
 int hq_dgemm(cudaStream_t stream, const hq_device_info* dev, char transa, char transb, int M,
              int N, int K, double alpha, const double* A, int lda, const double* B, int ldb,
              double beta, double* Cm, int ldc, double* ws, size_t ws_elems);
+/* The same; upper != 0 forms only the 16 x 16 parts of C that reach its upper
+ * triangle (a Gram matrix whose lower triangle nobody reads). */
+int hq_dgemm_part(cudaStream_t stream, const hq_device_info* dev, char transa, char transb, int M,
+                  int N, int K, double alpha, const double* A, int lda, const double* B, int ldb,
+                  double beta, double* Cm, int ldc, double* ws, size_t ws_elems, int upper);
 
 /* ---- Gaussian sketch: G (rows x cols, ld) ~ N(0,1) from Philox4x32-10 ---- */
 int hq_sketch_philox(cudaStream_t stream, int rows, int cols, double* G, int ldg,

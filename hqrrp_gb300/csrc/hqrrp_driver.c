@@ -524,6 +524,12 @@ static int ws_check(hq_ws* w) {
   CK(hq_dgemm(w->st, dev, ta, tb, M, N, K, al, A, lda, B, ldb, be, C, ldc, w->ws,       \
               w->ws_elems))
 
+/* Z = U^T U of a block's reflectors, as far as the T factor reads it (the
+ * upper triangle). */
+#define DGRAM(b, mp)                                                                       \
+  CK(hq_dgemm_part(w->st, dev, 'T', 'N', b, b, mp, 1.0, w->U, w->ldu, w->U, w->ldu, 0.0,  \
+                   w->Z, w->ldz, w->ws, w->ws_elems, 1))
+
 /* sign * X Y^T (mode 0: written to C; mode 1: added to C) with split-BF16
  * tensor-core products: X has M rows (element (r, k) at X[r*xrs + k*xks]),
  * Y has N rows, both K long; C element (r, c) at C[r*crs + c*ccs].
@@ -735,7 +741,7 @@ static int block_reflector(hq_ws* w, int mp, int b, const double* tau, double* C
     if (rc) return rc;
     CK(hq_gram_unit_fix(w->st, b, w->U, w->ldu, w->Z, w->ldz));
   } else {
-    DG('T', 'N', b, b, mp, 1.0, w->U, w->ldu, w->U, w->ldu, 0.0, w->Z, w->ldz);
+    DGRAM(b, mp);
   }
   /* T (one SM, a sequential recurrence) on the side stream, overlapped with
    * W1 = U^T C, which does not need it; st waits for T before W2. */
@@ -1733,7 +1739,7 @@ static int apply_qk(hq_ws* w, char trans, int m, int nc, int k, int nb, const do
     const int bi = tr ? step : nblk - 1 - step;
     const int j = bi * nb, b = imin(nb, k - j), mp = m - j;
     CK(hq_unit_lower(w->st, mp, b, F + j + (size_t)j * ldf, ldf, w->U, w->ldu));
-    DG('T', 'N', b, b, mp, 1.0, w->U, w->ldu, w->U, w->ldu, 0.0, w->Z, w->ldz);
+    DGRAM(b, mp);
     CK(hq_larft_from_gram(w->st, b, w->Z, w->ldz, tau + j, w->T, w->ldt));
     /* C[j:, :] -= U op(T) U^T C[j:, :] */
     DG('T', 'N', b, nc, mp, 1.0, w->U, w->ldu, C + j, ldc, 0.0, w->W1, w->ldw);
