@@ -54,8 +54,12 @@ int hq_sketch_philox(cudaStream_t stream, int rows, int cols, double* G, int ldg
  * *npairs (zeroed by the launcher). */
 int hq_skinny_qrp(cudaStream_t stream, const hq_device_info* dev, int mY, int N, int b,
                   const double* Y, int ldy, double* V, int ldv, int* pairs, int* npairs,
-                  double* part, size_t part_elems, unsigned* bar, int* err,
-                  unsigned spin_limit, int fp32);
+                  double* part, size_t part_elems, void* xch, unsigned* tag, unsigned* bar,
+                  int* err, unsigned spin_limit, int fp32);
+/* xch: hq_skinny_xch_bytes(mY, fp32) bytes, zeroed once per call of the
+ * library and used by its launches alone; *tag counts those launches' stages
+ * (0 at first). */
+size_t hq_skinny_xch_bytes(int mY, int fp32);
 size_t hq_skinny_part_elems(const hq_device_info* dev, int mY);
 
 /* ---- Panel: pivoted (or plain) QR of the mp x nc block P (ldp) ---------

@@ -190,6 +190,8 @@ typedef struct {
   double *G, *Y, *V, *U, *T, *Z, *W1, *W2, *Bm, *B2, *ws, *part, *rowbuf, *tmp;
   int *pairs, *npairs, *perm, *labels, *label_tmp, *err;
   unsigned* bar;
+  void* selx;       /* pivot selection's exchange area, and its next stage tag */
+  unsigned seltag;
   int ldg, ldy, ldu, ldw, ldt, ldz, ldb, tmp_rows, tmp_cols;
   size_t ws_elems, part_elems;
   prof_rec* prof; /* non-NULL while profiling */
@@ -445,6 +447,8 @@ static int ws_setup(hq_ws* w, int m, int n, int nb, int pp, int pw) {
   w->label_tmp = ws_alloc(w, sizeof(int) * (size_t)imax(n, 2 * kmax));
   w->err = ws_alloc(w, sizeof(int) * 2);
   w->bar = ws_alloc(w, sizeof(unsigned) * 2);
+  const size_t selx_bytes = hq_skinny_xch_bytes(imin(mY, HQ_MAX_MY), w->mixed);
+  if (mY > 0) w->selx = ws_alloc(w, selx_bytes);
   if (w->mixed) {
     /* Digit buffers of the split products: the sketch's (mY > 0) and those of
      * the block reflectors (HQRRP blocks and dgeqp4's fixed-column blocks). */
@@ -501,6 +505,7 @@ static int ws_setup(hq_ws* w, int m, int n, int nb, int pp, int pw) {
   w->ph_override = -1;
   if (w->failed) return HQ_E_NOMEM;
   CK(cudaMemsetAsync(w->err, 0, sizeof(int) * 2, w->st));
+  if (w->selx) CK(cudaMemsetAsync(w->selx, 0, selx_bytes, w->st));
   if (w->gcount) CK(cudaMemsetAsync(w->gcount, 0, sizeof(int) * 2, w->st));
   prof_start(w);
   return HQ_OK;
@@ -849,7 +854,8 @@ static int core_hqrrp_k(hq_ws* w, int m, int n, double* dA, int ldda, int* djpvt
       /* Mixed: the sketch's reflector applications in FP32 (it is formed from
        * two-digit BF16 operands and only steers pivots); norms stay FP64. */
       CK(hq_skinny_qrp(w->st, dev, mY, n - j, b, YR, w->ldy, w->V, w->ldy, w->pairs, w->npairs,
-                       w->part, w->part_elems, w->bar, w->err, spin, w->mixed));
+                       w->part, w->part_elems, w->selx, &w->seltag, w->bar, w->err, spin,
+                       w->mixed));
       CK(hq_permute_pairs(w->st, m, AR, ldda, n - j, w->pairs, w->npairs, 2 * b, w->tmp,
                           djpvt + j, w->label_tmp));
       CK(hq_permute_pairs(w->st, mY, YR, w->ldy, n - j, w->pairs, w->npairs, 2 * b, w->tmp,

@@ -269,344 +269,473 @@ __global__ void __launch_bounds__(NT, 1) skinny_qrp_kernel(SkArgs a) {
   }
 }
 
-// Register-resident variant: two adjacent lanes hold one sketch column, rows
-// interleaved (lane parity h holds rows 2i + h, i < RPT), so a stage reads its
-// columns from registers instead of shared memory; the reflector is staged in
-// shared memory (zero above the stage's row, so whole chunks of 16 rows above
-// it are skipped).  FP64 issue is the scarce resource on this GPU, so scalar
-// work is done once, not by every thread: one lane builds the reflector, one
-// thread per column downdates its norm, and pivot candidates compare integer
-// keys.  Used when a CTA's range has at most NT/2 columns and mY <= 2 * RPT;
-// otherwise the shared-memory kernel above runs.  Record layout (as 64-bit
-// integers): [0] norm key, [1] position, [2] column, then the column's entries.
+// Register-resident variant, used when mY and the columns per CTA fit it (see
+// launch_reg): LPC adjacent lanes hold one sketch column, rows interleaved
+// (lane l has rows LPC t + l, t < RPT), so a stage reads its columns from
+// registers; the reflector is staged in shared memory in the same order and
+// read 16 bytes at a time, whole chunks of 16 rows above the stage's row being
+// jumped over.  Scalar work is done once, not by every thread: one lane builds
+// the reflector, one thread per column downdates its norm, and pivot
+// candidates compare integer keys.
+//
+// What bounds a stage is the latency of agreeing on the pivot, so the exchange
+// has neither a fence nor a counter.  A CTA writes its best candidate -- norm
+// key and position, once for every CTA, and the column once -- in words that
+// carry the stage's tag next to the value (128- and 64-bit scalar stores,
+// which are single-copy atomic).  One warp per CTA polls its CTA's own copy of
+// the P headers, picks the winner and polls its column: a word whose tag
+// matches holds this stage's value, so nothing has to be ordered before
+// anything else.  (With one copy of the headers for all, the polls of 128 CTAs
+// queue up at the few cache lines that the headers are written to: 3500 clocks
+// in that wait alone, against 1400 for 24 CTAs.)  Headers and columns alternate between two
+// buffers.  A CTA overwrites a buffer at stage s + 2 after it has seen every
+// CTA's header of stage s + 1, which each wrote after it had read stage s.
+// Tags grow over all launches of a call and the area is zeroed once per call.
+//
+// Measured on GB300 a stage, against two lanes a column and a counter barrier
+// (release add and spin, then all headers, then the column): FP32, 138 rows,
+// 16384 columns 5.5 -> 3.5 us, 3000 columns 5.2 -> 2.8; FP64, 74 rows, 2000
+// columns 9.7 -> 4.6 (of which 1.6 the reflector's FP64 scalars and sums).
 //
 // T is the arithmetic of the reflector applications (the bulk of the FP64
 // work): double for the plain path, float for the mixed path, whose sketch is
 // formed from two-digit BF16 operands (~16 significant bits) and only steers
-// pivots.  Norms, their LAWN 176 downdate and recomputation, and the
-// reflector scalars are FP64 in both.  The mixed path keeps squared norms:
+// pivots.  Norms, their LAWN 176 downdate and recomputation, and in the plain
+// path the reflector scalars are FP64.  Norms are kept squared:
 // d^2 <- d^2 - r^2, recomputed when d^2 - r^2 <= tol3z e^2 -- LAPACK's test
 // t2 = (d^2 - r^2) / e^2 <= tol3z without its two divisions and square root
-// (~1.2k cycles of FP64 latency per stage on this GPU); the argmax of d^2 is
-// the argmax of d.
+// (~2.2k clocks of FP64 a stage on this GPU); the argmax of d^2 is the argmax
+// of d.  In FP32 a column's dot product is four chains (rows modulo 4) added
+// as (0 + 2) + (1 + 3), whatever the launch shape.
+struct RegArgs {
+  int mY, N, b;
+  const double* Y;
+  int ldy;
+  int* pairs;
+  int* npairs;
+  int max_pairs;
+  unsigned char* hdrs;  // [2][MAX_P copies][MAX_P] 16-byte headers
+  unsigned char* recs;  // [2][MAX_P] columns
+  unsigned tag0;        // stage s's tag is tag0 + s + 1
+  int* err;
+  unsigned spin_limit;
+};
+constexpr int MAX_P = 160;               // CTAs
+constexpr int HDR_LANE = MAX_P / 32;     // headers per polling lane
+
+__device__ __forceinline__ void st_word(unsigned char* p, unsigned long long lo,
+                                        unsigned long long hi) {
+  asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], t;\n}" ::"l"(p),
+               "l"(lo), "l"(hi)
+               : "memory");
+}
+__device__ __forceinline__ void ld_word(const unsigned char* p, unsigned long long& lo,
+                                        unsigned long long& hi) {
+  asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}"
+               : "=l"(lo), "=l"(hi)
+               : "l"(p)
+               : "memory");
+}
+__device__ __forceinline__ void st_word(unsigned char* p, unsigned long long v) {
+  asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ void ld_word(const unsigned char* p, unsigned long long& v) {
+  asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+}
+
+// One entry of a published column and its tag: 8 bytes in FP32, 16 in FP64.
+template <typename T>
+struct Tagged;
+template <>
+struct Tagged<float> {
+  static constexpr int BYTES = 8;
+  static __device__ __forceinline__ void put(unsigned char* p, float x, unsigned tag) {
+    st_word(p, ((unsigned long long)tag << 32) | __float_as_uint(x));
+  }
+  static __device__ __forceinline__ bool get(const unsigned char* p, unsigned tag, float& x) {
+    unsigned long long v;
+    ld_word(p, v);
+    x = __uint_as_float((unsigned)v);
+    return (unsigned)(v >> 32) == tag;
+  }
+};
+template <>
+struct Tagged<double> {
+  static constexpr int BYTES = 16;
+  static __device__ __forceinline__ void put(unsigned char* p, double x, unsigned tag) {
+    st_word(p, (unsigned long long)__double_as_longlong(x), tag);
+  }
+  static __device__ __forceinline__ bool get(const unsigned char* p, unsigned tag, double& x) {
+    unsigned long long lo, hi;
+    ld_word(p, lo, hi);
+    x = __longlong_as_double((long long)lo);
+    return hi == tag;
+  }
+};
+
 __device__ __forceinline__ bool better_key(long long k1, int p1, long long k2, int p2) {
   return k1 > k2 || (k1 == k2 && p1 < p2);
 }
 
-template <int RPT, typename T>
-__global__ void __launch_bounds__(NT, 1) skinny_qrp_reg_kernel(SkArgs a) {
+// Best (key, position) of the warp in every lane: largest key, then lowest
+// position; keys are >= -3.  Three integer reductions instead of five rounds
+// of shuffles.
+__device__ __forceinline__ void warp_best(long long& key, int& pos) {
+  const unsigned long long u = (unsigned long long)(key + 4);
+  const unsigned hi = (unsigned)(u >> 32);
+  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned lo = hi == mh ? (unsigned)u : 0u;
+  const unsigned ml = __reduce_max_sync(0xffffffffu, lo);
+  const bool mine = hi == mh && (unsigned)u == ml;
+  pos = __reduce_min_sync(0xffffffffu, mine ? pos : 0x7fffffff);
+  key = (long long)(((unsigned long long)mh << 32) | ml) - 4;
+}
+
+// case i of a switch over 16-row chunks: do it, and fall through to the next.
+#define HQ_CHUNKS(DO)                                                                        \
+  case 0: DO(0) case 1: DO(1) case 2: DO(2) case 3: DO(3) case 4: DO(4) case 5: DO(5)        \
+  case 6: DO(6) case 7: DO(7) case 8: DO(8) case 9: DO(9) case 10: DO(10) case 11: DO(11)    \
+  case 12: DO(12) case 13: DO(13) case 14: DO(14) case 15: DO(15)
+
+template <int CNT, int RPT, int LPC, typename T>
+__global__ void __launch_bounds__(CNT, 1) skinny_qrp_reg_kernel(RegArgs a) {
   HQ_PDL_WAIT();
-  constexpr int NCH = RPT / 8;  // chunks of 8 registers = 16 rows
-  constexpr bool SQ = sizeof(T) == 4;  // mixed path: squared norms
-  constexpr int NC = NT / 2;
-  __shared__ __align__(16) T sv[2 * RPT];   // winner column (raw; scaled in FP32)
-  __shared__ __align__(16) T sv2[2 * RPT];  // the reflector v
-  __shared__ long long s_bk[NWARP];
-  __shared__ int s_bp[NWARP], s_bc[NWARP];
-  __shared__ int spos[NC], sflag[NC];
-  __shared__ double sd[NC], se[NC], srs[NC];
-  __shared__ int s_flag, s_win_pos, s_win_cta, s_win_col;
-  __shared__ T s_tau, s_scale;
+  constexpr bool F32 = sizeof(T) == 4;
+  constexpr int NC = CNT / LPC;        // columns per CTA
+  constexpr int CE = 16 / LPC;         // entries of a lane per 16-row chunk
+  constexpr int NCH = RPT / CE;
+  constexpr int STR = RPT + 16 / (int)sizeof(T) * ((RPT * (int)sizeof(T)) % 128 == 0);  // no bank conflicts
+  constexpr int RLANE = (LPC * RPT + 31) / 32;  // rows per lane of the polling warp
+  // The reflector stays in registers between its two uses where they suffice.
+  constexpr bool KEEP = RPT * (int)sizeof(T) <= (F32 ? 144 : 256);
+  static_assert(RPT % CE == 0 && CE * sizeof(T) % 16 == 0 && NCH <= 16, "chunks");
+  static_assert(NC % 32 == 0, "downdating threads fill whole warps");
+  __shared__ __align__(16) T sv[LPC * STR];  // the reflector v, lane-major
+  __shared__ long long s_bk[NC / 32];
+  __shared__ int s_bp[NC / 32];
+  __shared__ int sflag[NC];
+  __shared__ T srs[NC];        // the columns' new entries of row s
+  __shared__ double snrm[NC];  // (re)computed squared norms
+  __shared__ int s_win_pos, s_dead;
+  __shared__ T s_tau;
   const int P = gridDim.x, cta = blockIdx.x, tid = threadIdx.x;
-  const int lane = tid & 31, warp = tid >> 5, h = lane & 1;
-  const unsigned pmask = 3u << (lane & 30);
+  const int lane = tid & 31, warp = tid >> 5, l = lane & (LPC - 1);
   const int mY = a.mY;
   const int c_lo = (int)((long long)cta * a.N / P);
   const int c_hi = (int)((long long)(cta + 1) * a.N / P);
   const int nloc = c_hi - c_lo;
-  const int c = tid >> 1;  // this pair's local column
+  const int c = tid / LPC;  // this lane group's local column
   const bool have = c < nloc;
+  const size_t rec_bytes = (size_t)mY * Tagged<T>::BYTES;
 
   T x[RPT];
   // FP32 registers hold the column times 2^-ec (ec from its norm), so FP32's
-  // range never limits the input; unscale = 2^ec converts back (exact).
-  double unscale = 1.0;
+  // range never limits the input; 2^ec converts back (exact).
+  int ec = 0;
   {
     const double* src = a.Y + (size_t)(c_lo + (have ? c : 0)) * a.ldy;
     double q = 0.0;
-    if constexpr (SQ) {
-#pragma unroll 8
-      for (int i = 0; i < RPT; ++i) {
-        const int r = 2 * i + h;
-        const double y = (have && r < mY) ? src[r] : 0.0;
-        q = fma(y, y, q);
-      }
-      q += __shfl_xor_sync(0xffffffffu, q, 1);
+#pragma unroll
+    for (int t = 0; t < RPT; ++t) {
+      const int r = LPC * t + l;
+      const double y = (have && r < mY) ? src[r] : 0.0;
+      if constexpr (!F32) x[t] = y;
+      q = fma(y, y, q);
+    }
+#pragma unroll
+    for (int o = LPC / 2; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+    if constexpr (F32) {
       int eq = (int)((__double_as_longlong(q) >> 52) & 0x7FF) - 1023;  // q >= 0
       if (eq < -1022) eq = -1022;
-      const int ec = eq / 2;
+      ec = eq / 2;
       const double sc = __longlong_as_double((long long)(1023 - ec) << 52);
-      unscale = __longlong_as_double((long long)(1023 + ec) << 52);
 #pragma unroll
-      for (int i = 0; i < RPT; ++i) {
-        const int r = 2 * i + h;
-        x[i] = (have && r < mY) ? (T)(src[r] * sc) : (T)0;
+      for (int t = 0; t < RPT; ++t) {
+        const int r = LPC * t + l;
+        x[t] = (have && r < mY) ? (T)(src[r] * sc) : (T)0;
       }
-    } else {
-#pragma unroll
-      for (int i = 0; i < RPT; ++i) {
-        const int r = 2 * i + h;
-        x[i] = (have && r < mY) ? (T)src[r] : (T)0;
-        q = fma((double)x[i], (double)x[i], q);
-      }
-      q += __shfl_xor_sync(0xffffffffu, q, 1);
     }
-    if (have && h == 0) {
-      sd[c] = SQ ? q : sqrt(q);
-      se[c] = sd[c];
-      spos[c] = c_lo + c;
+    if (l == 0) {
+      snrm[c] = q;
+      sflag[c] = ec;
     }
   }
-  for (int r = tid; r < 2 * RPT; r += NT) sv2[r] = (T)0;
+  for (int r = tid; r < LPC * STR; r += CNT) sv[r] = (T)0;
+  if (tid == 0) s_dead = 0;
   __syncthreads();
 
-  unsigned epoch = 0;
-  // Publish this CTA's best candidate for stage s (entries from row s on).
+  int mypos = have ? c_lo + c : -1;  // position of the group's column
+  const bool dd = tid < nloc;        // this thread downdates column tid
+  int dpos = dd ? c_lo + tid : -1;
+  double dn = dd ? snrm[tid] : 0.0;
+  double thr = HQ_TOL3Z * dn;  // recompute at or below this
+  const double unscale = __longlong_as_double((long long)(1023 + (tid < NC ? sflag[tid] : 0)) << 52);
+
+  // This warp's best candidate for stage s (warps of downdating threads).
+  auto local_best = [&](int s) {
+    if (tid < NC) {
+      long long k = -2;
+      int p = 0x7fffffff;
+      if (dd && dpos >= s) {
+        k = hq_norm_key(dn);
+        p = dpos;
+      }
+      warp_best(k, p);
+      if (lane == 0) {
+        s_bk[warp] = k;
+        s_bp[warp] = p;
+      }
+    }
+  };
+  // Write this CTA's best candidate for stage s (s_bk and s_bp complete): the
+  // warp that holds the column, or warp 0 when no column is active.
   auto publish = [&](int s) {
-    long long bk = -2;
-    int bp = 0x7fffffff, bc = -1;
-    if (tid < nloc && spos[tid] >= s) {
-      bk = hq_norm_key(sd[tid]);
-      bp = spos[tid];
-      bc = tid;
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      const long long ok = __shfl_xor_sync(0xffffffffu, bk, o);
-      const int op = __shfl_xor_sync(0xffffffffu, bp, o);
-      const int oc = __shfl_xor_sync(0xffffffffu, bc, o);
-      if (better_key(ok, op, bk, bp)) { bk = ok; bp = op; bc = oc; }
-    }
-    if (lane == 0) { s_bk[warp] = bk; s_bp[warp] = bp; s_bc[warp] = bc; }
-    __syncthreads();
-    bk = s_bk[0];
-    bp = s_bp[0];
-    bc = s_bc[0];
-    for (int w = 1; w < NWARP; ++w)
-      if (better_key(s_bk[w], s_bp[w], bk, bp)) { bk = s_bk[w]; bp = s_bp[w]; bc = s_bc[w]; }
-    double* rec = a.part + ((size_t)((epoch + 1) & 1) * P + cta) * a.rec;
-    if (tid == 0) {
-      long long* hdr = reinterpret_cast<long long*>(rec);
-      hdr[0] = bk;
-      hdr[1] = bp;
-      hdr[2] = bc >= 0 ? c_lo + bc : -1;
-    }
-    if (bc >= 0 && c == bc) {
-      T* recd = reinterpret_cast<T*>(rec + HDR);
+    long long k = s_bk[0];
+    int p = s_bp[0];
 #pragma unroll
-      for (int i = 0; i < RPT; ++i) {
-        const int r = 2 * i + h;
-        if (r >= s && r < mY) recd[r] = x[i];
+    for (int w = 1; w < NC / 32; ++w)
+      if (better_key(s_bk[w], s_bp[w], k, p)) { k = s_bk[w]; p = s_bp[w]; }
+    const unsigned tag = a.tag0 + (unsigned)s + 1u;
+    const bool mine = k > -2 && have && mypos == p;
+    if (__any_sync(0xffffffffu, mine) || (k <= -2 && warp == 0)) {
+      unsigned char* h = a.hdrs + ((size_t)(s & 1) * MAX_P * MAX_P + cta) * 16;
+      const unsigned long long w1 = ((unsigned long long)tag << 32) | (unsigned)p;
+#pragma unroll
+      for (int j = 0; j < HDR_LANE; ++j) {
+        const int q = lane + 32 * j;
+        if (32 * j < P && q < P) st_word(h + (size_t)q * MAX_P * 16, (unsigned long long)k, w1);
+      }
+      if (mine) {
+        unsigned char* rec = a.recs + ((size_t)(s & 1) * MAX_P + cta) * rec_bytes;
+#pragma unroll
+        for (int t = 0; t < RPT; ++t) {
+          const int r = LPC * t + l;
+          if (r >= s && r < mY) Tagged<T>::put(rec + (size_t)r * Tagged<T>::BYTES, x[t], tag);
+        }
       }
     }
   };
 
+  local_best(0);
+  __syncthreads();
   publish(0);
   for (int s = 0; s < a.b; ++s) {
-    ++epoch;
-    if (!hq_grid_barrier(a.bar, a.err, epoch, a.spin_limit, &s_flag)) return;
-    const double* recs = a.part + (size_t)(epoch & 1) * P * a.rec;
-
-    // Winner: every CTA reduces the same records in the same way; all header
-    // loads are issued before any is used.
     if (warp == 0) {
-      constexpr int QL = 5;  // records per lane: P <= 160
-      long long kk[QL];
-      int pp[QL], cc[QL];
+      const unsigned tag = a.tag0 + (unsigned)s + 1u;
+      // Winner: every CTA reduces the same headers in the same way.
+      const unsigned char* h0 = a.hdrs + ((size_t)(s & 1) * MAX_P + cta) * MAX_P * 16;
+      long long kk[HDR_LANE];
+      int pp[HDR_LANE];
+      bool ok = false;
+      unsigned it = 0;
+      for (;;) {
+        ok = true;
 #pragma unroll
-      for (int j = 0; j < QL; ++j) {
-        const int q = lane + 32 * j;
-        const long long* hdr = reinterpret_cast<const long long*>(recs + (size_t)q * a.rec);
-        kk[j] = q < P ? hq_ldcg(hdr) : -3;
-        pp[j] = q < P ? (int)hq_ldcg(hdr + 1) : 0x7fffffff;
-        cc[j] = q < P ? (int)hq_ldcg(hdr + 2) : -1;
+        for (int j = 0; j < HDR_LANE; ++j) {
+          const int q = lane + 32 * j;
+          kk[j] = -3;
+          pp[j] = 0x7fffffff;
+          if (32 * j < P && q < P) {
+            unsigned long long k0, w;
+            ld_word(h0 + (size_t)q * 16, k0, w);
+            kk[j] = (long long)k0;
+            pp[j] = (int)(unsigned)w;
+            ok = ok && (unsigned)(w >> 32) == tag;
+          }
+        }
+        ok = __all_sync(0xffffffffu, ok);
+        if (ok || ++it >= a.spin_limit) break;
+        if ((it & 15u) == 0u && __any_sync(0xffffffffu, hq_ld_volatile(a.err) != 0)) break;
       }
-      long long bk = -3;
-      int bp = 0x7fffffff, bq = -1, bcol = -1;
+      long long bk = kk[0];
+      int bp = pp[0], bq = lane;
 #pragma unroll
-      for (int j = 0; j < QL; ++j)
-        if (kk[j] > -2 && better_key(kk[j], pp[j], bk, bp)) {
+      for (int j = 1; j < HDR_LANE; ++j)
+        if (better_key(kk[j], pp[j], bk, bp)) {
           bk = kk[j];
           bp = pp[j];
           bq = lane + 32 * j;
-          bcol = cc[j];
         }
-      for (int o = 16; o > 0; o >>= 1) {
-        const long long ok = __shfl_xor_sync(0xffffffffu, bk, o);
-        const int op = __shfl_xor_sync(0xffffffffu, bp, o);
-        const int oq = __shfl_xor_sync(0xffffffffu, bq, o);
-        const int ocol = __shfl_xor_sync(0xffffffffu, bcol, o);
-        if (better_key(ok, op, bk, bp)) { bk = ok; bp = op; bq = oq; bcol = ocol; }
+      long long wk = bk;
+      int wp = bp;
+      warp_best(wk, wp);
+      const unsigned who = __ballot_sync(0xffffffffu, bk == wk && bp == wp);
+      const int wcta = __shfl_sync(0xffffffffu, bq, __ffs((int)who) - 1);
+      const bool none = ok && wk <= -2;  // no active column anywhere: cannot happen for b <= N
+      // The winner's column, rows s (every lane) and s + 1 + lane + 32 i.
+      T al = (T)0, z[RLANE];
+      if (ok && !none) {
+        const unsigned char* rec = a.recs + ((size_t)(s & 1) * MAX_P + wcta) * rec_bytes;
+        for (;;) {
+          bool got = Tagged<T>::get(rec + (size_t)s * Tagged<T>::BYTES, tag, al);
+#pragma unroll
+          for (int i = 0; i < RLANE; ++i) {
+            const int r = s + 1 + lane + 32 * i;
+            z[i] = (T)0;
+            if (r < mY) got = Tagged<T>::get(rec + (size_t)r * Tagged<T>::BYTES, tag, z[i]) && got;
+          }
+          ok = __all_sync(0xffffffffu, got);
+          if (ok || ++it >= a.spin_limit) break;
+          if ((it & 15u) == 0u && __any_sync(0xffffffffu, hq_ld_volatile(a.err) != 0)) break;
+        }
       }
-      if (lane == 0) {
-        s_win_pos = bp;
-        s_win_cta = bq;
-        s_win_col = bcol;
+      if (!ok || none) {
+        if (lane == 0) {
+          atomicCAS(a.err, 0, none ? HQ_ERR_BAD_SHAPE : HQ_ERR_BARRIER_TIMEOUT);
+          s_dead = 1;
+        }
+      } else {
+        if (lane == 0) s_win_pos = wp;
+        // Tail norm, reflector, v = [1; scale * tail].  In FP32 the reflector
+        // of the scaled column is built directly (it does not depend on the
+        // column's scale): beta = -sign(alpha) sqrt(alpha^2 + q), tau = (beta
+        // - alpha) / beta, scale = 1 / (alpha - beta); tau = 0 for a zero tail.
+        T q = (T)0;
+#pragma unroll
+        for (int i = 0; i < RLANE; ++i)
+          if (s + 1 + lane + 32 * i < mY) q = fma(z[i], z[i], q);
+        q = hq_warp_sum(q);
+        T tau, scale;
+        if constexpr (F32) {
+          tau = 0.f;
+          scale = 0.f;
+          if (q > 0.f) {
+            const float beta = -copysignf(sqrtf(fmaf(al, al, q)), al);
+            tau = (beta - al) / beta;
+            scale = 1.f / (al - beta);
+          }
+        } else {
+          const HqReflector hr = hq_make_reflector_sq(al, q);
+          tau = hr.tau;
+          scale = hr.scale;
+        }
+        auto put = [&](int r, T v) { sv[(r & (LPC - 1)) * STR + r / LPC] = v; };
+#pragma unroll
+        for (int i = 0; i < RLANE; ++i) {
+          const int r = s + 1 + lane + 32 * i;
+          if (r < mY) put(r, scale * z[i]);
+        }
+        if (lane == 0) {
+          s_tau = tau;
+          put(s, (T)1);
+          if (s > 0) put(s - 1, (T)0);
+        }
       }
     }
     __syncthreads();
-    const int wpos = s_win_pos, wcta = s_win_cta, wcol = s_win_col;
-    if (wcta < 0) {  // no active column anywhere: cannot happen for b <= N
-      if (tid == 0) atomicCAS(a.err, 0, HQ_ERR_BAD_SHAPE);
-      return;
-    }
+    if (s_dead != 0) return;  // an exchange gave up; the other CTAs see the error word
     // Position bookkeeping for the swap of positions s and wpos (columns are
     // never moved).
-    if (tid < nloc) {
-      if (wpos != s && spos[tid] == s) spos[tid] = wpos;
-      if (cta == wcta && c_lo + tid == wcol) spos[tid] = s;
-    }
-    // Winner column, rows s..mY-1.
-    const T* wrec = reinterpret_cast<const T*>(recs + (size_t)wcta * a.rec + HDR);
-    for (int r = s + tid; r < mY; r += NT) sv[r] = __ldcg(wrec + r);
-    __syncthreads();
+    const int wpos = s_win_pos;
+    if (have) mypos = mypos == wpos ? s : (mypos == s ? wpos : mypos);
+    if (dd) dpos = dpos == wpos ? s : (dpos == s ? wpos : dpos);
     if (s + 1 == a.b) break;  // the pivots are complete; V is discarded
-    // Warp 0: tail norm, reflector (one lane), v = [1; scale * tail].  In
-    // FP32 the reflector of the scaled column is built directly (it does not
-    // depend on the column's scale): beta = -sign(alpha) sqrt(alpha^2 + q),
-    // tau = (beta - alpha) / beta, scale = 1 / (alpha - beta); tau = 0 when
-    // the tail is zero.
-    if (warp == 0) {
-      T q = (T)0;
-      for (int r = s + 1 + lane; r < mY; r += 32) q = fma(sv[r], sv[r], q);
-      q = hq_warp_sum(q);
-      if (lane == 0) {
-        if constexpr (SQ) {
-          const float alpha = sv[s];
-          float tau = 0.f, scale = 0.f;
-          if (q > 0.f) {
-            const float beta = -copysignf(sqrtf(fmaf(alpha, alpha, q)), alpha);
-            tau = (beta - alpha) / beta;
-            scale = 1.f / (alpha - beta);
-          }
-          s_tau = tau;
-          s_scale = scale;
-        } else {
-          const HqReflector hr = hq_make_reflector_sq(sv[s], q);
-          s_tau = hr.tau;
-          s_scale = hr.scale;
-        }
-      }
-      __syncwarp();
-      const T scale = s_scale;
-      for (int r = s + 1 + lane; r < mY; r += 32) sv2[r] = scale * sv[r];
-      if (lane == 0) {
-        sv2[s] = (T)1;
-        if (s > 0) sv2[s - 1] = (T)0;
-      }
-    }
-    __syncthreads();
 
-    // Apply H = I - tau v v^T to this pair's column (if still active); the
+    // Apply H = I - tau v v^T to the group's column (if still active); the
     // new entry of row s goes to srs for the downdate.
-    const bool active = have && spos[c] > s;
-    if (active) {
+    const bool active = have && mypos > s;
+    if (__any_sync(0xffffffffu, active)) {
       const int sch = s >> 4;  // first chunk holding a row >= s
+      const T* vl = sv + l * STR;
+      __align__(16) T v[RPT];
+      auto load_chunk = [&](int ch) {
+#pragma unroll
+        for (int j = 0; j < CE * (int)sizeof(T) / 16; ++j)
+          reinterpret_cast<int4*>(v + CE * ch)[j] = reinterpret_cast<const int4*>(vl + CE * ch)[j];
+      };
       T w = (T)0;
-      if constexpr (SQ) {  // two chains: half the FP32 latency
-        T w1 = (T)0;
+#define HQ_DOT(I)                                                                   \
+  if constexpr (I < NCH) {                                                          \
+    load_chunk(I);                                                                  \
+    _Pragma("unroll") for (int j = 0; j < CE; ++j) w = fma(v[CE * I + j], x[CE * I + j], w); \
+  }
+      switch (sch) { HQ_CHUNKS(HQ_DOT) }
+#undef HQ_DOT
 #pragma unroll
-        for (int ch = 0; ch < NCH; ++ch) {
-          if (ch >= sch && 16 * ch < mY) {
-#pragma unroll
-            for (int j = 0; j < 8; j += 2) {
-              w = fma(sv2[16 * ch + 2 * j + h], x[8 * ch + j], w);
-              w1 = fma(sv2[16 * ch + 2 * j + 2 + h], x[8 * ch + j + 1], w1);
-            }
-          }
-        }
-        w += w1;
-      } else {
-#pragma unroll
-        for (int ch = 0; ch < NCH; ++ch) {
-          if (ch >= sch && 16 * ch < mY) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) w = fma(sv2[16 * ch + 2 * j + h], x[8 * ch + j], w);
-          }
-        }
+      for (int o = LPC / 2; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+      if (active) {
+        const T g = (T)(-s_tau) * w;
+        T xs = (T)0;  // the new entry of row s, in the lane that holds it
+        const int ts = s / LPC;
+#define HQ_UPD(I)                                                                    \
+  if constexpr (I < NCH) {                                                           \
+    if constexpr (!KEEP) load_chunk(I);                                              \
+    _Pragma("unroll") for (int j = 0; j < CE; ++j)                                   \
+      x[CE * I + j] = fma(g, v[CE * I + j], x[CE * I + j]);                          \
+  }
+        switch (sch) { HQ_CHUNKS(HQ_UPD) }
+#undef HQ_UPD
+#define HQ_PICK(I)                                                                  \
+  if constexpr (I < NCH) {                                                          \
+    _Pragma("unroll") for (int j = 0; j < CE; ++j) if (CE * I + j == ts) xs = x[CE * I + j]; \
+  }                                                                                 \
+  break;
+        switch (sch) { HQ_CHUNKS(HQ_PICK) }
+#undef HQ_PICK
+        if (l == (s & (LPC - 1))) srs[c] = xs;
       }
-      w += __shfl_xor_sync(pmask, w, 1);
-      const T g = (T)(-s_tau) * w;
-      T xs_new = (T)0;
-#pragma unroll
-      for (int ch = 0; ch < NCH; ++ch) {
-        if (ch >= sch && 16 * ch < mY) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            x[8 * ch + j] = fma(g, sv2[16 * ch + 2 * j + h], x[8 * ch + j]);
-            if (16 * ch + 2 * j + h == s) xs_new = x[8 * ch + j];
-          }
-        }
-      }
-      if (h == (s & 1)) srs[c] = SQ ? (double)xs_new * unscale : (double)xs_new;
     }
     __syncthreads();
-    // Norm downdate, one thread per column (LAWN 176); flagged norms are
-    // recomputed from the pair's registers.
+    // Norm downdate, one thread per column (LAWN 176 on squared norms, the
+    // comparison on the integer pipe: thr >= 0, and a negative difference
+    // orders below it); flagged norms are recomputed from the registers.
     int flag = 0;
-    if (tid < nloc && spos[tid] > s) {
-      double dc = sd[tid];
-      if (dc != 0.0) {
-        if (SQ) {
-          const double r = srs[tid];
-          const double nd = fma(-r, r, dc);
-          if (nd <= HQ_TOL3Z * se[tid]) flag = 1;
-          else sd[tid] = nd;
-        } else {
-          double t1 = fabs(srs[tid]) / dc;
-          t1 = (1.0 + t1) * (1.0 - t1);
-          if (0.0 > t1) t1 = 0.0;
-          const double ratio = dc / se[tid];
-          const double t2 = t1 * ratio * ratio;
-          if (t2 <= HQ_TOL3Z) flag = 1;
-          else sd[tid] = dc * sqrt(t1);
-        }
-      }
+    if (dd && dpos > s && dn != 0.0) {
+      const double r = F32 ? (double)srs[tid] * unscale : (double)srs[tid];
+      const double nd = fma(-r, r, dn);
+      const long long nb = __double_as_longlong(nd);
+      if (nb <= __double_as_longlong(thr) || nb > 0x7ff0000000000000LL) flag = 1;
+      else dn = nd;
     }
     if (tid < NC) sflag[tid] = flag;
+    local_best(s + 1);
     if (__syncthreads_or(flag)) {
       if (active && sflag[c]) {
-        double q2 = 0.0;
-        if constexpr (SQ) {
-          float f0 = 0.f, f1 = 0.f;
+        T f = (T)0;
 #pragma unroll
-          for (int i = 0; i < RPT; i += 2) {
-            if (2 * i + h > s) f0 = fmaf(x[i], x[i], f0);
-            if (i + 1 < RPT && 2 * (i + 1) + h > s) f1 = fmaf(x[i + 1], x[i + 1], f1);
-          }
-          f0 += f1;
-          f0 += __shfl_xor_sync(pmask, f0, 1);
-          q2 = (double)f0 * (unscale * unscale);
-        } else {
+        for (int t = 0; t < RPT; ++t)
+          if (LPC * t + l > s) f = fma(x[t], x[t], f);
+        const unsigned gmask = ((1u << LPC) - 1u) << (lane & ~(LPC - 1));
 #pragma unroll
-          for (int i = 0; i < RPT; ++i) {
-            const int r = 2 * i + h;
-            if (r > s) q2 = fma((double)x[i], (double)x[i], q2);
-          }
-          q2 += __shfl_xor_sync(pmask, q2, 1);
-        }
-        const double dc = (mY - s - 1 > 0) ? (SQ ? q2 : sqrt(q2)) : 0.0;
-        if (h == 0) {
-          sd[c] = dc;
-          se[c] = dc;
+        for (int o = LPC / 2; o > 0; o >>= 1) f += __shfl_xor_sync(gmask, f, o);
+        if (l == 0) {
+          const double up = __longlong_as_double((long long)(1023 + ec) << 52);
+          snrm[c] = mY - s - 1 > 0 ? (double)f * (up * up) : 0.0;
         }
       }
+      __syncthreads();
+      if (flag) {
+        dn = snrm[tid];
+        thr = HQ_TOL3Z * dn;
+      }
+      local_best(s + 1);
       __syncthreads();
     }
     publish(s + 1);
   }
 
   // Final permutation as (dst, src) pairs for the columns that moved.
-  for (int cc = tid; cc < nloc; cc += NT) {
-    if (spos[cc] != c_lo + cc) {
-      const int i = atomicAdd(a.npairs, 1);
-      if (i < a.max_pairs) {
-        a.pairs[2 * i] = spos[cc];
-        a.pairs[2 * i + 1] = c_lo + cc;
-      } else {
-        atomicCAS(a.err, 0, HQ_ERR_BAD_SHAPE);  // only after an aborted run
-      }
+  if (have && l == 0 && mypos != c_lo + c) {
+    const int i = atomicAdd(a.npairs, 1);
+    if (i < a.max_pairs) {
+      a.pairs[2 * i] = mypos;
+      a.pairs[2 * i + 1] = c_lo + c;
+    } else {
+      atomicCAS(a.err, 0, HQ_ERR_BAD_SHAPE);  // only after an aborted run
     }
   }
+}
+#undef HQ_CHUNKS
+
+// A launch shape of the register kernel: entry, threads, columns a CTA holds,
+// rows it takes.
+struct RegShape {
+  const void* fn;
+  int threads, cols, rows;
+};
+template <int CNT, int RPT, int LPC, typename T>
+RegShape reg_shape() {
+  return {(const void*)skinny_qrp_reg_kernel<CNT, RPT, LPC, T>, CNT, CNT / LPC, LPC * RPT};
 }
 
 int skinny_grid(const hq_device_info* dev, int N) {
@@ -622,10 +751,71 @@ extern "C" size_t hq_skinny_part_elems(const hq_device_info* dev, int mY) {
   return (size_t)2 * dev->num_sms * rec;
 }
 
+// The register kernel's exchange area: fixed places for MAX_P CTAs, so a word
+// never changes its meaning from one launch of a call to the next.
+extern "C" size_t hq_skinny_xch_bytes(int mY, int fp32) {
+  return (size_t)2 * MAX_P * (MAX_P * 16 + (size_t)mY * (fp32 ? 8 : 16));
+}
+
+// The register kernel, if a shape holds the sketch; cudaErrorNotSupported
+// otherwise.
+static int launch_reg(cudaStream_t stream, const hq_device_info* dev, const SkArgs& s, void* xch,
+                      unsigned* tag, int fp32) {
+  // Shapes by rows and columns per CTA, the first that holds the sketch on one
+  // CTA per SM.  FP32: four lanes a column, 64 columns a CTA, else 128 (3000
+  // columns: 128 a CTA 9.3 ms a factorization, 64 8.2, 32 8.2).  FP64: eight
+  // lanes and 32 columns, else four and 64, or two and 128.
+  constexpr int N_SHAPES = 14, F32_SHAPES = 6;
+  static const RegShape shapes[N_SHAPES] = {
+      reg_shape<256, 20, 4, float>(),  reg_shape<256, 36, 4, float>(),
+      reg_shape<256, 64, 4, float>(),  reg_shape<512, 20, 4, float>(),
+      reg_shape<512, 36, 4, float>(),  reg_shape<512, 64, 4, float>(),
+      reg_shape<256, 10, 8, double>(), reg_shape<256, 18, 8, double>(),
+      reg_shape<256, 32, 8, double>(), reg_shape<256, 20, 4, double>(),
+      reg_shape<256, 36, 4, double>(), reg_shape<256, 64, 4, double>(),
+      reg_shape<256, 40, 2, double>(), reg_shape<256, 72, 2, double>()};
+  const int max_p = dev->num_sms < MAX_P ? dev->num_sms : MAX_P;
+  for (int i = fp32 ? 0 : F32_SHAPES; i < (fp32 ? F32_SHAPES : N_SHAPES); ++i) {
+    const RegShape& sh = shapes[i];
+    const int hold = (s.N + sh.cols - 1) / sh.cols;
+    if (s.mY > sh.rows || hold > max_p) continue;
+    // CTAs: in FP32 as few as hold the columns (the stage is latency, and
+    // fewer headers are polled); in FP64 one per 16 columns, up to one per
+    // SM: the FP64 work of its columns is what a stage costs a CTA (2000
+    // columns of 74 rows: 16 a CTA 9.1 ms a factorization, 32 9.8).
+    int P = fp32 ? hold : (s.N + 15) / 16;
+    if (P > max_p) P = max_p;
+    if (P < hold) P = hold;
+    RegArgs a;
+    a.mY = s.mY;
+    a.N = s.N;
+    a.b = s.b;
+    a.Y = s.Y;
+    a.ldy = s.ldy;
+    a.pairs = s.pairs;
+    a.npairs = s.npairs;
+    a.max_pairs = s.max_pairs;
+    a.hdrs = static_cast<unsigned char*>(xch);
+    a.recs = a.hdrs + (size_t)2 * MAX_P * MAX_P * 16;
+    a.tag0 = *tag;
+    *tag += (unsigned)s.b;
+    a.err = s.err;
+    a.spin_limit = s.spin_limit;
+    const int z = hq_zero_words(stream, s.npairs, 1, nullptr, 0);
+    if (z) return z;
+    void* args[] = {&a};
+    const cudaError_t e = hq_launch_coop(sh.fn, dim3(P), dim3(sh.threads), args, 0, stream);
+    hq_count_launches(1);
+    return (int)e;
+  }
+  return (int)cudaErrorNotSupported;
+}
+
 extern "C" int hq_skinny_qrp(cudaStream_t stream, const hq_device_info* dev, int mY, int N,
                              int b, const double* Y, int ldy, double* V, int ldv, int* pairs,
-                             int* npairs, double* part, size_t part_elems, unsigned* bar,
-                             int* err, unsigned spin_limit, int fp32) {
+                             int* npairs, double* part, size_t part_elems, void* xch,
+                             unsigned* tag, unsigned* bar, int* err, unsigned spin_limit,
+                             int fp32) {
   if (mY > HQ_MAX_MY || b > mY || b > N || b <= 0) return (int)cudaErrorInvalidValue;
   SkArgs a;
   a.mY = mY;
@@ -643,14 +833,11 @@ extern "C" int hq_skinny_qrp(cudaStream_t stream, const hq_device_info* dev, int
   a.bar = bar;
   a.err = err;
   a.spin_limit = spin_limit;
-  // The register kernel holds up to NT / 2 columns per CTA; with as few CTAs
-  // as that allows, each stage's grid barrier has fewer arrivals to wait for
-  // (the per-column arithmetic, and so the pivots, do not depend on the
-  // partition).  The shared-memory kernel keeps one CTA per 16 columns up to
-  // one per SM.
-  const int p_reg = (N + NT / 2 - 1) / (NT / 2);
-  const bool reg_fit = mY <= 2 * 72 && p_reg <= dev->num_sms && p_reg <= 160;
-  const int P = reg_fit ? (p_reg < 1 ? 1 : p_reg) : skinny_grid(dev, N);
+  const int reg = launch_reg(stream, dev, a, xch, tag, fp32);
+  if (reg != (int)cudaErrorNotSupported) return reg;
+  // More columns than the registers of the grid hold: the shared-memory
+  // kernel, one CTA per 16 columns up to one per SM.
+  const int P = skinny_grid(dev, N);
   if ((size_t)2 * P * a.rec > part_elems) return (int)cudaErrorInvalidValue;
   a.nloc_max = (N + P - 1) / P;
   a.ldxs = mY | 1;
@@ -666,24 +853,13 @@ extern "C" int hq_skinny_qrp(cudaStream_t stream, const hq_device_info* dev, int
     smem = fixed;
     if (V == nullptr || smem > dev->smem_optin) return (int)cudaErrorInvalidValue;
   }
-  cudaError_t e;
   const int z = hq_zero_words(stream, bar, 1, npairs, 1);
   if (z) return z;
   void* args[] = {&a};
-  const void* fn = nullptr;
-  const bool reg_ok = a.nloc_max <= NT / 2 && P <= 160;  // 5 records per lane in the winner pick
-  if (reg_ok && mY <= 2 * 40)
-    fn = fp32 ? (const void*)skinny_qrp_reg_kernel<40, float> : (const void*)skinny_qrp_reg_kernel<40, double>;
-  else if (reg_ok && mY <= 2 * 72)
-    fn = fp32 ? (const void*)skinny_qrp_reg_kernel<72, float> : (const void*)skinny_qrp_reg_kernel<72, double>;
-  if (fn != nullptr) {
-    e = hq_launch_coop(fn, dim3(P), dim3(NT), args, 0, stream);
-  } else {
-    e = cudaFuncSetAttribute(skinny_qrp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    e = hq_launch_coop((const void*)skinny_qrp_kernel, dim3(P), dim3(NT), args, smem, stream);
-  }
+  cudaError_t e = cudaFuncSetAttribute(skinny_qrp_kernel,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return (int)e;
+  e = hq_launch_coop((const void*)skinny_qrp_kernel, dim3(P), dim3(NT), args, smem, stream);
   hq_count_launches(1);
   return (int)e;
 }
