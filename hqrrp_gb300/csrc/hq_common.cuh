@@ -182,24 +182,81 @@ __device__ __forceinline__ HqReflector hq_make_reflector(double alpha, double xn
   return r;
 }
 
+// f 2^k for a positive FP32 normal f, as an FP64 assembled from the bits (the
+// result must be in the FP64 normal range).
+__device__ __forceinline__ double hq_f32_2k(float f, int k) {
+  const unsigned b = __float_as_uint(f);
+  return __longlong_as_double((long long)((unsigned long long)((int)(b >> 23) + 896 + k) << 52 |
+                                          (unsigned long long)(b & 0x7FFFFFu) << 29));
+}
+
 // The same reflector from alpha and q = ||x||^2 (the tail's sum of squares).
-// Away from under/overflow, beta = -sign(alpha) sqrt(alpha^2 + q) takes one
-// square root and tau and the scale are two independent divisions -- a short
-// dependency chain, which matters where FP64 latency sits on a critical path;
-// beta agrees with DLAPY2's value to an ulp.  Near the range limits it falls
-// back to the careful form above.
+// Away from under/overflow, with t = alpha^2 + q, b = sqrt(t): beta =
+// -sign(alpha) b, tau = 1 + |alpha| / b and scale = sign(alpha) / (|alpha| + b).
+// The chain sits on every stage's critical path, and an FP64 instruction takes
+// 64 clocks here whatever the active lanes, so square root and reciprocals
+// start from the FP32 functions' values and take the fewest FP64
+// instructions that reach full accuracy: one third-order step (Halley's for
+// 1/sqrt; e + e^2 for the reciprocal), then one Newton correction on the
+// residual each -- 17 FP64 instructions in all.  (A square root alone measured
+// 662 clocks, a division 417.)  Near the range limits it falls back to the
+// careful form above.
 __device__ __forceinline__ HqReflector hq_make_reflector_sq(double alpha, double q) {
-  if (q == 0.0) return hq_make_reflector(alpha, 0.0);
+  if ((__double_as_longlong(q) << 1) == 0) return hq_make_reflector(alpha, 0.0);
   const double t = fma(alpha, alpha, q);
-  if (t >= 1e-280 && t <= 1e280) {
-    HqReflector r;
-    const double beta = -copysign(sqrt(t), alpha);
-    r.tau = (beta - alpha) / beta;
-    r.scale = 1.0 / (alpha - beta);
-    r.beta = beta;
-    return r;
-  }
-  return hq_make_reflector(alpha, sqrt(q));
+  const long long tb = __double_as_longlong(t);
+  const int ex = (int)(tb >> 52);  // t's exponent field; its sign is + or t is NaN
+  if (ex < 93 || ex > 1953) return hq_make_reflector(alpha, sqrt(q));  // outside 2^+-930
+  // y ~ 1 / sqrt(t): t = m 4^h, m in [1, 4).
+  const int h = (ex - 1023) >> 1;
+  const float m = __uint_as_float((unsigned)(ex - 1023 - 2 * h + 127) << 23 |
+                                  (unsigned)(tb >> 29 & 0x7FFFFF));
+  double y = hq_f32_2k(rsqrtf(m), -h);
+  double e = fma(-(t * y), y, 1.0);
+  y = fma(y, e * fma(0.375, e, 0.5), y);
+  double b = t * y;
+  const double half_y = __longlong_as_double(__double_as_longlong(y) - (1LL << 52));
+  b = fma(fma(-b, b, t), half_y, b);
+  y = fma(y, fma(-b, y, 1.0), y);  // 1 / b
+  const double aa = fabs(alpha), d = aa + b;
+  // r = 1 / d, d = m2 2^k2.
+  const long long db = __double_as_longlong(d);
+  const int k2 = (int)(db >> 52) - 1023;
+  const float m2 = __uint_as_float(127u << 23 | (unsigned)(db >> 29 & 0x7FFFFF));
+  double r = hq_f32_2k(__frcp_rn(m2), -k2);
+  e = fma(-d, r, 1.0);
+  r = fma(r, fma(e, e, e), r);
+  r = fma(r, fma(-d, r, 1.0), r);
+  HqReflector o;
+  o.tau = fma(aa, y, 1.0);
+  o.beta = -copysign(b, alpha);
+  o.scale = copysign(r, alpha);
+  return o;
+}
+
+// Words that carry a tag or a count beside their value, exchanged between CTAs
+// without fences: 64- and 128-bit scalar accesses, which are single-copy
+// atomic.
+__device__ __forceinline__ void hq_st_word(void* p, unsigned long long lo, unsigned long long hi) {
+  asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], t;\n}" ::"l"(p),
+               "l"(lo), "l"(hi)
+               : "memory");
+}
+__device__ __forceinline__ void hq_ld_word(const void* p, unsigned long long& lo,
+                                           unsigned long long& hi) {
+  asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}"
+               : "=l"(lo), "=l"(hi)
+               : "l"(p)
+               : "memory");
+}
+__device__ __forceinline__ void hq_st_word(void* p, unsigned long long v) {
+  asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ void hq_ld_word(const void* p, unsigned long long& v) {
+  asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+}
+__device__ __forceinline__ void hq_red_word(void* p, unsigned long long v) {
+  asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
 // LAPACK's tol3z = sqrt(dlamch('Epsilon')) with eps = 2^-53.

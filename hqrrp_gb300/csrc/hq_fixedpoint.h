@@ -100,8 +100,17 @@ HQ_FX_HD int hq_fx_split(double t, int ue, unsigned long long p[3], int* first) 
   return 1;
 }
 
-/* The value of the summed words (carries normalised in integers, then two
- * FMAs: within an ulp of the exact sum). */
+HQ_FX_HD int hq_fx_clz(unsigned long long x) {
+#if defined(__CUDA_ARCH__)
+  return __clzll((long long)x);
+#else
+  return __builtin_clzll(x);
+#endif
+}
+
+/* The value of the summed words, rounded to nearest (ties to even), in
+ * integer arithmetic: on this GPU an FP64 instruction costs as much as dozens
+ * of integer ones, and every CTA converts every column's sum. */
 HQ_FX_HD double hq_fx_combine(long long l0, long long l1, long long l2, int ue) {
   long long c = l0 >> 48; /* arithmetic shift: floor */
   l0 -= c * (1LL << 48);
@@ -109,9 +118,44 @@ HQ_FX_HD double hq_fx_combine(long long l0, long long l1, long long l2, int ue) 
   c = l1 >> 48;
   l1 -= c * (1LL << 48);
   l2 += c;
-  const double two48 = 281474976710656.0;
-  const double hi = fma((double)l2, two48, (double)l1);
-  return scalbn(fma(hi, two48, (double)l0), ue);
+  /* Two's complement over 160 bits: A2 (weight 2^128, sign) A1 A0. */
+  const int neg = l2 < 0;
+  unsigned long long A0 = (unsigned long long)l0 | ((unsigned long long)l1 << 48);
+  unsigned long long A1 = ((unsigned long long)l1 >> 16) | ((unsigned long long)l2 << 32);
+  unsigned long long A2 = (unsigned long long)(l2 >> 32);
+  if (neg) { /* magnitude */
+    A0 = ~A0 + 1ull;
+    A1 = ~A1 + (A0 == 0ull);
+    A2 = ~A2 + (A0 == 0ull && A1 == 0ull);
+  }
+  /* Left-justify the top 64 bits in H; sticky: anything below them. */
+  int base = 128;
+  unsigned long long H = A2, L = A1, R = A0;
+  if (H == 0ull) {
+    base = 64;
+    H = A1;
+    L = A0;
+    R = 0ull;
+    if (H == 0ull) {
+      base = 0;
+      H = A0;
+      L = 0ull;
+      if (H == 0ull) return 0.0;
+    }
+  }
+  const int z = hq_fx_clz(H);
+  const unsigned long long rest = z ? (L << z) : L;
+  if (z) H = (H << z) | (L >> (64 - z));
+  const unsigned long long sticky = (rest | R) != 0ull;
+  unsigned long long M = H >> 11;
+  const unsigned long long low = (H & 0x7FFull) << 1 | sticky;
+  M += low > 0x800ull || (low == 0x800ull && (M & 1ull)); /* half is 0x400 << 1 */
+  const int e = base + 63 - z + ue + 1023; /* of the leading bit, biased */
+  if (e > 0 && e < 2046) /* M's bit 52 (53 after a carry) adds one to e - 1 */
+    return hq_fx_double((long long)((neg ? 1ull << 63 : 0ull) +
+                                    ((unsigned long long)(e - 1) << 52) + M));
+  const double v = scalbn((double)M, e - 1023 - 52);
+  return neg ? -v : v;
 }
 
 #endif /* HQ_FIXEDPOINT_H */

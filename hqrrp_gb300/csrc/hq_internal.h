@@ -70,17 +70,14 @@ size_t hq_skinny_part_elems(const hq_device_info* dev, int mY);
  * tau[0..nc), U (mp x nc, ldu) = explicit unit-lower copy of the vectors,
  * perm[k] = source column of final column k. */
 int hq_panel_qrp(cudaStream_t stream, const hq_device_info* dev, int mp, int nc, int pivoting,
-                 double* P, int ldp, double* tau, double* U, int ldu,
-                 int* perm, double* part, size_t part_elems, double* rowbuf, unsigned* bar,
-                 int* err, unsigned spin_limit,
-                 int sqnorm, int ut);
+                 double* P, int ldp, double* tau, double* U, int ldu, int* perm, double* part,
+                 size_t part_elems, unsigned* bar, int* err, unsigned spin_limit, int ut);
 /* The same, skipped (every CTA returns at once) when *gram_stat == 0: the
  * mixed path's Gram panel (qrp_gram.cu) already factored this panel. */
 int hq_panel_qrp_fallback(cudaStream_t stream, const hq_device_info* dev, int mp, int nc,
                           int pivoting, double* P, int ldp, double* tau, double* U, int ldu,
-                          int* perm, double* part, size_t part_elems, double* rowbuf,
-                          unsigned* bar, int* err, unsigned spin_limit, int sqnorm, int ut,
-                          const int* gram_stat);
+                          int* perm, double* part, size_t part_elems, unsigned* bar, int* err,
+                          unsigned spin_limit, int ut, const int* gram_stat);
 size_t hq_panel_part_elems(const hq_device_info* dev, int nc);
 
 /* ---- Gram panel (mixed path): the b x b kernels of qrp_gram.cu -----------
@@ -130,14 +127,16 @@ int hq_gram_commit(cudaStream_t stream, int mp, int n, double* P, int ldp, doubl
                    double* tau, int* perm, const int* stat, int* count);
 /* Exchange area of the panel kernel for `ctas` CTAs and nc columns, in
  * doubles: [2][ps][ctas] FP64 partials (initial and recomputed norms), then
- * [3][ps][HQ_PANEL_FX_CS] 64-bit words of fixed-point stage sums (four used
+ * [2][R][ps][HQ_PANEL_FX_CS] 64-bit words of fixed-point stage sums (three used
  * per column; the stride spreads the columns' atomics over cache lines,
- * which measured 13 ms faster per 16384^2 factorization than packed words);
- * ps = nc rounded up to even (plus 2). */
-#define HQ_PANEL_FX_CS 16 /* one 128-byte line per column: fewer atomics per line */
+ * which measured 13 ms faster per 16384^2 factorization than packed words),
+ * then [2][ps][2] words of tagged row entries; ps = nc rounded up to even
+ * (plus 2).  R: words a column's adds are spread over. */
+#define HQ_PANEL_FX_CS 16 /* one 128-byte line per column and word set */
+#define HQ_PANEL_R(nc) ((nc) <= 128 ? 4 : 2)
 #define HQ_PANEL_PART_ELEMS(ctas, nc) \
-  (2 * (size_t)(ctas) * (size_t)(((nc) + 2) & ~1) + \
-   3 * (size_t)HQ_PANEL_FX_CS * (size_t)(((nc) + 2) & ~1))
+  ((2 * (size_t)(ctas) + 2 * (size_t)HQ_PANEL_R(nc) * HQ_PANEL_FX_CS + 4) * \
+   (size_t)(((nc) + 2) & ~1))
 
 /* ---- Wide pivoted QR: m <= HQ_WIDE_MAX_ROWS rows, any number of columns --
  * dgeqp3's result for an m x n matrix A (lda), in place except for the

@@ -187,7 +187,7 @@ typedef struct {
   int nalloc; /* allocations attempted by this call */
   int failed;
   /* HQRRP buffers */
-  double *G, *Y, *V, *U, *T, *Z, *W1, *W2, *Bm, *B2, *ws, *part, *rowbuf, *tmp;
+  double *G, *Y, *V, *U, *T, *Z, *W1, *W2, *Bm, *B2, *ws, *part, *tmp;
   int *pairs, *npairs, *perm, *labels, *label_tmp, *err;
   unsigned* bar;
   void* selx;       /* pivot selection's exchange area, and its next stage tag */
@@ -438,7 +438,6 @@ static int ws_setup(hq_ws* w, int m, int n, int nb, int pp, int pw) {
   w->W2 = ws_alloc(w, sizeof(double) * (size_t)w->ldw * imax(n, 1));
   w->ws = ws_alloc(w, sizeof(double) * w->ws_elems);
   w->part = ws_alloc(w, sizeof(double) * w->part_elems);
-  w->rowbuf = ws_alloc(w, sizeof(double) * 2 * (size_t)imax(kmax, 1));
   w->tmp = ws_alloc(w, sizeof(double) * (size_t)w->tmp_rows * w->tmp_cols);
   w->pairs = ws_alloc(w, sizeof(int) * 4 * (size_t)kmax);
   w->npairs = ws_alloc(w, sizeof(int) * 2);
@@ -868,8 +867,6 @@ static int core_hqrrp_k(hq_ws* w, int m, int n, double* dA, int ldda, int* djpvt
 
     NV_PUSH("hqrrp.panel");
     /* Panel QR (pivoted within its b columns), U, tau. */
-    /* Mixed: squared column norms in the panel's pivoting (division-free
-     * LAWN 176 downdate); plain keeps LAPACK's formula. */
     const int use_gram = w->gram && w->gQ && !w->ut && b <= HQ_GRAM_MAX;
     if (use_gram) {
       int rc = gram_panel(w, m, j, b, panel_piv, AR, ldda, djpvt + j, dtau + j,
@@ -877,8 +874,8 @@ static int core_hqrrp_k(hq_ws* w, int m, int n, double* dA, int ldda, int* djpvt
       if (rc) return rc;
     }
     CK(hq_panel_qrp_fallback(w->st, dev, mp, b, panel_piv, ABR, ldda, dtau + j, w->U, w->ldu,
-                             w->perm, w->part, w->part_elems, w->rowbuf, w->bar + 1, w->err,
-                             spin, w->mixed, w->ut, use_gram ? w->gstat : NULL));
+                             w->perm, w->part, w->part_elems, w->bar + 1, w->err, spin, w->ut,
+                             use_gram ? w->gstat : NULL));
     if (w->mixed) CK(hq_set_diag(w->st, b, w->U, w->ldu, 0.0)); /* U' for the digit products */
     /* The panel's swaps on the rows above it and on the labels. */
     CK(hq_permute_cols(w->st, j, AR, ldda, b, w->perm, w->tmp, djpvt + j, w->label_tmp));
@@ -1252,7 +1249,7 @@ static int core_dgeqp4(hq_ws* w, int m, int n, double* dA, int ldda, int* hjp, i
     const int b = imin(FIXED_BLOCK, nf - j), mp = m - j;
     double* ABR = dA + j + (size_t)j * ldda;
     CK(hq_panel_qrp(w->st, dev, mp, b, 0, ABR, ldda, dtau + j, w->U, w->ldu, w->perm, w->part,
-                    w->part_elems, w->rowbuf, w->bar + 1, w->err, spin, 0, 0));
+                    w->part_elems, w->bar + 1, w->err, spin, 0));
     if (w->mixed) CK(hq_set_diag(w->st, b, w->U, w->ldu, 0.0)); /* U' for the digit products */
     int rc = block_reflector(w, mp, b, dtau + j, ABR + (size_t)b * ldda, ldda, n - j - b, NULL,
                              NULL);
@@ -1290,7 +1287,7 @@ static int core_dgeqp4(hq_ws* w, int m, int n, double* dA, int ldda, int* hjp, i
                           wtmp, djp + nf, wlab));
     } else if (small) {
       CK(hq_panel_qrp(w->st, dev, mt, nt, 1, At, ldda, dtau + nf, NULL, w->ldu, w->perm,
-                      w->part, w->part_elems, w->rowbuf, w->bar + 1, w->err, spin, 0, 0));
+                      w->part, w->part_elems, w->bar + 1, w->err, spin, 0));
       CK(hq_permute_cols(w->st, nf, dA + (size_t)nf * ldda, ldda, nt, w->perm, w->tmp,
                          djp + nf, w->label_tmp));
     } else {

@@ -27,17 +27,16 @@
 namespace {
 
 constexpr size_t kPartElems = HQ_PANEL_PART_ELEMS(NOALLOC_MAX_CTAS, NOALLOC_MAX_N);
-constexpr size_t kRowbufElems = 2ull * NOALLOC_MAX_N;
 constexpr size_t kPermElems = NOALLOC_MAX_N / 2;  // NOALLOC_MAX_N ints
 constexpr size_t kFlagElems = 2;                  // barrier counter, error word
-constexpr size_t kScratchElems = kPartElems + kRowbufElems + kPermElems + kFlagElems;
+constexpr size_t kScratchElems = kPartElems + kPermElems + kFlagElems;
 
 // Return codes, the same values as the rest of the library's entry points.
 constexpr int kRcCuda = 1, kRcDevice = 2, kRcUnsupported = 3;
 
 }  // namespace
 
-// 2 x 160 x 258 + 48 x 258 + 512 + 128 + 2 doubles = 764,688 bytes (747 KiB)
+// (2 x 160 + 2 x 2 x 16 + 4) x 258 + 128 + 2 doubles = 801,872 bytes (783 KiB)
 // per GPU.
 static __device__ __align__(256) double hq_noalloc_scratch[kScratchElems];
 
@@ -103,15 +102,14 @@ extern "C" __attribute__((visibility("default"))) int hqrrp_gb300_qrp_noalloc(
     return kRcCuda;
   }
   double* part = base;
-  double* rowbuf = part + kPartElems;
-  int* perm = reinterpret_cast<int*>(rowbuf + kRowbufElems);
-  unsigned* bar = reinterpret_cast<unsigned*>(rowbuf + kRowbufElems + kPermElems);
+  int* perm = reinterpret_cast<int*>(part + kPartElems);
+  unsigned* bar = reinterpret_cast<unsigned*>(part + kPartElems + kPermElems);
   int* err = reinterpret_cast<int*>(bar + 1);
 
   rc = (int)cudaMemsetAsync(err, 0, sizeof(int), st);
   if (rc == 0)
     rc = hq_panel_qrp(st, &dev, m, n, 1, dA, ldda, d_tau, nullptr, 1, perm, part, kPartElems,
-                      rowbuf, bar, err, hq_spin_limit(), 0, 0);
+                      bar, err, hq_spin_limit(), 0);
   if (rc == 0) {
     labels_from_perm<<<(n + 255) / 256, 256, 0, st>>>(perm, n, d_jpvt);
     hq_count_launches(1);

@@ -323,26 +323,6 @@ struct RegArgs {
 constexpr int MAX_P = 160;               // CTAs
 constexpr int HDR_LANE = MAX_P / 32;     // headers per polling lane
 
-__device__ __forceinline__ void st_word(unsigned char* p, unsigned long long lo,
-                                        unsigned long long hi) {
-  asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], t;\n}" ::"l"(p),
-               "l"(lo), "l"(hi)
-               : "memory");
-}
-__device__ __forceinline__ void ld_word(const unsigned char* p, unsigned long long& lo,
-                                        unsigned long long& hi) {
-  asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}"
-               : "=l"(lo), "=l"(hi)
-               : "l"(p)
-               : "memory");
-}
-__device__ __forceinline__ void st_word(unsigned char* p, unsigned long long v) {
-  asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-__device__ __forceinline__ void ld_word(const unsigned char* p, unsigned long long& v) {
-  asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-}
-
 // One entry of a published column and its tag: 8 bytes in FP32, 16 in FP64.
 template <typename T>
 struct Tagged;
@@ -350,11 +330,11 @@ template <>
 struct Tagged<float> {
   static constexpr int BYTES = 8;
   static __device__ __forceinline__ void put(unsigned char* p, float x, unsigned tag) {
-    st_word(p, ((unsigned long long)tag << 32) | __float_as_uint(x));
+    hq_st_word(p, ((unsigned long long)tag << 32) | __float_as_uint(x));
   }
   static __device__ __forceinline__ bool get(const unsigned char* p, unsigned tag, float& x) {
     unsigned long long v;
-    ld_word(p, v);
+    hq_ld_word(p, v);
     x = __uint_as_float((unsigned)v);
     return (unsigned)(v >> 32) == tag;
   }
@@ -363,11 +343,11 @@ template <>
 struct Tagged<double> {
   static constexpr int BYTES = 16;
   static __device__ __forceinline__ void put(unsigned char* p, double x, unsigned tag) {
-    st_word(p, (unsigned long long)__double_as_longlong(x), tag);
+    hq_st_word(p, (unsigned long long)__double_as_longlong(x), tag);
   }
   static __device__ __forceinline__ bool get(const unsigned char* p, unsigned tag, double& x) {
     unsigned long long lo, hi;
-    ld_word(p, lo, hi);
+    hq_ld_word(p, lo, hi);
     x = __longlong_as_double((long long)lo);
     return hi == tag;
   }
@@ -503,7 +483,7 @@ __global__ void __launch_bounds__(CNT, 1) skinny_qrp_reg_kernel(RegArgs a) {
 #pragma unroll
       for (int j = 0; j < HDR_LANE; ++j) {
         const int q = lane + 32 * j;
-        if (32 * j < P && q < P) st_word(h + (size_t)q * MAX_P * 16, (unsigned long long)k, w1);
+        if (32 * j < P && q < P) hq_st_word(h + (size_t)q * MAX_P * 16, (unsigned long long)k, w1);
       }
       if (mine) {
         unsigned char* rec = a.recs + ((size_t)(s & 1) * MAX_P + cta) * rec_bytes;
@@ -537,7 +517,7 @@ __global__ void __launch_bounds__(CNT, 1) skinny_qrp_reg_kernel(RegArgs a) {
           pp[j] = 0x7fffffff;
           if (32 * j < P && q < P) {
             unsigned long long k0, w;
-            ld_word(h0 + (size_t)q * 16, k0, w);
+            hq_ld_word(h0 + (size_t)q * 16, k0, w);
             kk[j] = (long long)k0;
             pp[j] = (int)(unsigned)w;
             ok = ok && (unsigned)(w >> 32) == tag;
