@@ -209,14 +209,19 @@ int hq_ozk_gemm_short(cudaStream_t stream, const hq_device_info* dev, int M, int
                       int mode, double sign, double* C, long long crs, long long ccs,
                       int* colexp, int row_lo, int* err, unsigned spin_limit);
 
-/* ---- Batched pivoted QR (one persistent launch, device work queue) -------
+/* ---- Batched pivoted QR (one persistent launch, device work queues) ------
  * d_work: hq_qrp_batched_workspace(batch) bytes; ints [32..32+batch) hold the
- * schedule (matrix indices, largest first), int 0 the queue head. */
+ * schedule (matrix indices, largest first), ints 0 and 1 the queue heads, int
+ * HQ_BATCHED_TEAM_SLOT + c, c = ctas_per_sm < 8, how many of the schedule's
+ * first matrices (none of more than HQ_BATCHED_TEAM_ROWS rows) go to teams of
+ * `team` CTAs when team > 1. */
+#define HQ_BATCHED_TEAM_SLOT 8
+#define HQ_BATCHED_TEAM_ROWS 1024
 size_t hq_qrp_batched_workspace(int batch);
 int hq_qrp_batched(cudaStream_t stream, const hq_device_info* dev, int batch, const int* d_m,
                    const int* d_n, double* const* d_A, const int* d_lda, int* const* d_jpvt,
                    double* const* d_tau, int* d_info, void* d_work, int max_n, int threads,
-                   int stage_kb, int ctas_per_sm);
+                   int stage_kb, int ctas_per_sm, int team);
 
 /* ---- Adjoint helpers (adjoint.cu) ---- */
 int hq_unit_lower(cudaStream_t st, int rows, int b, const double* F, int ldf, double* U, int ldu);

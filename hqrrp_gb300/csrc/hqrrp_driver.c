@@ -1493,14 +1493,17 @@ HQ_API int hqrrp_gb300_ozaki_dgemm(char transa, char transb, int m, int n, int k
 
 typedef struct {
   int threads, stage_kb, ctas_per_sm;
+  int team; /* CTAs per cluster: the largest matrices are shared by that many */
 } batched_cfg;
 
 /* Launch shapes the autotuner tries: threads per CTA, shared-memory staging
- * budget for a matrix (KB; larger matrices are worked on in place in L2),
- * CTAs per SM. */
+ * budget for a matrix (KB), CTAs per SM, team.  Small budgets: what shared
+ * memory leaves of the 256 KB serves as L1 for the matrices worked on in
+ * place, which are most of the work (4096 matrices of the benchmark, 256
+ * threads, teams of two: 32 KB 106 ms, 64 KB 113, 96 KB 147). */
 static const batched_cfg g_batched_cfgs[] = {
-    {128, 0, 4},   {128, 48, 4}, {256, 0, 2},  {256, 96, 2},
-    {256, 200, 1}, {512, 96, 2}, {512, 200, 1},
+    {128, 48, 4, 1}, {256, 32, 2, 1}, {512, 64, 1, 1}, {256, 32, 2, 2},
+    {256, 32, 2, 4}, {512, 64, 1, 2}, {256, 64, 2, 8},
 };
 #define N_BATCHED_CFGS ((int)(sizeof g_batched_cfgs / sizeof g_batched_cfgs[0]))
 
@@ -1579,12 +1582,12 @@ static int autotune_batched(hq_ws* w, int batch, const int* h_m, const int* h_n,
       float ms = 0.f;
       int rc = hq_qrp_batched(w->st, &w->ds->dev, batch, dm, dn, (double* const*)dptr, dl,
                               (int* const*)(dptr + batch), (double* const*)(dptr + 2 * batch),
-                              NULL, d_work, max_n, k->threads, k->stage_kb, k->ctas_per_sm);
+                              NULL, d_work, max_n, k->threads, k->stage_kb, k->ctas_per_sm, k->team);
       if (rc) continue; /* shape does not fit this device: skip it */
       cudaEventRecord(e0, w->st);
       rc = hq_qrp_batched(w->st, &w->ds->dev, batch, dm, dn, (double* const*)dptr, dl,
                           (int* const*)(dptr + batch), (double* const*)(dptr + 2 * batch), NULL,
-                          d_work, max_n, k->threads, k->stage_kb, k->ctas_per_sm);
+                          d_work, max_n, k->threads, k->stage_kb, k->ctas_per_sm, k->team);
       cudaEventRecord(e1, w->st);
       if (rc || cudaStreamSynchronize(w->st) != cudaSuccess) continue;
       cudaEventElapsedTime(&ms, e0, e1);
@@ -1615,6 +1618,9 @@ HQ_API int hqrrp_gb300_qrp_batched_plan(int batch, const int* h_m, const int* h_
   }
   int max_n = 1;
   double total = 0.0;
+  dev_state* ds = current_device();
+  if (!ds) return -HQ_E_CUDA;
+  const double sms = (double)ds->dev.num_sms;
   cost_idx* ord = malloc(sizeof(cost_idx) * (size_t)batch);
   int* hord = malloc(sizeof(int) * (size_t)batch);
   if (!ord || !hord) {
@@ -1636,13 +1642,30 @@ HQ_API int hqrrp_gb300_qrp_batched_plan(int batch, const int* h_m, const int* h_
     if (h_n[i] > max_n) max_n = h_n[i];
   }
   qsort(ord, (size_t)batch, sizeof(cost_idx), cost_desc);
-  for (int i = 0; i < batch; ++i) hord[i] = ord[i].idx;
+  /* The teams' share, by CTAs per SM (a CTA has that part of its SM's FP64
+   * rate): the largest matrices, as long as a single CTA would take over a
+   * quarter of what the whole batch takes on all SMs (batches of 1024 and 4096
+   * from all to a quarter: 35 -> 30 and 126 -> 111 ms), and the matrix is
+   * large enough (16384 entries) that a stage's FP64 work outweighs the team's
+   * exchange. */
+  int n_team[8] = {0};
+  for (int i = 0; i < batch; ++i) {
+    const int id = ord[i].idx;
+    hord[i] = id;
+    for (int c = 1; c < 8; ++c)
+      if (n_team[c] == i && 4.0 * c * ord[i].cost * sms > total &&
+          h_m[id] <= HQ_BATCHED_TEAM_ROWS && (double)h_m[id] * h_n[id] >= 16384.0)
+        ++n_team[c];
+  }
   free(ord);
   hq_ws w;
   int rc = ws_begin(&w, (cudaStream_t)stream, 1);
   if (!rc) {
     int e = (int)cudaMemcpyAsync((int*)d_work + 32, hord, sizeof(int) * batch,
                                  cudaMemcpyHostToDevice, w.st);
+    if (!e)
+      e = (int)cudaMemcpyAsync((int*)d_work + HQ_BATCHED_TEAM_SLOT, n_team, sizeof n_team,
+                               cudaMemcpyHostToDevice, w.st);
     if (!e) e = (int)cudaStreamSynchronize(w.st);
     if (e) {
       set_err("schedule upload failed: %s", cudaGetErrorString((cudaError_t)e));
@@ -1651,7 +1674,8 @@ HQ_API int hqrrp_gb300_qrp_batched_plan(int batch, const int* h_m, const int* h_
   }
   free(hord);
   if (rc) return -rc;
-  int cfg = 3; /* 256 threads, 96 KB staging, 2 CTAs per SM */
+  /* 256 threads, 32 KB staging, 2 CTAs per SM; teams of four where they have work. */
+  int cfg = n_team[2] > 0 ? 4 : 1;
   if (autotune) {
     for (int i = 0; i < g_ntuned; ++i)
       if (g_tuned[i].batch == batch && g_tuned[i].max_n == max_n && g_tuned[i].cost == total)
@@ -1685,7 +1709,7 @@ HQ_API int hqrrp_gb300_qrp_batched_run(int batch, const int* d_m, const int* d_n
   if (!ds) return HQ_E_CUDA;
   const batched_cfg* k = &g_batched_cfgs[cfg];
   int rc = hq_qrp_batched((cudaStream_t)stream, &ds->dev, batch, d_m, d_n, d_A, d_lda, d_jpvt,
-                          d_tau, d_info, d_work, max_n, k->threads, k->stage_kb, k->ctas_per_sm);
+                          d_tau, d_info, d_work, max_n, k->threads, k->stage_kb, k->ctas_per_sm, k->team);
   if (rc) {
     set_err("batched launch failed: %s", cudaGetErrorString((cudaError_t)rc));
     return HQ_E_CUDA;

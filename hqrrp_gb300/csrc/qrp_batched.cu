@@ -4,14 +4,35 @@
 // dgeqp4 hands every matrix with min(m, n) < 1000 to LAPACK's dgeqpf / dgeqp3
 // (lapack_compatible_sources/NoFLA_HQRRP_WY_blk_var4.c:189-199); both produce
 // the Businger-Golub column-pivoted Householder QR with LAWN 176 norm
-// downdating, the algorithm restated per matrix here (one CTA per matrix).
-// A batch is scheduled through a device work queue: the host orders the
-// matrices by cost (largest first), and each resident CTA takes the next
-// index with an atomic until the queue is empty, so uneven sizes balance
-// across the SMs.  A matrix is staged in shared memory when it fits in the
-// launch's staging budget and worked on in place (L2-resident) otherwise.
-// The launch shape -- threads per CTA and the staging budget -- is chosen by
-// the host autotuner (hqrrp_driver.c) per batch signature.
+// downdating, the algorithm restated per matrix here.  A batch is scheduled
+// through device work queues: the host orders the matrices by cost (largest
+// first), and whoever is free takes the next index with an atomic until the
+// queue is empty, so uneven sizes balance across the SMs.
+//
+// One SM runs 2 FP64 FMAs per clock, so a 1024 x 512 matrix alone holds it for
+// 55 ms and bounds a batch of any size.  The launch is therefore made of
+// clusters of T CTAs (T = 1, 2, 4 or 8, part of the launch shape).  The
+// largest matrices go through a first queue to whole clusters, columns dealt
+// out cyclically; the CTAs then take the rest one by one from a second queue.
+// In a team, every CTA pushes its best candidate into the shared memory of the
+// others, one cluster barrier per stage, and each reads the winning column
+// from its owner -- shared memory over the cluster's network, or L2 -- and
+// builds the reflector itself.
+//
+// Columns never move: a pivot is bookkeeping (each column's position), and the
+// final order is made once, on the way out.  A matrix is staged in shared
+// memory when its CTA's columns fit the launch's staging budget and worked on
+// in place (L2-resident) otherwise.  FP64 instructions are the time (an SM
+// issues one per 16 clocks), so a warp takes four columns together: their dot
+// products' partial sums are reduced by six additions instead of twenty, and
+// norms are kept squared, without divisions or square roots, one thread per
+// column.
+//
+// The launch shape -- threads per CTA, the staging budget, T -- is chosen by
+// the host autotuner (hqrrp_driver.c) per batch signature.  Measured on GB300
+// against one CTA per matrix, swapped columns and a column per warp: 1024
+// matrices of the benchmark's sizes 90 -> 29 ms (FP64 alone: 16), 4096 of them
+// 139 -> 107 (63).
 //
 // All columns are free (LAPACK jpvt = 0 input); on return jpvt[k] is the
 // 1-based original index of column k, tau[0..min(m,n)) the reflector scalars,
@@ -19,6 +40,9 @@
 #include "hq_common.cuh"
 
 namespace {
+
+constexpr int T_MAX = 8;        // CTAs per cluster (the portable limit)
+constexpr int TEAM_ROWS = HQ_BATCHED_TEAM_ROWS;  // rows of a matrix a team takes
 
 struct BatchArgs {
   int batch;
@@ -29,218 +53,558 @@ struct BatchArgs {
   int* const* jpvt;
   double* const* tau;
   int* info;
-  const int* order;  // schedule: matrix indices, largest first
-  int* next;         // queue head (zeroed before the launch)
-  int stage_bytes;   // dynamic shared memory available for staging a matrix
+  const int* order;   // schedule: matrix indices, largest first
+  int* next;          // queue heads: [0] single CTAs, [1] teams (zeroed before the launch)
+  const int* n_team;  // the first *n_team of the schedule are the teams' (T > 1)
+  int stage_bytes;    // dynamic shared memory available for staging a matrix
   int max_n;
 };
 
+__device__ __forceinline__ unsigned cluster_rank() {
+  unsigned r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ unsigned cluster_size() {
+  unsigned r;
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+// Every thread of every CTA of the cluster; what was written before, to any of
+// the cluster's shared memories or to global memory, is read after.
+__device__ __forceinline__ void cluster_barrier() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::
+                   : "memory");
+}
+__device__ __forceinline__ unsigned cluster_addr(const void* smem, unsigned rank) {
+  unsigned r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((unsigned)__cvta_generic_to_shared(smem)), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void cluster_st(unsigned addr, long long a, long long b) {
+  asm volatile("st.shared::cluster.v2.b64 [%0], {%1, %2};" ::"r"(addr), "l"(a), "l"(b) : "memory");
+}
+__device__ __forceinline__ double cluster_ld(unsigned addr) {
+  double v;
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(addr) : "memory");
+  return v;
+}
+
+// Larger key first, then the lower position (the upper word of at).
+__device__ __forceinline__ bool better(long long k1, long long at1, long long k2, long long at2) {
+  return k1 > k2 || (k1 == k2 && at1 < at2);
+}
+
+// Sums over the lanes of NY values per lane, in the lanes [32 / NY c, 32 / NY
+// (c + 1)) for value c: each halving of the lanes that share a value also
+// halves the values a lane keeps, so four take 2 + 1 + 3 additions.
+template <int NY>
+__device__ __forceinline__ double lanes_sum(const double (&d)[NY], int lane) {
+  double t;
+  if constexpr (NY == 4) {
+    const bool up = lane & 16;
+    const double a = (up ? d[2] : d[0]) + __shfl_xor_sync(0xffffffffu, up ? d[0] : d[2], 16);
+    const double b = (up ? d[3] : d[1]) + __shfl_xor_sync(0xffffffffu, up ? d[1] : d[3], 16);
+    const bool up8 = lane & 8;
+    t = (up8 ? b : a) + __shfl_xor_sync(0xffffffffu, up8 ? a : b, 8);
+  } else if constexpr (NY == 2) {
+    const bool up = lane & 16;
+    t = (up ? d[1] : d[0]) + __shfl_xor_sync(0xffffffffu, up ? d[0] : d[1], 16);
+    t += __shfl_xor_sync(0xffffffffu, t, 8);
+  } else {
+    t = d[0] + __shfl_xor_sync(0xffffffffu, d[0], 16);
+    t += __shfl_xor_sync(0xffffffffu, t, 8);
+  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  return t;
+}
+
+// y_c -= tau (v^T y_c) v over rows s..m-1 for NY columns y_c of one warp; the
+// new entries of row s go to rs[c].  CH > 0: the columns stay in registers
+// between the two uses (at most 32 CH rows); CH = 0: read twice.
+template <int NY, int CH>
+__device__ __forceinline__ void apply_warp(const double* __restrict__ v, double* const (&y)[NY],
+                                           double tau, int s, int m, int lane, double* (&rs)[NY]) {
+  double d[NY];
+#pragma unroll
+  for (int c = 0; c < NY; ++c) d[c] = 0.0;
+  if constexpr (CH > 0) {
+    double x[NY][CH];
+#pragma unroll
+    for (int t = 0; t < CH; ++t) {
+      const int i = s + lane + 32 * t;
+#pragma unroll
+      for (int c = 0; c < NY; ++c) x[c][t] = i < m ? y[c][i] : 0.0;
+    }
+#pragma unroll
+    for (int t = 0; t < CH; ++t) {
+      const int i = s + lane + 32 * t;
+      if (s + 32 * t < m) {  // uniform: no FP64 for rows that are not there
+        const double vi = i < m ? v[i] : 0.0;
+#pragma unroll
+        for (int c = 0; c < NY; ++c) d[c] = fma(vi, x[c][t], d[c]);
+      }
+    }
+    const double t = lanes_sum<NY>(d, lane) * -tau;
+    double w[NY];
+#pragma unroll
+    for (int c = 0; c < NY; ++c) w[c] = __shfl_sync(0xffffffffu, t, 32 / NY * c);
+#pragma unroll
+    for (int t2 = 0; t2 < CH; ++t2) {
+      const int i = s + lane + 32 * t2;
+      if (s + 32 * t2 < m) {
+        const double vi = i < m ? v[i] : 0.0;
+#pragma unroll
+        for (int c = 0; c < NY; ++c) {
+          const double z = fma(vi, w[c], x[c][t2]);
+          if (i < m) y[c][i] = z;
+          if (t2 == 0 && lane == 0) *rs[c] = z;
+        }
+      }
+    }
+  } else {
+#pragma unroll 4
+    for (int i = s + lane; i < m; i += 32) {
+      const double vi = v[i];
+#pragma unroll
+      for (int c = 0; c < NY; ++c) d[c] = fma(vi, y[c][i], d[c]);
+    }
+    const double t = lanes_sum<NY>(d, lane) * -tau;
+    double w[NY];
+#pragma unroll
+    for (int c = 0; c < NY; ++c) w[c] = __shfl_sync(0xffffffffu, t, 32 / NY * c);
+#pragma unroll 4
+    for (int i = s + lane; i < m; i += 32) {
+      const double vi = v[i];
+#pragma unroll
+      for (int c = 0; c < NY; ++c) {
+        const double z = fma(vi, w[c], y[c][i]);
+        y[c][i] = z;
+        if (i == s) *rs[c] = z;
+      }
+    }
+  }
+}
+
+template <int NY, int CH>
+struct Take {
+  static constexpr int ny = NY, ch = CH;
+};
+
 template <int NT>
-__global__ void __launch_bounds__(NT) qrp_batched_kernel(BatchArgs a) {
+__global__ void __launch_bounds__(NT, 512 / NT) qrp_batched_kernel(BatchArgs a) {
   extern __shared__ __align__(16) double smem[];
   constexpr int NW = NT / 32;
-  __shared__ int s_item, s_kp;
-  __shared__ double s_red[NW];
-  __shared__ int s_bk[NW];
+  // FP64 work that is one value per thread goes to four warps, one per quarter
+  // of the SM: more would only queue up for the same pipes.
+  constexpr int ND = 128, NDW = ND / 32;
+  __shared__ __align__(16) long long s_cand[2][T_MAX][2];  // the team's candidates, by stage parity
+  __shared__ __align__(16) long long s_item[2][2];
+  __shared__ double s_red[NDW];
+  __shared__ long long s_bk[NDW], s_at[NDW];
   __shared__ double s_tau, s_scale, s_beta;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  double* sd = smem;                 // partial norms, max_n
-  double* se = sd + a.max_n;         // norms at the last recomputation, max_n
-  double* sw = se + a.max_n;         // spare, max_n
-  int* sperm = (int*)(sw + a.max_n);  // max_n
-  double* sX = (double*)(sperm + ((a.max_n + 1) & ~1));
+  const unsigned rank = cluster_rank();
+  const int T_all = (int)cluster_size();
+  double* sd = smem;                  // squared partial norms of this CTA's columns, max_n
+  double* sthr = sd + a.max_n;        // recompute at or below, max_n
+  double* srs = sthr + a.max_n;       // the stage's new entries of row s, max_n
+  int* spos = (int*)(srs + a.max_n);  // positions, max_n
+  int* sact = spos + a.max_n;         // columns not yet factored, max_n
+  double* sv = srs + 2 * a.max_n;     // a team's reflector, TEAM_ROWS
+  double* sX = sv + (T_all > 1 ? TEAM_ROWS : 0);
 
-  for (;;) {
-    if (tid == 0) {
-      const int q = atomicAdd(a.next, 1);
-      s_item = q < a.batch ? a.order[q] : -1;
+  // Every CTA of the cluster has started before its shared memory is written.
+  if (T_all > 1) cluster_barrier();
+  bool teams = T_all > 1;
+  for (int turn = 0;; ++turn) {
+    // The next matrix: of the teams' queue while it lasts, then of the CTAs'.
+    int item;
+    if (teams) {
+      if (rank == 0 && tid == 0) {
+        const int q = atomicAdd(a.next + 1, 1);
+        const long long it = q < min(*a.n_team, a.batch) ? a.order[q] : -1;
+        for (int r = 0; r < T_all; ++r) cluster_st(cluster_addr(s_item[turn & 1], r), it, 0);
+      }
+      cluster_barrier();
+      item = (int)s_item[turn & 1][0];
+      if (item < 0) {
+        teams = false;
+        continue;
+      }
+    } else {
+      __syncthreads();
+      if (tid == 0) {
+        const int q = atomicAdd(a.next, 1) + (T_all > 1 ? *a.n_team : 0);
+        s_item[turn & 1][0] = q < a.batch ? a.order[q] : -1;
+      }
+      __syncthreads();
+      item = (int)s_item[turn & 1][0];
+      if (item < 0) break;
     }
-    __syncthreads();
-    const int item = s_item;
-    __syncthreads();
-    if (item < 0) break;
+    const int T = teams ? T_all : 1, me = teams ? (int)rank : 0;
     const int m = a.m[item], n = a.n[item], lda = a.lda[item];
     double* Ag = a.A[item];
     // A size the kernel cannot take (negative, lda < max(1, m), more than
     // max_n columns) is flagged and left untouched; an empty matrix is done.
-    const bool bad = m < 0 || n < 0 || n > a.max_n || lda < max(1, m);
+    // (The host gives no matrix of more than TEAM_ROWS rows to a team.)
+    const bool bad = m < 0 || n < 0 || n > a.max_n || lda < max(1, m) || (T > 1 && m > TEAM_ROWS);
     if (bad || m == 0 || n == 0) {
-      if (tid == 0 && a.info) a.info[item] = bad ? HQ_ERR_BAD_SHAPE : 0;
+      if (tid == 0 && me == 0 && a.info) a.info[item] = bad ? HQ_ERR_BAD_SHAPE : 0;
       continue;
     }
-    const int lds = m;
-    const bool staged = (long long)lds * n * 8 <= a.stage_bytes;
-    double* X = staged ? sX : Ag;
-    const int ldx = staged ? lds : lda;
-    if (staged)
-      for (long long e = tid; e < (long long)m * n; e += NT) {
-        const int i = (int)(e % m), k = (int)(e / m);
-        sX[i + (long long)k * lds] = Ag[i + (long long)k * lda];
+    // This CTA's columns are me, me + T, ...: local index q, column me + T q.
+    const int nl = (n - me + T - 1) / T;
+    const bool staged = (long long)m * ((n + T - 1) / T) * 8 <= a.stage_bytes;
+    auto colp = [&](int q) { return staged ? sX + (size_t)q * m : Ag + (size_t)(me + T * q) * lda; };
+    // Load, initial norms (warp per column, fixed lane order).
+    for (int q = warp; q < nl; q += NW) {
+      const double* g = Ag + (size_t)(me + T * q) * lda;
+      double* x = colp(q);
+      double t = 0.0;
+#pragma unroll 4
+      for (int i = lane; i < m; i += 32) {
+        const double v = g[i];
+        if (staged) x[i] = v;
+        t = fma(v, v, t);
       }
-    __syncthreads();
-    // Initial norms (warp per column, fixed lane order).
-    for (int k = warp; k < n; k += NW) {
-      const double* x = X + (long long)k * ldx;
-      double q = 0.0;
-      for (int i = lane; i < m; i += 32) q = fma(x[i], x[i], q);
-      q = hq_warp_sum(q);
+      t = hq_warp_sum(t);
       if (lane == 0) {
-        sd[k] = sqrt(q);
-        se[k] = sd[k];
-        sperm[k] = k;
+        sd[q] = t;
+        sthr[q] = HQ_TOL3Z * t;
+        spos[q] = me + T * q;
+        sact[q] = q;
       }
     }
     __syncthreads();
+    int cnt = nl;  // columns in sact
+    // Each warp's best (largest norm, then lowest position) of the columns
+    // not yet factored; at = position << 32 | column.
+    auto warp_best = [&](long long k, long long at) {
+      const unsigned long long u = (unsigned long long)(k + 4);
+      const unsigned hi = (unsigned)(u >> 32);
+      const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+      const unsigned lo = hi == mh ? (unsigned)u : 0u;
+      const unsigned ml = __reduce_max_sync(0xffffffffu, lo);
+      const bool mine = hi == mh && (unsigned)u == ml;
+      const int p = (int)(at >> 32);
+      const int bp = __reduce_min_sync(0xffffffffu, mine ? p : 0x7fffffff);
+      if (mine && p == bp) {
+        s_bk[warp] = k;
+        s_at[warp] = at;
+      }
+    };
+    auto best_of_columns = [&]() {
+      if (tid >= ND) return;
+      long long k = -2, at = 0x7fffffffLL << 32;
+      for (int j = tid; j < cnt; j += ND) {
+        const int q = sact[j];
+        const long long kj = hq_norm_key(sd[q]);
+        const long long aj = ((long long)spos[q] << 32) | (unsigned)(me + T * q);
+        if (better(kj, aj, k, at)) { k = kj; at = aj; }
+      }
+      warp_best(k, at);
+    };
+    best_of_columns();
+    __syncthreads();
+
     const int mn = min(m, n);
+    int pend = -1;  // a team's own pivot column, to be written after the next barrier
+    double pend_beta = 0.0;
+    auto flush = [&](int s_of) {  // v (still in sv) below row s_of, beta on it
+      if (pend < 0) return;
+      double* x = colp(pend);
+      for (int i = s_of + 1 + tid; i < m; i += NT) x[i] = sv[i];
+      if (tid == 0) x[s_of] = pend_beta;
+      pend = -1;
+    };
     for (int s = 0; s < mn; ++s) {
-      // Pivot: first maximum of the partial norms (idamax).
-      {
-        double bd = -1.0;
-        int bk = 0x7fffffff;
-        for (int k = s + tid; k < n; k += NT) {
-          const double d = sd[k];
-          if (d > bd || (d == bd && k < bk)) { bd = d; bk = k; }
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-          const double od = __shfl_xor_sync(0xffffffffu, bd, o);
-          const int ok = __shfl_xor_sync(0xffffffffu, bk, o);
-          if (od > bd || (od == bd && ok < bk)) { bd = od; bk = ok; }
-        }
-        if (lane == 0) { s_red[warp] = bd; s_bk[warp] = bk; }
-        __syncthreads();
-        if (tid == 0) {
-          for (int w = 1; w < NW; ++w)
-            if (s_red[w] > bd || (s_red[w] == bd && s_bk[w] < bk)) { bd = s_red[w]; bk = s_bk[w]; }
-          s_kp = bk == 0x7fffffff ? s : bk;
-        }
-        __syncthreads();
+      // 1. The pivot.
+      long long bk = s_bk[0], at = s_at[0];
+#pragma unroll
+      for (int w = 1; w < NDW; ++w)
+        if (better(s_bk[w], s_at[w], bk, at)) { bk = s_bk[w]; at = s_at[w]; }
+      if (T > 1) {
+        if (tid < T) cluster_st(cluster_addr(s_cand[s & 1][me], (unsigned)tid), bk, at);
+        cluster_barrier();
+        bk = s_cand[s & 1][0][0];
+        at = s_cand[s & 1][0][1];
+        for (int r = 1; r < T; ++r)
+          if (better(s_cand[s & 1][r][0], s_cand[s & 1][r][1], bk, at)) {
+            bk = s_cand[s & 1][r][0];
+            at = s_cand[s & 1][r][1];
+          }
+        flush(s - 1);
       }
-      const int kp = s_kp;
-      if (kp != s) {
-        double* c1 = X + (long long)s * ldx;
-        double* c2 = X + (long long)kp * ldx;
-        for (int i = tid; i < m; i += NT) {
-          const double t = c1[i];
-          c1[i] = c2[i];
-          c2[i] = t;
-        }
-        if (tid == 0) {
-          const int t = sperm[s];
-          sperm[s] = sperm[kp];
-          sperm[kp] = t;
-          sd[kp] = sd[s];
-          se[kp] = se[s];
+      const int wpos = (int)(at >> 32), wcol = (int)(unsigned)at;
+      const int owner = wcol % T, wq = wcol / T;
+      for (int j = tid; j < cnt; j += NT) {
+        const int q = sact[j];
+        const int p = spos[q];
+        if (owner == me && q == wq) {
+          spos[q] = s;
+          sact[j] = -1;  // replaced by the last one below
+        } else if (p == s) {
+          spos[q] = wpos;
         }
       }
-      __syncthreads();
-      // Reflector for column s (rows s..m-1).
-      double* xs = X + (long long)s * ldx;
+      if (T > 1) __syncthreads();  // sv is rewritten below
+
+      // 2. The pivot column and its reflector; v in place (one CTA), or in sv.
+      double* v = T > 1 ? sv : colp(wq);
       {
-        double q = 0.0;
-        for (int i = s + 1 + tid; i < m; i += NT) q = fma(xs[i], xs[i], q);
-        q = hq_warp_sum(q);
-        if (lane == 0) s_red[warp] = q;
-        __syncthreads();
-        if (tid == 0) {
-          double t = 0.0;
-          for (int w = 0; w < NW; ++w) t += s_red[w];
-          const HqReflector h = hq_make_reflector_sq(xs[s], m - s > 1 ? t : 0.0);
-          s_tau = h.tau;
-          s_scale = h.scale;
-          s_beta = h.beta;
-          a.tau[item][s] = h.tau;
+        if (T > 1) {
+          const double* g = Ag + (size_t)wcol * lda;
+          const unsigned r0 = cluster_addr(sX + (size_t)wq * m, (unsigned)owner);
+          for (int i = s + tid; i < m; i += NT)
+            sv[i] = staged ? cluster_ld(r0 + 8u * (unsigned)i) : hq_ldcg(g + i);
+          __syncthreads();
         }
+        if (tid < ND) {
+          double t0 = 0.0, t1 = 0.0;
+          int i = s + 1 + tid;
+          for (; i + ND < m; i += 2 * ND) {
+            t0 = fma(v[i], v[i], t0);
+            t1 = fma(v[i + ND], v[i + ND], t1);
+          }
+          if (i < m) t0 = fma(v[i], v[i], t0);
+          t0 = hq_warp_sum(t0 + t1);
+          if (lane == 0) s_red[warp] = t0;
+        }
+        __syncthreads();
+        if (warp == 0) {
+          double q = s_red[lane & (NDW - 1)];
+#pragma unroll
+          for (int o = NDW / 2; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+          if (lane == 0) {
+            const HqReflector h = hq_make_reflector_sq(v[s], m - s > 1 ? q : 0.0);
+            s_tau = h.tau;
+            s_scale = h.scale;
+            s_beta = h.beta;
+            if (me == 0) a.tau[item][s] = h.tau;
+          }
+        } else if (warp == 1) {
+          // The list without the pivot: its place takes the last column.
+          if (owner == me) {
+            for (int j = lane; j < cnt - 1; j += 32)
+              if (sact[j] < 0) sact[j] = sact[cnt - 1];
+          }
+        }
+        if (owner == me) --cnt;
         __syncthreads();
         const double scale = s_scale;
-        for (int i = s + 1 + tid; i < m; i += NT) xs[i] *= scale;
-        __syncthreads();
-        if (tid == 0) xs[s] = 1.0;  // v_s, restored to beta after the update
+        for (int i = s + 1 + tid; i < m; i += NT) v[i] *= scale;
+        if (tid == 0) v[s] = 1.0;  // restored to beta after the update
+        if (T > 1 && owner == me) {
+          pend = wq;
+          pend_beta = s_beta;
+        }
         __syncthreads();
       }
-      // w_k = tau * v^T X[s:, k]; X[s:, k] -= v w_k, a warp per column.
+
+      // 3. X[s:, k] -= tau v (v^T X[s:, k]): as many columns a warp as its
+      //    registers hold of this many rows (four of 256, two of 512, one of
+      //    1024; longer columns are read twice), fewer when not every warp
+      //    would have as many.
       const double tau = s_tau;
-      for (int k = s + 1 + warp; k < n; k += NW) {
-        double* xk = X + (long long)k * ldx;
-        double w = 0.0;
-        for (int i = s + lane; i < m; i += 32) w = fma(xs[i], xk[i], w);
-        w = hq_warp_sum(w) * tau;
-        for (int i = s + lane; i < m; i += 32) xk[i] = fma(-xs[i], w, xk[i]);
+      auto apply = [&](auto take, int j) {
+        constexpr int NY = decltype(take)::ny;
+        double* y[NY];
+        double* rs[NY];
+#pragma unroll
+        for (int c = 0; c < NY; ++c) {
+          const int q = sact[j + c];
+          y[c] = colp(q);
+          rs[c] = srs + q;
+        }
+        apply_warp<NY, decltype(take)::ch>(v, y, tau, s, m, lane, rs);
+      };
+      int j = 0;
+      const int rows = m - s;
+      if (rows <= 256)
+        for (; j + 4 * NW <= cnt; j += 4 * NW) apply(Take<4, 8>{}, j + 4 * warp);
+      if (rows <= 512)
+        for (; j + 2 * NW <= cnt; j += 2 * NW) apply(Take<2, 16>{}, j + 2 * warp);
+      if (rows > 1024)
+        for (; j + 4 * NW <= cnt; j += 4 * NW) apply(Take<4, 0>{}, j + 4 * warp);
+      j += warp;
+      if (rows <= 256) {
+        for (; j < cnt; j += NW) apply(Take<1, 8>{}, j);
+      } else if (rows <= 1024) {
+        for (; j < cnt; j += NW) apply(Take<1, 32>{}, j);
+      } else {
+        for (; j < cnt; j += NW) apply(Take<1, 0>{}, j);
       }
       __syncthreads();
-      // LAWN 176 downdate of the partial norms, one thread per column, from
-      // the new entries of row s (a warp per column would repeat its
-      // divisions and square root on 32 lanes of the scarce FP64 pipe);
-      // columns that need their norm recomputed are flagged and recomputed
-      // below, a warp per column (rare).
-      int* sflag = reinterpret_cast<int*>(sw);
+
+      // 4. LAWN 176 downdate of the squared norms, one thread per column; the
+      //    next pivot.  Norms to be recomputed (rare): a warp per column.
+      if (T == 1 && tid == 0) v[s] = s_beta;
       int any = 0;
-      for (int k = s + 1 + tid; k < n; k += NT) {
-        double dk = sd[k];
+      for (int jj = tid; tid < ND && jj < cnt; jj += ND) {
+        const int q = sact[jj];
+        const double d = sd[q];
         int flag = 0;
-        if (dk != 0.0) {
-          double t1 = fabs(X[s + (long long)k * ldx]) / dk;
-          t1 = (1.0 + t1) * (1.0 - t1);
-          if (0.0 > t1) t1 = 0.0;
-          const double ratio = dk / se[k];
-          const double t2 = t1 * ratio * ratio;
-          if (t2 <= HQ_TOL3Z) flag = 1;
-          else sd[k] = dk * sqrt(t1);
+        if (d != 0.0) {
+          const double r = srs[q];
+          const double nd = fma(-r, r, d);
+          const long long nb = __double_as_longlong(nd);
+          if (nb <= __double_as_longlong(sthr[q]) || nb > 0x7ff0000000000000LL) flag = 1;
+          else sd[q] = nd;
         }
-        sflag[k] = flag;
+        if (flag) sd[q] = -1.0;
         any |= flag;
       }
+      best_of_columns();
       if (__syncthreads_or(any)) {
-        for (int k = s + 1 + warp; k < n; k += NW) {
-          if (!sflag[k]) continue;  // uniform across the warp
-          const double* xk = X + (long long)k * ldx;
-          double q = 0.0;
-          for (int i = s + 1 + lane; i < m; i += 32) q = fma(xk[i], xk[i], q);
-          q = hq_warp_sum(q);
+        for (int jj = warp; jj < cnt; jj += NW) {
+          const int q = sact[jj];
+          if (sd[q] != -1.0) continue;  // uniform across the warp
+          const double* x = colp(q);
+          double t = 0.0;
+          for (int i = s + 1 + lane; i < m; i += 32) t = fma(x[i], x[i], t);
+          t = hq_warp_sum(t);
+          __syncwarp();
           if (lane == 0) {
-            const double nv = m - s - 1 > 0 ? sqrt(q) : 0.0;
-            sd[k] = nv;
-            se[k] = nv;
+            sd[q] = t;
+            sthr[q] = HQ_TOL3Z * t;
           }
         }
         __syncthreads();
+        best_of_columns();
+        __syncthreads();
       }
-      if (tid == 0) xs[s] = s_beta;
+    }
+    if (T > 1) {
+      cluster_barrier();  // every CTA has read the last pivot column
+      flush(mn - 1);
       __syncthreads();
     }
-    if (staged)
-      for (long long e = tid; e < (long long)m * n; e += NT) {
-        const int i = (int)(e % m), k = (int)(e / m);
-        Ag[i + (long long)k * lda] = sX[i + (long long)k * lds];
+
+    // The way out: jpvt, and the columns in their final order.
+    for (int q = tid; q < nl; q += NT) a.jpvt[item][spos[q]] = me + T * q + 1;
+    if (staged) {
+      // Every CTA of a team has loaded its columns long before (a barrier ago).
+      for (int q = warp; q < nl; q += NW) {
+        const double* x = colp(q);
+        double* g = Ag + (size_t)spos[q] * lda;
+        for (int i = lane; i < m; i += 32) g[i] = x[i];
       }
-    for (int k = tid; k < n; k += NT) a.jpvt[item][k] = sperm[k] + 1;
-    if (tid == 0 && a.info) a.info[item] = 0;
-    __syncthreads();
+      __syncthreads();
+      if (T > 1) cluster_barrier();  // s_cand, sv and sX may be reused
+    } else {
+      // In place: rows are dealt out over the threads, and each walks the
+      // cycles of the permutation (position p takes the column jpvt[p]).
+      if (T > 1) cluster_barrier();  // jpvt and the columns are written
+      else __syncthreads();
+      int* from = spos;  // column that position p takes; then marked by its complement
+      int* seq = sact;   // the cycles one after the other, a cycle's first entry complemented
+      __shared__ int s_len;
+      for (int p = tid; p < n; p += NT) from[p] = __ldcg(a.jpvt[item] + p) - 1;
+      __syncthreads();
+      if (tid == 0) {
+        int len = 0;
+        for (int p = 0; p < n; ++p) {
+          if (from[p] < 0 || from[p] == p) continue;
+          int c = p;
+          bool first = true;
+          while (from[c] >= 0) {
+            const int nx = from[c];
+            seq[len++] = first ? ~c : c;
+            first = false;
+            from[c] = ~nx;
+            c = nx;
+          }
+        }
+        s_len = len;
+      }
+      __syncthreads();
+      const int len = s_len;
+      for (int i = me * NT + tid; i < m; i += T * NT) {
+        double* x = Ag + i;
+        double first = 0.0;  // value of the current cycle's first entry
+        constexpr int B = 8;  // loads in flight along a cycle
+        for (int e = 0; e < len; e += B) {
+          // Entry e receives the next one's value; the last of a cycle its
+          // first's.  All loads of a batch precede its stores, and a batch's
+          // stores only reach entries whose values are already loaded.
+          double val[B];
+#pragma unroll
+          for (int u = 0; u < B; ++u) {
+            if (e + u < len) {
+              const int c = seq[e + u];
+              if (c < 0) first = __ldcg(x + (size_t)(~c) * lda);
+              const int nx = e + u + 1 < len ? seq[e + u + 1] : -1;
+              val[u] = nx < 0 ? first : __ldcg(x + (size_t)nx * lda);
+            }
+          }
+#pragma unroll
+          for (int u = 0; u < B; ++u) {
+            if (e + u < len) {
+              const int c = seq[e + u];
+              x[(size_t)(c < 0 ? ~c : c) * lda] = val[u];
+            }
+          }
+        }
+      }
+      __syncthreads();
+      if (T > 1) cluster_barrier();
+    }
+    if (tid == 0 && me == 0 && a.info) a.info[item] = 0;
   }
 }
 
 template <int NT>
-int launch_t(cudaStream_t st, const hq_device_info* dev, const BatchArgs& a, int ctas_per_sm) {
-  const size_t fixed = sizeof(double) * 3 * (size_t)a.max_n + sizeof(int) * (size_t)((a.max_n + 1) & ~1);
+int launch_t(cudaStream_t st, const hq_device_info* dev, BatchArgs a, int ctas_per_sm,
+             int team) {
+  const size_t fixed = sizeof(double) * 4 * (size_t)a.max_n +
+                       (team > 1 ? sizeof(double) * TEAM_ROWS : 0);
+  if (fixed > dev->smem_optin) return (int)cudaErrorInvalidValue;
+  if ((size_t)a.stage_bytes > dev->smem_optin - fixed) a.stage_bytes = (int)(dev->smem_optin - fixed);
   const size_t smem = fixed + (size_t)a.stage_bytes;
-  if (smem > dev->smem_optin) return (int)cudaErrorInvalidValue;
-  cudaError_t e = cudaFuncSetAttribute(qrp_batched_kernel<NT>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  auto kernel = qrp_batched_kernel<NT>;
+  cudaError_t e =
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
   int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, qrp_batched_kernel<NT>, NT, smem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, NT, smem);
   if (e != cudaSuccess) return (int)e;
   if (per_sm < 1) return (int)cudaErrorInvalidConfiguration;
   if (ctas_per_sm < per_sm) per_sm = ctas_per_sm;
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3(NT);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)team;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = team > 1 ? 1 : 0;
   int grid = dev->num_sms * per_sm;
-  if (grid > a.batch) grid = a.batch;
-  qrp_batched_kernel<NT><<<grid, NT, smem, st>>>(a);
+  if (team > 1) {
+    int ncl = 0;
+    cfg.gridDim = dim3((unsigned)team);
+    e = cudaOccupancyMaxActiveClusters(&ncl, kernel, &cfg);
+    if (e != cudaSuccess) return (int)e;
+    if (ncl < 1) return (int)cudaErrorInvalidConfiguration;
+    if (grid > ncl * team) grid = ncl * team;
+    grid = grid / team * team;
+    if (grid < team) grid = team;
+  } else if (grid > a.batch) {
+    grid = a.batch;
+  }
+  cfg.gridDim = dim3((unsigned)grid);
+  e = cudaLaunchKernelEx(&cfg, kernel, a);
   hq_count_launches(1);
-  return (int)cudaGetLastError();
+  return (int)e;
 }
 
 }  // namespace
 
-// Workspace: queue head + schedule.
+// Workspace: queue heads, the teams' counts, schedule.
 extern "C" size_t hq_qrp_batched_workspace(int batch) {
   return sizeof(int) * (size_t)(batch + 64);
 }
@@ -249,9 +613,11 @@ extern "C" int hq_qrp_batched(cudaStream_t stream, const hq_device_info* dev, in
                               const int* d_m, const int* d_n, double* const* d_A,
                               const int* d_lda, int* const* d_jpvt, double* const* d_tau,
                               int* d_info, void* d_work, int max_n, int threads, int stage_kb,
-                              int ctas_per_sm) {
+                              int ctas_per_sm, int team) {
   if (batch <= 0) return 0;
   if (max_n <= 0 || max_n > 4096) return (int)cudaErrorInvalidValue;
+  if (team != 1 && team != 2 && team != 4 && team != T_MAX) return (int)cudaErrorInvalidValue;
+  if (ctas_per_sm < 1 || ctas_per_sm > 7) return (int)cudaErrorInvalidValue;
   BatchArgs a;
   a.batch = batch;
   a.m = d_m;
@@ -262,15 +628,16 @@ extern "C" int hq_qrp_batched(cudaStream_t stream, const hq_device_info* dev, in
   a.tau = d_tau;
   a.info = d_info;
   a.next = static_cast<int*>(d_work);
+  a.n_team = static_cast<const int*>(d_work) + HQ_BATCHED_TEAM_SLOT + ctas_per_sm;
   a.order = static_cast<const int*>(d_work) + 32;
   a.stage_bytes = stage_kb * 1024;
   a.max_n = max_n;
-  cudaError_t e = cudaMemsetAsync(a.next, 0, sizeof(int), stream);
+  cudaError_t e = cudaMemsetAsync(a.next, 0, 2 * sizeof(int), stream);
   if (e != cudaSuccess) return (int)e;
   switch (threads) {
-    case 128: return launch_t<128>(stream, dev, a, ctas_per_sm);
-    case 256: return launch_t<256>(stream, dev, a, ctas_per_sm);
-    case 512: return launch_t<512>(stream, dev, a, ctas_per_sm);
+    case 128: return launch_t<128>(stream, dev, a, ctas_per_sm, team);
+    case 256: return launch_t<256>(stream, dev, a, ctas_per_sm, team);
+    case 512: return launch_t<512>(stream, dev, a, ctas_per_sm, team);
     default: return (int)cudaErrorInvalidValue;
   }
 }
