@@ -1269,20 +1269,19 @@ static int core_dgeqp4(hq_ws* w, int m, int n, double* dA, int ldda, int* hjp, i
     const int mt = m - nf, nt = n - nf;
     double* At = dA + nf + (size_t)nf * ldda;
     CK(hq_fill_iota(w->st, w->labels, nt, 0));
-    if (small && nt > HQ_MAX_PANEL) {
-      /* Wide: min(m, n) < 1000 and more than HQ_MAX_PANEL free columns, so
-       * mt < 1000 rows.  The column-partitioned kernel leaves the columns in
-       * place and reports the final order as pairs, applied here to all m
-       * rows of the free columns (the rows above them included) and to jpvt. */
+    if (small && mt <= HQ_WIDE_MAX_ROWS && nt > HQ_WIDE_MIN_COLS) {
+      /* The column-partitioned kernel leaves the columns in place and reports
+       * the final order as pairs, applied here to all m rows of the free
+       * columns (the rows above them included) and to jpvt.  (More than
+       * HQ_MAX_PANEL columns imply fewer rows than HQ_WIDE_MAX_ROWS.) */
       const int ns = imin(mt, nt);
-      int* phys = ws_alloc(w, sizeof(int) * (size_t)nt);
-      long long* cand = ws_alloc(w, sizeof(long long) * hq_wide_cand_elems(dev));
+      void* xch = ws_alloc(w, hq_wide_xch_bytes(dev, mt, nt));
       int* wpairs = ws_alloc(w, sizeof(int) * 4 * (size_t)ns);
       int* wlab = ws_alloc(w, sizeof(int) * 2 * (size_t)ns);
       double* wtmp = ws_alloc(w, sizeof(double) * (size_t)m * 2 * ns);
       if (w->failed) return HQ_E_NOMEM;
-      CK(hq_wide_qrp(w->st, dev, mt, nt, At, ldda, dtau + nf, phys, cand, wpairs, w->npairs,
-                     w->bar + 1, w->err, spin));
+      CK(hq_wide_qrp(w->st, dev, mt, nt, At, ldda, dtau + nf, xch, wpairs, w->npairs, w->err,
+                     spin));
       CK(hq_permute_pairs(w->st, m, dA + (size_t)nf * ldda, ldda, nt, wpairs, w->npairs, 2 * ns,
                           wtmp, djp + nf, wlab));
     } else if (small) {

@@ -37,7 +37,7 @@
 // All columns are free (LAPACK jpvt = 0 input); on return jpvt[k] is the
 // 1-based original index of column k, tau[0..min(m,n)) the reflector scalars,
 // R and the reflectors overwrite A.
-#include "hq_common.cuh"
+#include "hq_columns.cuh"
 
 namespace {
 
@@ -90,108 +90,6 @@ __device__ __forceinline__ double cluster_ld(unsigned addr) {
   asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(addr) : "memory");
   return v;
 }
-
-// Larger key first, then the lower position (the upper word of at).
-__device__ __forceinline__ bool better(long long k1, long long at1, long long k2, long long at2) {
-  return k1 > k2 || (k1 == k2 && at1 < at2);
-}
-
-// Sums over the lanes of NY values per lane, in the lanes [32 / NY c, 32 / NY
-// (c + 1)) for value c: each halving of the lanes that share a value also
-// halves the values a lane keeps, so four take 2 + 1 + 3 additions.
-template <int NY>
-__device__ __forceinline__ double lanes_sum(const double (&d)[NY], int lane) {
-  double t;
-  if constexpr (NY == 4) {
-    const bool up = lane & 16;
-    const double a = (up ? d[2] : d[0]) + __shfl_xor_sync(0xffffffffu, up ? d[0] : d[2], 16);
-    const double b = (up ? d[3] : d[1]) + __shfl_xor_sync(0xffffffffu, up ? d[1] : d[3], 16);
-    const bool up8 = lane & 8;
-    t = (up8 ? b : a) + __shfl_xor_sync(0xffffffffu, up8 ? a : b, 8);
-  } else if constexpr (NY == 2) {
-    const bool up = lane & 16;
-    t = (up ? d[1] : d[0]) + __shfl_xor_sync(0xffffffffu, up ? d[0] : d[1], 16);
-    t += __shfl_xor_sync(0xffffffffu, t, 8);
-  } else {
-    t = d[0] + __shfl_xor_sync(0xffffffffu, d[0], 16);
-    t += __shfl_xor_sync(0xffffffffu, t, 8);
-  }
-#pragma unroll
-  for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-  return t;
-}
-
-// y_c -= tau (v^T y_c) v over rows s..m-1 for NY columns y_c of one warp; the
-// new entries of row s go to rs[c].  CH > 0: the columns stay in registers
-// between the two uses (at most 32 CH rows); CH = 0: read twice.
-template <int NY, int CH>
-__device__ __forceinline__ void apply_warp(const double* __restrict__ v, double* const (&y)[NY],
-                                           double tau, int s, int m, int lane, double* (&rs)[NY]) {
-  double d[NY];
-#pragma unroll
-  for (int c = 0; c < NY; ++c) d[c] = 0.0;
-  if constexpr (CH > 0) {
-    double x[NY][CH];
-#pragma unroll
-    for (int t = 0; t < CH; ++t) {
-      const int i = s + lane + 32 * t;
-#pragma unroll
-      for (int c = 0; c < NY; ++c) x[c][t] = i < m ? y[c][i] : 0.0;
-    }
-#pragma unroll
-    for (int t = 0; t < CH; ++t) {
-      const int i = s + lane + 32 * t;
-      if (s + 32 * t < m) {  // uniform: no FP64 for rows that are not there
-        const double vi = i < m ? v[i] : 0.0;
-#pragma unroll
-        for (int c = 0; c < NY; ++c) d[c] = fma(vi, x[c][t], d[c]);
-      }
-    }
-    const double t = lanes_sum<NY>(d, lane) * -tau;
-    double w[NY];
-#pragma unroll
-    for (int c = 0; c < NY; ++c) w[c] = __shfl_sync(0xffffffffu, t, 32 / NY * c);
-#pragma unroll
-    for (int t2 = 0; t2 < CH; ++t2) {
-      const int i = s + lane + 32 * t2;
-      if (s + 32 * t2 < m) {
-        const double vi = i < m ? v[i] : 0.0;
-#pragma unroll
-        for (int c = 0; c < NY; ++c) {
-          const double z = fma(vi, w[c], x[c][t2]);
-          if (i < m) y[c][i] = z;
-          if (t2 == 0 && lane == 0) *rs[c] = z;
-        }
-      }
-    }
-  } else {
-#pragma unroll 4
-    for (int i = s + lane; i < m; i += 32) {
-      const double vi = v[i];
-#pragma unroll
-      for (int c = 0; c < NY; ++c) d[c] = fma(vi, y[c][i], d[c]);
-    }
-    const double t = lanes_sum<NY>(d, lane) * -tau;
-    double w[NY];
-#pragma unroll
-    for (int c = 0; c < NY; ++c) w[c] = __shfl_sync(0xffffffffu, t, 32 / NY * c);
-#pragma unroll 4
-    for (int i = s + lane; i < m; i += 32) {
-      const double vi = v[i];
-#pragma unroll
-      for (int c = 0; c < NY; ++c) {
-        const double z = fma(vi, w[c], y[c][i]);
-        y[c][i] = z;
-        if (i == s) *rs[c] = z;
-      }
-    }
-  }
-}
-
-template <int NY, int CH>
-struct Take {
-  static constexpr int ny = NY, ch = CH;
-};
 
 template <int NT>
 __global__ void __launch_bounds__(NT, 512 / NT) qrp_batched_kernel(BatchArgs a) {
@@ -280,22 +178,8 @@ __global__ void __launch_bounds__(NT, 512 / NT) qrp_batched_kernel(BatchArgs a) 
     }
     __syncthreads();
     int cnt = nl;  // columns in sact
-    // Each warp's best (largest norm, then lowest position) of the columns
-    // not yet factored; at = position << 32 | column.
-    auto warp_best = [&](long long k, long long at) {
-      const unsigned long long u = (unsigned long long)(k + 4);
-      const unsigned hi = (unsigned)(u >> 32);
-      const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
-      const unsigned lo = hi == mh ? (unsigned)u : 0u;
-      const unsigned ml = __reduce_max_sync(0xffffffffu, lo);
-      const bool mine = hi == mh && (unsigned)u == ml;
-      const int p = (int)(at >> 32);
-      const int bp = __reduce_min_sync(0xffffffffu, mine ? p : 0x7fffffff);
-      if (mine && p == bp) {
-        s_bk[warp] = k;
-        s_at[warp] = at;
-      }
-    };
+    // Each warp's best of the columns not yet factored; at = position << 32 |
+    // column.
     auto best_of_columns = [&]() {
       if (tid >= ND) return;
       long long k = -2, at = 0x7fffffffLL << 32;
@@ -305,7 +189,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) qrp_batched_kernel(BatchArgs a) 
         const long long aj = ((long long)spos[q] << 32) | (unsigned)(me + T * q);
         if (better(kj, aj, k, at)) { k = kj; at = aj; }
       }
-      warp_best(k, at);
+      warp_best(k, at, s_bk + warp, s_at + warp);
     };
     best_of_columns();
     __syncthreads();
@@ -363,15 +247,8 @@ __global__ void __launch_bounds__(NT, 512 / NT) qrp_batched_kernel(BatchArgs a) 
           __syncthreads();
         }
         if (tid < ND) {
-          double t0 = 0.0, t1 = 0.0;
-          int i = s + 1 + tid;
-          for (; i + ND < m; i += 2 * ND) {
-            t0 = fma(v[i], v[i], t0);
-            t1 = fma(v[i + ND], v[i + ND], t1);
-          }
-          if (i < m) t0 = fma(v[i], v[i], t0);
-          t0 = hq_warp_sum(t0 + t1);
-          if (lane == 0) s_red[warp] = t0;
+          const double t = tail_squares<ND>(v, s, m, tid);
+          if (lane == 0) s_red[warp] = t;
         }
         __syncthreads();
         if (warp == 0) {
@@ -404,39 +281,8 @@ __global__ void __launch_bounds__(NT, 512 / NT) qrp_batched_kernel(BatchArgs a) 
         __syncthreads();
       }
 
-      // 3. X[s:, k] -= tau v (v^T X[s:, k]): as many columns a warp as its
-      //    registers hold of this many rows (four of 256, two of 512, one of
-      //    1024; longer columns are read twice), fewer when not every warp
-      //    would have as many.
-      const double tau = s_tau;
-      auto apply = [&](auto take, int j) {
-        constexpr int NY = decltype(take)::ny;
-        double* y[NY];
-        double* rs[NY];
-#pragma unroll
-        for (int c = 0; c < NY; ++c) {
-          const int q = sact[j + c];
-          y[c] = colp(q);
-          rs[c] = srs + q;
-        }
-        apply_warp<NY, decltype(take)::ch>(v, y, tau, s, m, lane, rs);
-      };
-      int j = 0;
-      const int rows = m - s;
-      if (rows <= 256)
-        for (; j + 4 * NW <= cnt; j += 4 * NW) apply(Take<4, 8>{}, j + 4 * warp);
-      if (rows <= 512)
-        for (; j + 2 * NW <= cnt; j += 2 * NW) apply(Take<2, 16>{}, j + 2 * warp);
-      if (rows > 1024)
-        for (; j + 4 * NW <= cnt; j += 4 * NW) apply(Take<4, 0>{}, j + 4 * warp);
-      j += warp;
-      if (rows <= 256) {
-        for (; j < cnt; j += NW) apply(Take<1, 8>{}, j);
-      } else if (rows <= 1024) {
-        for (; j < cnt; j += NW) apply(Take<1, 32>{}, j);
-      } else {
-        for (; j < cnt; j += NW) apply(Take<1, 0>{}, j);
-      }
+      // 3. X[s:, k] -= tau v (v^T X[s:, k]).
+      apply_columns<NW>(v, s_tau, s, m, cnt, sact, srs, colp, warp, lane);
       __syncthreads();
 
       // 4. LAWN 176 downdate of the squared norms, one thread per column; the

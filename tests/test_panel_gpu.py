@@ -65,3 +65,40 @@ def test_non_finite_input_ends(hq, m, n, bad):
     F, jp, tau, info, _ = hq.dgeqp4(A)
     assert info == 0 and sorted(jp) == list(range(1, n + 1))
     assert not np.all(np.isfinite(F))
+
+
+# The column-partitioned kernel (more than 512 columns, at most 1024 rows): one
+# and several columns a CTA, columns in registers four, two and one at a time,
+# a matrix that does not fit the grid's shared memory, one row.
+@pytest.mark.parametrize("m,n", [
+    (1, 600), (7, 513), (40, 1100), (129, 700), (257, 2000), (513, 900), (1000, 999), (999, 5200)])
+def test_wide_shapes(hq, m, n):
+    _check(hq, oracle.gaussian(m, n, 5 * m + n))
+
+
+def test_wide_recomputed_norms(hq):
+    import scipy.linalg as sl
+    rng = np.random.default_rng(8)
+    m, n = 300, 1500
+    A = np.asfortranarray(rng.standard_normal((m, 5)) @ rng.standard_normal((5, n))
+                          + rng.standard_normal((m, n)) * 10.0 ** -rng.uniform(5.0, 6.0, n))
+    hq.set_precision(hq.PLAIN)
+    F, jp, tau, info, _ = hq.dgeqp4(A)
+    Ro, po = sl.qr(A, mode="r", pivoting=True)[:2]
+    np.testing.assert_array_equal(jp, po + 1)
+    d, do = np.abs(np.diag(F)), np.abs(np.diag(Ro))
+    assert np.max(np.abs(d - do)) <= 50.0 * m * np.finfo(float).eps * do[0]
+
+
+def test_wide_wait_that_gives_up(hq):
+    A = oracle.gaussian(200, 1200, 4)
+    hq.set_precision(hq.PLAIN)
+    want = hq.dgeqp4(A)
+    hq.set_spin_limit(1)
+    try:
+        with pytest.raises(hq.HQRRPError, match="barrier"):
+            hq.dgeqp4(A)
+    finally:
+        hq.set_spin_limit(0)
+    for w, g in zip(want[:3], hq.dgeqp4(A)[:3]):
+        np.testing.assert_array_equal(w, g)
