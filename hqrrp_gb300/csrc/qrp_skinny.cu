@@ -274,28 +274,32 @@ __global__ void __launch_bounds__(NT, 1) skinny_qrp_kernel(SkArgs a) {
 // (lane l has rows LPC t + l, t < RPT), so a stage reads its columns from
 // registers; the reflector is staged in shared memory in the same order and
 // read 16 bytes at a time, whole chunks of 16 rows above the stage's row being
-// jumped over.  Scalar work is done once, not by every thread: one lane builds
+// jumped over.  Scalar work is done once, not by every thread: one warp builds
 // the reflector, one thread per column downdates its norm, and pivot
 // candidates compare integer keys.
 //
 // What bounds a stage is the latency of agreeing on the pivot, so the exchange
 // has neither a fence nor a counter.  A CTA writes its best candidate -- norm
-// key and position, once for every CTA, and the column once -- in words that
-// carry the stage's tag next to the value (128- and 64-bit scalar stores,
-// which are single-copy atomic).  One warp per CTA polls its CTA's own copy of
-// the P headers, picks the winner and polls its column: a word whose tag
-// matches holds this stage's value, so nothing has to be ordered before
-// anything else.  (With one copy of the headers for all, the polls of 128 CTAs
-// queue up at the few cache lines that the headers are written to: 3500 clocks
-// in that wait alone, against 1400 for 24 CTAs.)  Headers and columns alternate between two
-// buffers.  A CTA overwrites a buffer at stage s + 2 after it has seen every
-// CTA's header of stage s + 1, which each wrote after it had read stage s.
+// key and position, once for every CTA -- in words that carry the stage's tag
+// next to the value (128- and 64-bit scalar stores, which are single-copy
+// atomic), and then, as if it had won, the reflector of the candidate's column:
+// its sums and square root are off the path everyone waits on, and a loser's
+// cost nothing but an idle warp.  A warp of its own in each CTA polls the
+// CTA's own copy of the P headers, picks the winner and polls its reflector: a
+// word whose tag matches holds this stage's value, so nothing has to be
+// ordered before anything else.  (With one copy of the headers for all, the
+// polls of 128 CTAs queue up at the few cache lines that the headers are
+// written to: 3500 clocks in that wait alone, against 1400 for 24 CTAs.)
+// Headers and reflectors alternate between two buffers.  A CTA overwrites a
+// buffer at stage s + 2 after it has seen every CTA's header of stage s + 1,
+// which each wrote after it had read stage s.
 // Tags grow over all launches of a call and the area is zeroed once per call.
 //
 // Measured on GB300 a stage, against two lanes a column and a counter barrier
-// (release add and spin, then all headers, then the column): FP32, 138 rows,
-// 16384 columns 5.5 -> 3.5 us, 3000 columns 5.2 -> 2.8; FP64, 74 rows, 2000
-// columns 9.7 -> 4.6 (of which 1.6 the reflector's FP64 scalars and sums).
+// (release add and spin, then all headers, then the column) -> with the
+// reflector built by everyone after the exchange -> this: FP32, 138 rows,
+// 16384 columns 5.5 -> 3.5 -> 3.2 us, 3000 columns 5.2 -> 2.8 -> 2.6; FP64, 74
+// rows, 2000 columns 9.7 -> 4.2 -> 3.5.
 //
 // T is the arithmetic of the reflector applications (the bulk of the FP64
 // work): double for the plain path, float for the mixed path, whose sketch is
@@ -315,7 +319,7 @@ struct RegArgs {
   int* npairs;
   int max_pairs;
   unsigned char* hdrs;  // [2][MAX_P copies][MAX_P] 16-byte headers
-  unsigned char* recs;  // [2][MAX_P] columns
+  unsigned char* recs;  // [2][MAX_P] reflectors
   unsigned tag0;        // stage s's tag is tag0 + s + 1
   int* err;
   unsigned spin_limit;
@@ -378,19 +382,21 @@ __device__ __forceinline__ void warp_best(long long& key, int& pos) {
   case 12: DO(12) case 13: DO(13) case 14: DO(14) case 15: DO(15)
 
 template <int CNT, int RPT, int LPC, typename T>
-__global__ void __launch_bounds__(CNT, 1) skinny_qrp_reg_kernel(RegArgs a) {
+__global__ void __launch_bounds__(CNT + 32, 1) skinny_qrp_reg_kernel(RegArgs a) {
   HQ_PDL_WAIT();
+  constexpr int POLLER = CNT / 32;     // the warp that exchanges; it holds no columns
   constexpr bool F32 = sizeof(T) == 4;
   constexpr int NC = CNT / LPC;        // columns per CTA
   constexpr int CE = 16 / LPC;         // entries of a lane per 16-row chunk
   constexpr int NCH = RPT / CE;
   constexpr int STR = RPT + 16 / (int)sizeof(T) * ((RPT * (int)sizeof(T)) % 128 == 0);  // no bank conflicts
-  constexpr int RLANE = (LPC * RPT + 31) / 32;  // rows per lane of the polling warp
+  constexpr int RLANE = (LPC * RPT + 31) / 32;  // rows per lane of one warp
   // The reflector stays in registers between its two uses where they suffice.
-  constexpr bool KEEP = RPT * (int)sizeof(T) <= (F32 ? 144 : 256);
+  constexpr bool KEEP = CNT <= 256 && RPT * (int)sizeof(T) <= 144;
   static_assert(RPT % CE == 0 && CE * sizeof(T) % 16 == 0 && NCH <= 16, "chunks");
   static_assert(NC % 32 == 0, "downdating threads fill whole warps");
   __shared__ __align__(16) T sv[LPC * STR];  // the reflector v, lane-major
+  __shared__ T sraw[LPC * RPT];              // the candidate's column, by rows
   __shared__ long long s_bk[NC / 32];
   __shared__ int s_bp[NC / 32];
   __shared__ int sflag[NC];
@@ -435,12 +441,12 @@ __global__ void __launch_bounds__(CNT, 1) skinny_qrp_reg_kernel(RegArgs a) {
         x[t] = (have && r < mY) ? (T)(src[r] * sc) : (T)0;
       }
     }
-    if (l == 0) {
+    if (l == 0 && c < NC) {
       snrm[c] = q;
       sflag[c] = ec;
     }
   }
-  for (int r = tid; r < LPC * STR; r += CNT) sv[r] = (T)0;
+  for (int r = tid; r < LPC * STR; r += CNT + 32) sv[r] = (T)0;
   if (tid == 0) s_dead = 0;
   __syncthreads();
 
@@ -467,8 +473,10 @@ __global__ void __launch_bounds__(CNT, 1) skinny_qrp_reg_kernel(RegArgs a) {
       }
     }
   };
-  // Write this CTA's best candidate for stage s (s_bk and s_bp complete): the
-  // warp that holds the column, or warp 0 when no column is active.
+  // Write this CTA's best candidate for stage s (s_bk and s_bp complete) and
+  // then the reflector it would give, by the warp that holds the column (a
+  // header alone, by warp 0, when no column is active).  Entry s of the record
+  // is tau, the entries below v's.
   auto publish = [&](int s) {
     long long k = s_bk[0];
     int p = s_bp[0];
@@ -477,22 +485,56 @@ __global__ void __launch_bounds__(CNT, 1) skinny_qrp_reg_kernel(RegArgs a) {
       if (better_key(s_bk[w], s_bp[w], k, p)) { k = s_bk[w]; p = s_bp[w]; }
     const unsigned tag = a.tag0 + (unsigned)s + 1u;
     const bool mine = k > -2 && have && mypos == p;
-    if (__any_sync(0xffffffffu, mine) || (k <= -2 && warp == 0)) {
-      unsigned char* h = a.hdrs + ((size_t)(s & 1) * MAX_P * MAX_P + cta) * 16;
-      const unsigned long long w1 = ((unsigned long long)tag << 32) | (unsigned)p;
+    const bool here = __any_sync(0xffffffffu, mine);
+    if (!here && !(k <= -2 && warp == 0)) return;
+    unsigned char* h = a.hdrs + ((size_t)(s & 1) * MAX_P * MAX_P + cta) * 16;
+    const unsigned long long w1 = ((unsigned long long)tag << 32) | (unsigned)p;
 #pragma unroll
-      for (int j = 0; j < HDR_LANE; ++j) {
-        const int q = lane + 32 * j;
-        if (32 * j < P && q < P) hq_st_word(h + (size_t)q * MAX_P * 16, (unsigned long long)k, w1);
-      }
-      if (mine) {
-        unsigned char* rec = a.recs + ((size_t)(s & 1) * MAX_P + cta) * rec_bytes;
+    for (int j = 0; j < HDR_LANE; ++j) {
+      const int q = lane + 32 * j;
+      if (32 * j < P && q < P) hq_st_word(h + (size_t)q * MAX_P * 16, (unsigned long long)k, w1);
+    }
+    if (!here) return;
+    if (mine) {
 #pragma unroll
-        for (int t = 0; t < RPT; ++t) {
-          const int r = LPC * t + l;
-          if (r >= s && r < mY) Tagged<T>::put(rec + (size_t)r * Tagged<T>::BYTES, x[t], tag);
-        }
+      for (int t = 0; t < RPT; ++t) sraw[LPC * t + l] = x[t];
+    }
+    __syncwarp();
+    // Tail norm, reflector, v = [1; scale * tail].  In FP32 the reflector of
+    // the scaled column is built directly (it does not depend on the column's
+    // scale): beta = -sign(alpha) sqrt(alpha^2 + q), tau = (beta - alpha) /
+    // beta, scale = 1 / (alpha - beta); tau = 0 for a zero tail.
+    const T al = sraw[s];
+    T z[RLANE], q = (T)0;
+#pragma unroll
+    for (int i = 0; i < RLANE; ++i) {
+      const int r = s + 1 + lane + 32 * i;
+      z[i] = r < mY ? sraw[r] : (T)0;
+    }
+#pragma unroll
+    for (int i = 0; i < RLANE; ++i)
+      if (s + 1 + 32 * i < mY) q = fma(z[i], z[i], q);
+    q = hq_warp_sum(q);
+    T tau, scale;
+    if constexpr (F32) {
+      tau = 0.f;
+      scale = 0.f;
+      if (q > 0.f) {
+        const float beta = -copysignf(sqrtf(fmaf(al, al, q)), al);
+        tau = (beta - al) / beta;
+        scale = 1.f / (al - beta);
       }
+    } else {
+      const HqReflector hr = hq_make_reflector_sq(al, q);
+      tau = hr.tau;
+      scale = hr.scale;
+    }
+    unsigned char* rec = a.recs + ((size_t)(s & 1) * MAX_P + cta) * rec_bytes;
+    if (lane == 0) Tagged<T>::put(rec + (size_t)s * Tagged<T>::BYTES, tau, tag);
+#pragma unroll
+    for (int i = 0; i < RLANE; ++i) {
+      const int r = s + 1 + lane + 32 * i;
+      if (r < mY) Tagged<T>::put(rec + (size_t)r * Tagged<T>::BYTES, scale * z[i], tag);
     }
   };
 
@@ -500,7 +542,7 @@ __global__ void __launch_bounds__(CNT, 1) skinny_qrp_reg_kernel(RegArgs a) {
   __syncthreads();
   publish(0);
   for (int s = 0; s < a.b; ++s) {
-    if (warp == 0) {
+    if (warp == POLLER) {
       const unsigned tag = a.tag0 + (unsigned)s + 1u;
       // Winner: every CTA reduces the same headers in the same way.
       const unsigned char* h0 = a.hdrs + ((size_t)(s & 1) * MAX_P + cta) * MAX_P * 16;
@@ -542,12 +584,12 @@ __global__ void __launch_bounds__(CNT, 1) skinny_qrp_reg_kernel(RegArgs a) {
       const unsigned who = __ballot_sync(0xffffffffu, bk == wk && bp == wp);
       const int wcta = __shfl_sync(0xffffffffu, bq, __ffs((int)who) - 1);
       const bool none = ok && wk <= -2;  // no active column anywhere: cannot happen for b <= N
-      // The winner's column, rows s (every lane) and s + 1 + lane + 32 i.
-      T al = (T)0, z[RLANE];
+      // The winner's tau, and v in rows s + 1 + lane + 32 i.
+      T tau = (T)0, z[RLANE];
       if (ok && !none) {
         const unsigned char* rec = a.recs + ((size_t)(s & 1) * MAX_P + wcta) * rec_bytes;
         for (;;) {
-          bool got = Tagged<T>::get(rec + (size_t)s * Tagged<T>::BYTES, tag, al);
+          bool got = Tagged<T>::get(rec + (size_t)s * Tagged<T>::BYTES, tag, tau);
 #pragma unroll
           for (int i = 0; i < RLANE; ++i) {
             const int r = s + 1 + lane + 32 * i;
@@ -566,34 +608,11 @@ __global__ void __launch_bounds__(CNT, 1) skinny_qrp_reg_kernel(RegArgs a) {
         }
       } else {
         if (lane == 0) s_win_pos = wp;
-        // Tail norm, reflector, v = [1; scale * tail].  In FP32 the reflector
-        // of the scaled column is built directly (it does not depend on the
-        // column's scale): beta = -sign(alpha) sqrt(alpha^2 + q), tau = (beta
-        // - alpha) / beta, scale = 1 / (alpha - beta); tau = 0 for a zero tail.
-        T q = (T)0;
-#pragma unroll
-        for (int i = 0; i < RLANE; ++i)
-          if (s + 1 + lane + 32 * i < mY) q = fma(z[i], z[i], q);
-        q = hq_warp_sum(q);
-        T tau, scale;
-        if constexpr (F32) {
-          tau = 0.f;
-          scale = 0.f;
-          if (q > 0.f) {
-            const float beta = -copysignf(sqrtf(fmaf(al, al, q)), al);
-            tau = (beta - al) / beta;
-            scale = 1.f / (al - beta);
-          }
-        } else {
-          const HqReflector hr = hq_make_reflector_sq(al, q);
-          tau = hr.tau;
-          scale = hr.scale;
-        }
         auto put = [&](int r, T v) { sv[(r & (LPC - 1)) * STR + r / LPC] = v; };
 #pragma unroll
         for (int i = 0; i < RLANE; ++i) {
           const int r = s + 1 + lane + 32 * i;
-          if (r < mY) put(r, scale * z[i]);
+          if (r < mY) put(r, z[i]);
         }
         if (lane == 0) {
           s_tau = tau;
@@ -784,7 +803,7 @@ static int launch_reg(cudaStream_t stream, const hq_device_info* dev, const SkAr
     const int z = hq_zero_words(stream, s.npairs, 1, nullptr, 0);
     if (z) return z;
     void* args[] = {&a};
-    const cudaError_t e = hq_launch_coop(sh.fn, dim3(P), dim3(sh.threads), args, 0, stream);
+    const cudaError_t e = hq_launch_coop(sh.fn, dim3(P), dim3(sh.threads + 32), args, 0, stream);
     hq_count_launches(1);
     return (int)e;
   }
