@@ -14,12 +14,11 @@
 // carries its level's weight.  Levels 0..3 each get a TMEM accumulator, exact
 // per 256-deep slice of K (integers below 2^24 in their unit); level 4 gets its
 // own; levels 5 and 6 need at most 2^-12 relative precision and share one.
-// All are drained every 256 K into float-float running sums (FP32 pairs, ~48
-// bits).  (Folding level 4 in as well measured 2^-47.5 instead of 2^-52: the
+// All are drained every 256 K into running sums: float-float (FP32 pairs, ~48
+// bits), or 64-bit integers where K is at most 256.  (Folding level 4 in as well measured 2^-47.5 instead of 2^-52: the
 // tensor core's FP32 accumulation loses more than IEEE rounding when products
 // of very different magnitude meet in one accumulator.)  Six accumulators
-// instead of seven leave TMEM room for 80-column tiles in the short-K kernel --
-// a tcgen05 BF16 MMA takes the same time for N = 64 as for N = 128.  The
+// instead of seven leave TMEM room for 80-column tiles.  The
 // result is recombined in FP64.  With S = 7 the product is accurate to about
 // 2^-52 relative to |A| |B| row/column-wise.
 //
@@ -33,7 +32,7 @@
 //
 // The GEMM kernels are warp-specialised: warp 20 issues the bulk copies into a
 // 3-stage (2 for seven digits) ring, one thread of warp 21 issues tcgen05.mma
-// (cta_group::1, kind::f16, 128 x 80 x 16) into TMEM, warps 0-19 drain TMEM
+// (cta_group::1, kind::f16, 128 x 80..240 x 16) into TMEM, warps 0-19 drain TMEM
 // (tcgen05.ld, five warps per 32-lane quadrant, 16 columns each) and write
 // the output.  Every wait is bounded; on expiry the
 // kernel records an error, waits (bounded) for its in-flight copies and MMAs,
@@ -52,7 +51,6 @@ constexpr int KB_PER_DRAIN = 8;  // 256 K elements
 constexpr int MAX_ACC = 6;  // levels 0..4 alone (0..3 exact), 5 and 6 shared
 
 __host__ __device__ constexpr int n_acc(int S) { return S < MAX_ACC ? S : MAX_ACC; }
-__device__ __forceinline__ int acc_of_level(int L) { return L < MAX_ACC - 1 ? L : MAX_ACC - 1; }
 __host__ __device__ inline uint32_t tmem_pow2(uint32_t c) {
   return c <= 32 ? 32u : (c <= 64 ? 64u : (c <= 128 ? 128u : (c <= 256 ? 256u : 512u)));
 }
@@ -528,6 +526,12 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* b) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(b)) : "memory");
 }
 
+// One arrival for the warp, after all its lanes.
+__device__ __forceinline__ void warp_arrive(uint64_t* b, int lane) {
+  __syncwarp();
+  if (lane == 0) mbar_arrive(b);
+}
+
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* b, unsigned bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(b)),
                "r"(bytes)
@@ -596,9 +600,6 @@ __device__ __forceinline__ double f32_scaled(float f, int ek, unsigned neg) {
   return (ex == 0 || e64 <= 0) ? 0.0 : __longlong_as_double(bits);
 }
 
-// Epilogue thread's share of a tile: TMEM lanes of its quadrant (one output
-// row each), EPI_COLS columns starting at col0.  Adds the nacc accumulators
-// of those columns into the float-float running sums.
 // 16 consecutive TMEM columns of this warp's 32 lanes (one load, one wait).
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
   uint32_t r[16];
@@ -615,24 +616,111 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
   for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
 }
 
-// One 16-column TMEM load per accumulator (EPI_COLS = 16): half the
-// load-and-wait round trips of 8-column loads, on the path the MMAs wait for.
-__device__ __forceinline__ void drain_tmem(uint32_t tacc, int nacc, float* hi, float* lo) {
+// The accumulators change hands in groups of ACC_GROUP, the first levels'
+// first: the MMAs finish them in that order (issue_block), each with a commit
+// on full[g], and the epilogue warps give each back on empty[g] as soon as it
+// is read.  So the first groups are drained while the last one is still being
+// added to, and the next MMAs start on the first ones while the last is
+// drained; handed over in one piece the tensor core idled through every drain.
+// A group is what one MMA can cover: three levels.  Over a 16384^2 mixed
+// factorization the products took 218 ms with one level an MMA, 188 with two
+// and 180 with three.
+constexpr int ACC_GROUP = 3;
+constexpr int MAX_GROUPS = MAX_ACC / ACC_GROUP;
+static_assert(MAX_ACC % ACC_GROUP == 0 && ACC_GROUP * TN <= 256, "one MMA covers a group");
+struct Handover {
+  uint64_t* full;   // [MAX_GROUPS]
+  uint64_t* empty;  // [MAX_GROUPS]
+};
+
+// Drains the nacc accumulators of this warp's 16 columns, take(q, values), as
+// the round'th use of the barriers; false (in every lane) if a wait gave up.
+template <typename Take>
+__device__ __forceinline__ bool drain_levels(uint32_t tacc, int nacc, Handover h, int round,
+                                             unsigned lim, volatile int* abort_flag, int lane,
+                                             Take take) {
   static_assert(EPI_COLS == 16, "one 16-column load per accumulator");
-  for (int q = 0; q < nacc; ++q) {
+#pragma unroll
+  for (int q = 0; q < MAX_ACC; ++q) {
+    if (q >= nacc) continue;
+    const int g = q / ACC_GROUP;
+    if (q % ACC_GROUP == 0) {
+      // One outcome per warp: TMEM loads are warp-wide.
+      if (!__all_sync(0xffffffffu, mbar_wait(&h.full[g], round & 1, lim, abort_flag)))
+        return false;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    }
     float v[16];
     tmem_ld16(tacc + (uint32_t)(q * TN), v);
-#pragma unroll
-    for (int j = 0; j < 16; ++j) ff_add(hi[j], lo[j], v[j]);
+    if (q % ACC_GROUP == ACC_GROUP - 1 || q == nacc - 1) {
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      warp_arrive(&h.empty[g], lane);
+    }
+    take(q, v);
   }
+  return true;
 }
 
-// Output of one row's EPI_COLS columns: out = sign * (hi + lo) * 2^(ea + eb - 14)
+// The running sums of a thread's 16 outputs.  Over any K: float-float pairs
+// (FloatSums).  Over K <= 256 (ExactSums): one 64-bit integer in units of 2^-40,
+// level 5's -- the accumulators of levels 0 to 4 are integers there, their
+// weighted sum stays below 2^63, and the shared accumulator of levels 5 and 6
+// is rounded to that unit.  That takes a few instructions an accumulator
+// instead of ten, makes the FP64 value on the integer pipe, which leaves
+// one FP64 addition an output instead of two, and errs less (1.9e-16 of the
+// product's norm against 5.9e-16, Gaussian operands, K = 64 to 256).
+struct FloatSums {
+  float hi[EPI_COLS], lo[EPI_COLS];
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int c = 0; c < EPI_COLS; ++c) hi[c] = lo[c] = 0.f;
+  }
+  __device__ __forceinline__ void add(int, const float* v) {
+#pragma unroll
+    for (int c = 0; c < EPI_COLS; ++c) ff_add(hi[c], lo[c], v[c]);
+  }
+  // sign * sum * 2^ek: the two exact conversions take no FP64 instruction,
+  // their sum one (exact: hi + lo fits in FP64).
+  __device__ __forceinline__ double value(int c, int ek, unsigned neg) const {
+    return f32_scaled(hi[c], ek, neg) + f32_scaled(lo[c], ek, neg);
+  }
+};
+
+struct ExactSums {
+  long long sum[EPI_COLS];
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int c = 0; c < EPI_COLS; ++c) sum[c] = 0;
+  }
+  __device__ __forceinline__ void add(int q, const float* v) {  // q: a constant once unrolled
+    const float unit = __uint_as_float((uint32_t)(127 + 8 * q) << 23);
+#pragma unroll
+    for (int c = 0; c < EPI_COLS; ++c)
+      sum[c] += (long long)__float2int_rn(v[c] * unit) * (1LL << (40 - 8 * q));
+  }
+  // sign * sum * 2^(ek - 40), rounded to FP64 (half away from zero); results
+  // below the FP64 normal range give 0.
+  __device__ __forceinline__ double value(int c, int ek, unsigned neg) const {
+    const long long v = sum[c];
+    const unsigned long long u = (unsigned long long)(v < 0 ? -v : v);
+    const int z = __clzll((long long)u);
+    const unsigned long long m = u << (z & 63);
+    const unsigned long long mant = (m >> 11) + ((m >> 10) & 1ull);
+    const int e = 63 - z + ek - 40 + 1023;  // of the leading bit, biased
+    unsigned long long bits = ((unsigned long long)(unsigned)(e - 1) << 52) + mant;
+    if (e >= 2047) bits = 0x7FFull << 52;
+    bits |= (unsigned long long)((unsigned)(v < 0) ^ neg) << 63;
+    return (u == 0ull || e <= 0) ? 0.0 : __longlong_as_double((long long)bits);
+  }
+};
+
+// Output of one row's EPI_COLS columns: out = sign * sum * 2^(ea + eb - 14)
 // (mode 0) or C += that (mode 1).  In update mode the row's C entries are
 // first prefetched into L2 (no registers held), then read in batches of 8
 // with every load of a batch issued before its stores.
+template <typename Sums>
 __device__ __forceinline__ void write_row(const OzkArgs& a, int r, int n0, double* crow,
-                                          const float* hi, const float* lo, bool live) {
+                                          const Sums& sums, bool live) {
   const unsigned neg = a.sign < 0.0 ? 1u : 0u;
   const int er = live ? a.ea[r] - 14 : 0;
   const bool counted = live && r >= a.row_lo;
@@ -658,9 +746,7 @@ __device__ __forceinline__ void write_row(const OzkArgs& a, int r, int n0, doubl
       const int n = n0 + c8 + j;
       fx[j] = 0u;
       if (live && n < a.N) {
-        // sign * (hi + lo) * 2^ek: the two exact conversions take no FP64
-        // instruction, their sum one (exact: hi + lo fits in FP64).
-        const double v = f32_scaled(hi[c8 + j], ek[j], neg) + f32_scaled(lo[c8 + j], ek[j], neg);
+        const double v = sums.value(c8 + j, ek[j], neg);
         const double out = a.mode == 0 ? v : cv[j] + v;
         crow[(long long)n * a.ccs] = out;
         if (counted) fx[j] = (unsigned)((__double_as_longlong(out) >> 52) & 0x7FF);
@@ -678,58 +764,62 @@ __device__ __forceinline__ void write_row(const OzkArgs& a, int r, int n0, doubl
 }
 
 // Digit-pair MMAs of one K block into the accumulators at tb: pair (s, t) into
-// acc_of_level(s + t).  fresh: bit q set = the next MMA into q overwrites.
-__device__ __forceinline__ void issue_block(uint32_t tb, uint64_t da0, uint64_t db0, int S,
-                                            uint32_t idesc, unsigned& fresh) {
-  for (int s = 0; s < S; ++s) {
-    const uint64_t da = da0 + (uint64_t)((s * A_TILE) >> 4);  // start address advances by bytes >> 4
-    for (int t = 0; s + t < S; ++t) {
-      const int q = acc_of_level(s + t);
-      const uint64_t db = db0 + (uint64_t)((t * B_TILE) >> 4);
+// acc_of_level(s + t).  The B digits of a stage follow one another in shared
+// memory and so do the accumulators in TMEM, so one MMA of N = n x TN columns
+// multiplies digit s of A with n consecutive digits of B into n consecutive
+// levels: an MMA costs at least 62 clocks, whatever its N up to 128, and 1/2
+// clock a column beyond, and reads its A tile from shared memory once.
+// FIRST: the accumulators restart -- each group is waited for (its round'th
+// hand-back) and overwritten; last: each group is committed once complete.
+// False if a wait gave up.
+template <int S, bool FIRST>
+__device__ __forceinline__ bool issue_pairs(uint32_t tb, uint64_t da0, uint64_t db0, int s_rt,
+                                            uint32_t idesc, bool last, Handover h, int round,
+                                            unsigned lim, volatile int* abort_flag) {
+  // S > 0: fully unrolled (every descriptor offset, TMEM column and accumulate
+  // flag a constant, so the single issuing thread spends its time on
+  // tcgen05.mma instead of loop and index arithmetic); S = 0: s_rt digits.
+  const int ns = S > 0 ? S : s_rt;
+  const int nacc = S > 0 ? n_acc(S) : n_acc(s_rt);
+#pragma unroll
+  for (int g = 0; g < MAX_GROUPS; ++g) {
+    const int lo = g * ACC_GROUP;
+    const int hi = lo + ACC_GROUP < nacc ? lo + ACC_GROUP : nacc;
+    if (lo >= nacc) continue;
+    if (FIRST) {
+      if (!mbar_wait(&h.empty[g], (round & 1) ^ 1, lim, abort_flag)) return false;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    }
+#pragma unroll
+    for (int s = 0; s < 7; ++s) {
 #pragma unroll
       for (int kk = 0; kk < TK / 16; ++kk) {
-        mma_bf16(tb + (uint32_t)(q * TN), da + 2 * kk, db + 2 * kk, idesc, ((fresh >> q) & 1u) ^ 1u);
-        fresh &= ~(1u << q);
+        const uint64_t da = da0 + (uint64_t)((s * A_TILE) >> 4) + 2 * kk;
+        if (s < hi) {
+          const int q0 = s > lo ? s : lo, n = hi - q0;
+          mma_bf16(tb + (uint32_t)(q0 * TN), da,
+                   db0 + (uint64_t)(((q0 - s) * B_TILE) >> 4) + 2 * kk,
+                   idesc + ((uint32_t)(n * TN >> 3) << 17), FIRST && s == 0 && kk == 0 ? 0u : 1u);
+        }
+        if (ns > nacc && hi == nacc && s < ns)  // level 6 shares the last accumulator
+          mma_bf16(tb + (uint32_t)((nacc - 1) * TN), da,
+                   db0 + (uint64_t)(((ns - 1 - s) * B_TILE) >> 4) + 2 * kk,
+                   idesc + ((uint32_t)(TN >> 3) << 17), 1u);
       }
     }
+    if (last) mma_commit(&h.full[g]);
   }
+  return true;
 }
 
-// The same for seven digits, fully unrolled: every descriptor offset, TMEM
-// column and accumulate flag is a constant, so the single issuing thread
-// spends its time on tcgen05.mma instead of loop and index arithmetic.
-// FIRST: the first K block after a drain (the first MMA into each
-// accumulator overwrites it; with seven digits every accumulator's first
-// pair has s = 0).
-template <bool FIRST>
-__device__ __forceinline__ void issue_block7(uint32_t tb, uint64_t da0, uint64_t db0,
-                                             uint32_t idesc) {
-  constexpr int S = 7;
-#pragma unroll
-  for (int s = 0; s < S; ++s) {
-#pragma unroll
-    for (int t = 0; t < S - s; ++t) {
-      const int L = s + t;
-      const int q = L < MAX_ACC - 1 ? L : MAX_ACC - 1;
-#pragma unroll
-      for (int kk = 0; kk < TK / 16; ++kk) {
-        const bool overwrite = FIRST && s == 0 && kk == 0 && t <= MAX_ACC - 1;
-        mma_bf16(tb + (uint32_t)(q * TN), da0 + (uint64_t)((s * A_TILE) >> 4) + 2 * kk,
-                 db0 + (uint64_t)((t * B_TILE) >> 4) + 2 * kk, idesc, overwrite ? 0u : 1u);
-      }
-    }
-  }
-}
-
-__device__ __forceinline__ void issue_any(uint32_t tb, uint64_t da0, uint64_t db0, int S,
-                                          uint32_t idesc, unsigned& fresh) {
-  if (S == 7) {
-    if (fresh == 0xFFu) issue_block7<true>(tb, da0, db0, idesc);
-    else issue_block7<false>(tb, da0, db0, idesc);
-    fresh = 0u;
-  } else {
-    issue_block(tb, da0, db0, S, idesc, fresh);
-  }
+__device__ __forceinline__ bool issue_block(uint32_t tb, uint64_t da0, uint64_t db0, int S,
+                                            uint32_t idesc, bool first, bool last, Handover h,
+                                            int round, unsigned lim, volatile int* abort_flag) {
+  if (S == 7)
+    return first ? issue_pairs<7, true>(tb, da0, db0, S, idesc, last, h, round, lim, abort_flag)
+                 : issue_pairs<7, false>(tb, da0, db0, S, idesc, last, h, round, lim, abort_flag);
+  return first ? issue_pairs<0, true>(tb, da0, db0, S, idesc, last, h, round, lim, abort_flag)
+               : issue_pairs<0, false>(tb, da0, db0, S, idesc, last, h, round, lim, abort_flag);
 }
 
 __global__ void __launch_bounds__(NT, 1) ozk_gemm_kernel(OzkArgs a,
@@ -738,7 +828,7 @@ __global__ void __launch_bounds__(NT, 1) ozk_gemm_kernel(OzkArgs a,
   HQ_PDL_WAIT();
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[MAX_STAGES], empty_bar[MAX_STAGES];
-  __shared__ __align__(8) uint64_t drain_full, drain_empty, done_bar;
+  __shared__ __align__(8) uint64_t acc_full[MAX_GROUPS], acc_empty[MAX_GROUPS], done_bar;
   __shared__ uint32_t tmem_base;
   __shared__ volatile int s_abort;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -753,15 +843,17 @@ __global__ void __launch_bounds__(NT, 1) ozk_gemm_kernel(OzkArgs a,
   const int mt = blockIdx.x, nt = blockIdx.y, z = blockIdx.z;
   const int kb0 = z * a.kb_per_z;
   const int nkb = min(a.KB - kb0, a.kb_per_z);
-  const int ndrain = nkb > 0 ? (nkb - 1) / KB_PER_DRAIN : 0;  // drains before the final one
+  const int ndrain = (nkb + KB_PER_DRAIN - 1) / KB_PER_DRAIN;
 
   if (tid == 0) {
     for (int i = 0; i < STAGES; ++i) {
       mbar_init(&full_bar[i], 1);
       mbar_init(&empty_bar[i], 1);
     }
-    mbar_init(&drain_full, 1);
-    mbar_init(&drain_empty, NEPI);
+    for (int g = 0; g < MAX_GROUPS; ++g) {
+      mbar_init(&acc_full[g], 1);
+      mbar_init(&acc_empty[g], NEPI / 32);
+    }
     mbar_init(&done_bar, 1);
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -777,7 +869,7 @@ __global__ void __launch_bounds__(NT, 1) ozk_gemm_kernel(OzkArgs a,
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tbase = tmem_base;
   const unsigned lim = a.spin_limit;
-  int mma_issued = 0;  // MMA thread: any tcgen05.mma issued
+  const Handover hand = {acc_full, acc_empty};
   int copies_issued = 0;
 
   if (warp == PRODUCER_WARP) {
@@ -798,10 +890,7 @@ __global__ void __launch_bounds__(NT, 1) ozk_gemm_kernel(OzkArgs a,
     }
   } else if (warp == MMA_WARP) {
     if (lane == 0) {
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TN >> 3) << 17) |
-                             ((uint32_t)(TM >> 4) << 24);
-      unsigned fresh = 0xFFu;
-      int d = 0;
+      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TM >> 4) << 24);
       for (int i = 0; i < nkb; ++i) {
         const int st = i % STAGES;
         if (!mbar_wait(&full_bar[st], (i / STAGES) & 1, lim, &s_abort)) {
@@ -809,56 +898,42 @@ __global__ void __launch_bounds__(NT, 1) ozk_gemm_kernel(OzkArgs a,
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        issue_any(tbase, sw64_desc(smem_u32(sA + st * a_stage)),
-                  sw64_desc(smem_u32(sB + st * b_stage)), S, idesc, fresh);
-        mma_issued = 1;
-        mma_commit(&empty_bar[st]);
-        if ((i + 1) % KB_PER_DRAIN == 0 && i + 1 < nkb) {
-          mma_commit(&drain_full);
-          if (!mbar_wait(&drain_empty, d & 1, lim, &s_abort)) {
-            s_abort = 1;
-            break;
-          }
-          ++d;
-          fresh = 0xFFu;  // every accumulator restarts after a drain
+        // Every accumulator restarts after a drain, every KB_PER_DRAIN blocks.
+        if (!issue_block(tbase, sw64_desc(smem_u32(sA + st * a_stage)),
+                         sw64_desc(smem_u32(sB + st * b_stage)), S, idesc, i % KB_PER_DRAIN == 0,
+                         (i + 1) % KB_PER_DRAIN == 0 || i + 1 == nkb, hand, i / KB_PER_DRAIN, lim,
+                         &s_abort)) {
+          s_abort = 1;
+          break;
         }
+        mma_commit(&empty_bar[st]);
       }
+      // Nothing of the tensor core's may arrive in shared memory after exit.
       mma_commit(&done_bar);
+      if (!mbar_wait(&done_bar, 0, lim, nullptr)) s_abort = 1;
     }
   } else {
     // Epilogue warps 0-19: TMEM lanes 32*(warp&3).. = tile rows, columns
     // (warp>>2)*EPI_COLS.. of the tile.
-    float hi[EPI_COLS], lo[EPI_COLS];
-#pragma unroll
-    for (int c = 0; c < EPI_COLS; ++c) {
-      hi[c] = 0.f;
-      lo[c] = 0.f;
-    }
+    FloatSums sums;
+    sums.clear();
     const int col0 = (warp >> 2) * EPI_COLS;
     const uint32_t tacc = tbase + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)col0;
     bool ok = true;
-    for (int d = 0; d < ndrain && ok; ++d) {
-      ok = mbar_wait(&drain_full, d & 1, lim, &s_abort);
-      if (!ok) break;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      drain_tmem(tacc, nacc, hi, lo);
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      mbar_arrive(&drain_empty);
-    }
-    if (ok) ok = mbar_wait(&done_bar, 0, lim, &s_abort);
+    for (int d = 0; d < ndrain && ok; ++d)
+      ok = drain_levels(tacc, nacc, hand, d, lim, &s_abort, lane,
+                        [&](int q, const float* v) { sums.add(q, v); });
     if (!ok) {
       s_abort = 1;
     } else {
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      drain_tmem(tacc, nacc, hi, lo);
       const int r = mt * TM + (warp & 3) * 32 + lane;
       if (r < a.M)
-        write_row(a, r, nt * TN + col0, a.C + (long long)r * a.crs + (long long)z * a.zstride, hi,
-                  lo, true);
+        write_row(a, r, nt * TN + col0, a.C + (long long)r * a.crs + (long long)z * a.zstride,
+                  sums, true);
     }
   }
 
-  // Teardown: on abort, wait (bounded) for in-flight copies and MMAs first.
+  // Teardown: on abort, wait (bounded) for in-flight copies first.
   __syncthreads();
   if (s_abort) {
     if (tid == 0) atomicCAS(a.err, 0, HQ_ERR_BARRIER_TIMEOUT);
@@ -867,10 +942,6 @@ __global__ void __launch_bounds__(NT, 1) ozk_gemm_kernel(OzkArgs a,
       // be in flight.
       for (int i = copies_issued > STAGES ? copies_issued - STAGES : 0; i < copies_issued; ++i)
         mbar_wait(&full_bar[i % STAGES], (i / STAGES) & 1, lim, nullptr);
-    }
-    if (warp == MMA_WARP && lane == 0 && mma_issued) {
-      // done_bar was committed after the loop; its completion covers all MMAs.
-      mbar_wait(&done_bar, 0, lim, nullptr);
     }
     __syncthreads();
   }
@@ -894,6 +965,8 @@ __global__ void __launch_bounds__(NT, 1) ozk_gemm_kernel(OzkArgs a,
 // 14 bytes of digits per entry and read back.  The digits are those
 // ozk_split_chunk_kernel writes.  A conversion barrier per stage orders the
 // digit writes (generic proxy, fenced to the async proxy) before the MMAs.
+// K <= 256 takes the sums that the short-K kernel takes (the last blocks of a
+// factorization), so both routes give the same bits there too.
 constexpr int C64_TILE = TN * TK * 8;  // 20 KB of FP64 per stage
 
 // One thread's share of a block's conversion: 4 consecutive K entries (h-th
@@ -940,6 +1013,7 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
       : "memory");
 }
 
+template <typename Sums>
 __global__ void __launch_bounds__(NT, 1) ozk_gemm_c64_kernel(
     OzkArgs a, const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmC) {
   HQ_PDL_WAIT();
@@ -952,7 +1026,7 @@ __global__ void __launch_bounds__(NT, 1) ozk_gemm_c64_kernel(
   // block i - 2's was converted, so its load never waits for the MMAs.
   __shared__ __align__(8) uint64_t a_full[MAX_STAGES], c_full[MAX_STAGES], c_empty[MAX_STAGES],
       empty_bar[MAX_STAGES], conv_bar[MAX_STAGES];
-  __shared__ __align__(8) uint64_t drain_full, drain_empty, done_bar;
+  __shared__ __align__(8) uint64_t acc_full[MAX_GROUPS], acc_empty[MAX_GROUPS], done_bar;
   __shared__ uint32_t tmem_base;
   __shared__ volatile int s_abort;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -967,18 +1041,19 @@ __global__ void __launch_bounds__(NT, 1) ozk_gemm_c64_kernel(
   const int mt = blockIdx.x, nt = blockIdx.y, z = blockIdx.z;
   const int kb0 = z * a.kb_per_z;
   const int nkb = min(a.KB - kb0, a.kb_per_z);
-  const int ndrain = nkb > 0 ? (nkb - 1) / KB_PER_DRAIN : 0;
 
   if (tid == 0) {
     for (int i = 0; i < STAGES; ++i) {
       mbar_init(&a_full[i], 1);
       mbar_init(&c_full[i], 1);
-      mbar_init(&c_empty[i], NEPI);
+      mbar_init(&c_empty[i], NEPI / 32);
       mbar_init(&empty_bar[i], 1);
-      mbar_init(&conv_bar[i], NEPI);
+      mbar_init(&conv_bar[i], NEPI / 32);
     }
-    mbar_init(&drain_full, 1);
-    mbar_init(&drain_empty, NEPI);
+    for (int g = 0; g < MAX_GROUPS; ++g) {
+      mbar_init(&acc_full[g], 1);
+      mbar_init(&acc_empty[g], NEPI / 32);
+    }
     mbar_init(&done_bar, 1);
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -994,7 +1069,7 @@ __global__ void __launch_bounds__(NT, 1) ozk_gemm_c64_kernel(
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tbase = tmem_base;
   const unsigned lim = a.spin_limit;
-  int mma_issued = 0;
+  const Handover hand = {acc_full, acc_empty};
   int a_issued = 0, c_issued = 0;  // producer lanes 0 and 1
 
   if (warp == PRODUCER_WARP) {
@@ -1023,10 +1098,7 @@ __global__ void __launch_bounds__(NT, 1) ozk_gemm_c64_kernel(
     }
   } else if (warp == MMA_WARP) {
     if (lane == 0) {
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TN >> 3) << 17) |
-                             ((uint32_t)(TM >> 4) << 24);
-      unsigned fresh = 0xFFu;
-      int d = 0;
+      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TM >> 4) << 24);
       for (int i = 0; i < nkb; ++i) {
         const int st = i % STAGES;
         if (!mbar_wait(&a_full[st], (i / STAGES) & 1, lim, &s_abort) ||
@@ -1035,30 +1107,23 @@ __global__ void __launch_bounds__(NT, 1) ozk_gemm_c64_kernel(
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        issue_any(tbase, sw64_desc(smem_u32(sA + st * a_stage)),
-                  sw64_desc(smem_u32(sB + st * b_stage)), S, idesc, fresh);
-        mma_issued = 1;
-        mma_commit(&empty_bar[st]);
-        if ((i + 1) % KB_PER_DRAIN == 0 && i + 1 < nkb) {
-          mma_commit(&drain_full);
-          if (!mbar_wait(&drain_empty, d & 1, lim, &s_abort)) {
-            s_abort = 1;
-            break;
-          }
-          ++d;
-          fresh = 0xFFu;
+        if (!issue_block(tbase, sw64_desc(smem_u32(sA + st * a_stage)),
+                         sw64_desc(smem_u32(sB + st * b_stage)), S, idesc, i % KB_PER_DRAIN == 0,
+                         (i + 1) % KB_PER_DRAIN == 0 || i + 1 == nkb, hand, i / KB_PER_DRAIN, lim,
+                         &s_abort)) {
+          s_abort = 1;
+          break;
         }
+        mma_commit(&empty_bar[st]);
       }
+      // Nothing of the tensor core's may arrive in shared memory after exit.
       mma_commit(&done_bar);
+      if (!mbar_wait(&done_bar, 0, lim, nullptr)) s_abort = 1;
     }
   } else {
     // Epilogue warps 0-19: convert every K block, drain every 256 K, write.
-    float hi[EPI_COLS], lo[EPI_COLS];
-#pragma unroll
-    for (int c = 0; c < EPI_COLS; ++c) {
-      hi[c] = 0.f;
-      lo[c] = 0.f;
-    }
+    Sums sums;
+    sums.clear();
     const int col0 = (warp >> 2) * EPI_COLS;
     const uint32_t tacc = tbase + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)col0;
     // Conversion task of this thread: column cc of the tile, quarter cq
@@ -1071,43 +1136,42 @@ __global__ void __launch_bounds__(NT, 1) ozk_gemm_c64_kernel(
       shift_base = 8 * S - 1076 - (n < a.N ? scale_of_raw(a.eb_raw[n]) : 0);
     }
     bool ok = true;
-    int d = 0;
+    auto drain = [&](int d) {
+      return drain_levels(tacc, nacc, hand, d, lim, &s_abort, lane,
+                          [&](int q, const float* v) { sums.add(q, v); });
+    };
     for (int i = 0; i < nkb && ok; ++i) {
       const int st = i % STAGES;
       // The FP64 tile is here, and the MMAs of block i - STAGES are done with
       // the B stage the digits go to.
-      ok = mbar_wait(&c_full[st], (i / STAGES) & 1, lim, &s_abort) &&
-           mbar_wait(&empty_bar[st], ((i / STAGES) & 1) ^ 1, lim, &s_abort);
+      ok = __all_sync(0xffffffffu,
+                      mbar_wait(&c_full[st], (i / STAGES) & 1, lim, &s_abort) &&
+                          mbar_wait(&empty_bar[st], ((i / STAGES) & 1) ^ 1, lim, &s_abort));
       if (!ok) break;
       convert_quarter<S>(reinterpret_cast<const double*>(sC + st * C64_TILE), sB + st * b_stage,
                          cc, cq, shift_base);
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      mbar_arrive(&conv_bar[st]);
-      mbar_arrive(&c_empty[st]);
-      if ((i + 1) % KB_PER_DRAIN == 0 && i + 1 < nkb && d < ndrain) {
-        ok = mbar_wait(&drain_full, d & 1, lim, &s_abort);
-        if (!ok) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        drain_tmem(tacc, nacc, hi, lo);
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        mbar_arrive(&drain_empty);
-        ++d;
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(&conv_bar[st]);
+        mbar_arrive(&c_empty[st]);
       }
+      // The drain of the K blocks before this one, after this one's digits are
+      // out: the MMAs that follow the drain find their operands ready.
+      if (i % KB_PER_DRAIN == 0 && i > 0) ok = drain(i / KB_PER_DRAIN - 1);
     }
-    if (ok) ok = mbar_wait(&done_bar, 0, lim, &s_abort);
+    if (ok && nkb > 0) ok = drain((nkb - 1) / KB_PER_DRAIN);
     if (!ok) {
       s_abort = 1;
     } else {
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      drain_tmem(tacc, nacc, hi, lo);
       const int r = mt * TM + (warp & 3) * 32 + lane;
       if (r < a.M)
-        write_row(a, r, nt * TN + col0, a.C + (long long)r * a.crs + (long long)z * a.zstride, hi,
-                  lo, true);
+        write_row(a, r, nt * TN + col0, a.C + (long long)r * a.crs + (long long)z * a.zstride,
+                  sums, true);
     }
   }
 
-  // Teardown: on abort, wait (bounded) for in-flight copies and MMAs first.
+  // Teardown: on abort, wait (bounded) for in-flight copies first.
   __syncthreads();
   if (s_abort) {
     if (tid == 0) atomicCAS(a.err, 0, HQ_ERR_BARRIER_TIMEOUT);
@@ -1119,7 +1183,6 @@ __global__ void __launch_bounds__(NT, 1) ozk_gemm_c64_kernel(
       for (int i = c_issued > STAGES ? c_issued - STAGES : 0; i < c_issued; ++i)
         mbar_wait(&c_full[i % STAGES], (i / STAGES) & 1, lim, nullptr);
     }
-    if (warp == MMA_WARP && lane == 0 && mma_issued) mbar_wait(&done_bar, 0, lim, nullptr);
     __syncthreads();
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -1142,7 +1205,7 @@ __global__ void __launch_bounds__(NT, 1) ozk_gemm_short_kernel(
   HQ_PDL_WAIT();
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[MAX_STAGES], empty_bar[MAX_STAGES];
-  __shared__ __align__(8) uint64_t tfull, tempty, done_bar;
+  __shared__ __align__(8) uint64_t acc_full[MAX_GROUPS], acc_empty[MAX_GROUPS], done_bar;
   __shared__ uint32_t tmem_base;
   __shared__ volatile int s_abort;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -1162,8 +1225,10 @@ __global__ void __launch_bounds__(NT, 1) ozk_gemm_short_kernel(
       mbar_init(&full_bar[i], 1);
       mbar_init(&empty_bar[i], 1);
     }
-    mbar_init(&tfull, 1);
-    mbar_init(&tempty, NEPI);
+    for (int g = 0; g < MAX_GROUPS; ++g) {
+      mbar_init(&acc_full[g], 1);
+      mbar_init(&acc_empty[g], NEPI / 32);
+    }
     mbar_init(&done_bar, 1);
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -1179,7 +1244,7 @@ __global__ void __launch_bounds__(NT, 1) ozk_gemm_short_kernel(
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tbase = tmem_base;
   const unsigned lim = a.spin_limit;
-  int mma_issued = 0;
+  const Handover hand = {acc_full, acc_empty};
   int copies_issued = 0;
 
   if (warp == PRODUCER_WARP) {
@@ -1202,69 +1267,52 @@ __global__ void __launch_bounds__(NT, 1) ozk_gemm_short_kernel(
     }
   } else if (warp == MMA_WARP) {
     if (lane == 0) {
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TN >> 3) << 17) |
-                             ((uint32_t)(TM >> 4) << 24);
+      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TM >> 4) << 24);
       int i = 0, lt = 0;
       for (int t = blockIdx.x; t < ntiles && !s_abort; t += gridDim.x, ++lt) {
-        if (!mbar_wait(&tempty, (lt & 1) ^ 1, lim, &s_abort)) {
-          s_abort = 1;
-          break;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        unsigned fresh = 0xFFu;
         bool ok = true;
-        for (int kb = 0; kb < nkb; ++kb, ++i) {
+        for (int kb = 0; kb < nkb && ok; ++kb, ++i) {
           const int st = i % STAGES;
-          if (!mbar_wait(&full_bar[st], (i / STAGES) & 1, lim, &s_abort)) {
-            ok = false;
-            break;
-          }
+          ok = mbar_wait(&full_bar[st], (i / STAGES) & 1, lim, &s_abort);
+          if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          issue_any(tbase, sw64_desc(smem_u32(sA + st * a_stage)),
-                    sw64_desc(smem_u32(sB + st * b_stage)), S, idesc, fresh);
-          mma_issued = 1;
-          mma_commit(&empty_bar[st]);
+          ok = issue_block(tbase, sw64_desc(smem_u32(sA + st * a_stage)),
+                           sw64_desc(smem_u32(sB + st * b_stage)), S, idesc, kb == 0,
+                           kb + 1 == nkb, hand, lt, lim, &s_abort);
+          if (ok) mma_commit(&empty_bar[st]);
         }
         if (!ok) {
           s_abort = 1;
           break;
         }
-        mma_commit(&tfull);
       }
+      // Nothing of the tensor core's may arrive in shared memory after exit.
       mma_commit(&done_bar);
+      if (!mbar_wait(&done_bar, 0, lim, nullptr)) s_abort = 1;
     }
   } else {
     const int col0 = (warp >> 2) * EPI_COLS;
     const uint32_t tacc = tbase + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)col0;
     int lt = 0;
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++lt) {
-      // One outcome per warp: the TMEM loads and the exponent reduction
-      // below are warp-wide, so no lane may leave the loop alone.
-      if (!__all_sync(0xffffffffu, mbar_wait(&tfull, lt & 1, lim, &s_abort))) {
+      ExactSums sums;
+      sums.clear();
+      // One outcome per warp: the TMEM loads and the exponent reduction are
+      // warp-wide, so no lane may leave the loop alone.
+      if (!drain_levels(tacc, nacc, hand, lt, lim, &s_abort, lane,
+                        [&](int q, const float* v) { sums.add(q, v); })) {
         s_abort = 1;
         break;
       }
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      float hi[EPI_COLS], lo[EPI_COLS];
-#pragma unroll
-      for (int c = 0; c < EPI_COLS; ++c) {
-        hi[c] = 0.f;
-        lo[c] = 0.f;
-      }
-      drain_tmem(tacc, nacc, hi, lo);
-      // The sums are in registers: hand the TMEM back for the next tile.
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      mbar_arrive(&tempty);
       const int mt = t / NTL, nt = t % NTL;
       const int r = mt * TM + (warp & 3) * 32 + lane;
       // Every lane takes part (the column-exponent reduction is warp-wide);
       // rows past M only skip their loads and stores.
-      write_row(a, r, nt * TN + col0, a.C + (long long)(r < a.M ? r : 0) * a.crs, hi, lo,
-                r < a.M);
+      write_row(a, r, nt * TN + col0, a.C + (long long)(r < a.M ? r : 0) * a.crs, sums, r < a.M);
     }
   }
 
-  // Teardown: on abort, wait (bounded) for in-flight copies and MMAs first.
+  // Teardown: on abort, wait (bounded) for in-flight copies first.
   __syncthreads();
   if (s_abort) {
     if (tid == 0) atomicCAS(a.err, 0, HQ_ERR_BARRIER_TIMEOUT);
@@ -1272,7 +1320,6 @@ __global__ void __launch_bounds__(NT, 1) ozk_gemm_short_kernel(
       for (int i = copies_issued > STAGES ? copies_issued - STAGES : 0; i < copies_issued; ++i)
         mbar_wait(&full_bar[i % STAGES], (i / STAGES) & 1, lim, nullptr);
     }
-    if (warp == MMA_WARP && lane == 0 && mma_issued) mbar_wait(&done_bar, 0, lim, nullptr);
     __syncthreads();
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -1613,10 +1660,12 @@ extern "C" int hq_ozk_gemm_c64(cudaStream_t stream, const hq_device_info* dev, i
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return (int)cudaErrorNotSupported;
   }
-  cudaError_t e = cudaFuncSetAttribute(ozk_gemm_c64_kernel,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const auto kernel =
+      KB <= KB_PER_DRAIN ? ozk_gemm_c64_kernel<ExactSums> : ozk_gemm_c64_kernel<FloatSums>;
+  cudaError_t e =
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  hq_launch(ozk_gemm_c64_kernel, dim3(MT, NTL, Z), NT, smem, stream, a, tmA, tmC);
+  hq_launch(kernel, dim3(MT, NTL, Z), NT, smem, stream, a, tmA, tmC);
   hq_count_launches(1);
   if (Z > 1) {
     long long total = (long long)M * N;
