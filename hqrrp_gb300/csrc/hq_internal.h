@@ -173,8 +173,8 @@ int hq_permute_cols(cudaStream_t stream, int rows, double* X, int ldx, int nc, c
  * mode 1 adds it; C element (r, c) at C[r*crs + c*ccs]; ws (optional) holds
  * split-K slices for mode 0. */
 size_t hq_ozk_tile_bytes(int rows, int K, int S, int side);
-/* raw (may be NULL): rows_total ints of scratch; when given, the two-pass
- * split of few long rows takes its row maxima with several CTAs per row. */
+/* raw: rows_total ints of scratch for the row maxima of rows of 512 or more,
+ * which take two passes. */
 int hq_ozk_split(cudaStream_t stream, const double* X, long long rs, long long ks, int R, int K,
                  int S, int side, void* tiles, int* exps, int* raw);
 /* Rows rounded up to the tile height of a side. */

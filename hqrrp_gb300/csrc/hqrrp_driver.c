@@ -1465,6 +1465,7 @@ HQ_API int hqrrp_gb300_ozaki_dgemm(char transa, char transb, int m, int n, int k
   w.ozB = ws_alloc(&w, ozk_b_bytes(n, k, slices));
   w.ozea = ws_alloc(&w, sizeof(int) * (size_t)(m + 128));
   w.ozeb = ws_alloc(&w, sizeof(int) * (size_t)(n + 128));
+  w.ozraw = ws_alloc(&w, sizeof(int) * (size_t)(imax(m, n) + 128));
   w.err = ws_alloc(&w, sizeof(int) * 2);
   if (w.failed) rc = HQ_E_NOMEM;
   if (!rc) {

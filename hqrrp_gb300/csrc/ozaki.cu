@@ -22,12 +22,12 @@
 // result is recombined in FP64.  With S = 7 the product is accurate to about
 // 2^-52 relative to |A| |B| row/column-wise.
 //
-// Layout: the split writes each operand as S plain K-major BF16 digit
-// matrices D[s][row][k] (rows padded to the tile height, K to 32).  The GEMM
-// kernels read them with tensor-map TMA loads (cp.async.bulk.tensor.3d): one
-// load per operand per pipeline stage brings a box of 32 K x tile rows x S
-// digits into shared memory, swizzled by the copy engine into the 64-byte
-// pattern the MMA descriptors name (rows of 64 B, 8-row atoms of 512 B).
+// Layout: the split writes each operand as the tiles the MMA descriptors
+// read: for each row tile and block of 32 K, S digit tiles of (tile rows) x 64
+// bytes one after the other, 64-byte swizzled (16-byte chunk c of row r at
+// chunk c ^ ((r >> 1) & 3); 8-row atoms of 512 B).  So a pipeline stage is one
+// contiguous bulk copy per operand; a tensor-map box of 64-byte rows out of
+// plain K-major digit matrices took a tenth longer per tile of a short product.
 // M tile 128 rows, N tile 80, K block 32.
 //
 // The GEMM kernels are warp-specialised: warp 20 issues the bulk copies into a
@@ -74,48 +74,82 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 // ---------------------------------------------------------------------------
 // Split
 
-// The fixed-point integer V = round(x * 2^(8S - 1 - e)) of one FP64 entry,
-// computed from its bits (no FP64 arithmetic); |V| <= 2^(8S-1).
-__device__ __forceinline__ long long fixed_point(double x, int shift_base) {
-  const long long bits = __double_as_longlong(x);
-  const int ex = (int)((bits >> 52) & 0x7FF);
-  if (ex == 0 || ex == 0x7FF) return 0;  // zeros and subnormals -> 0
-  const long long mant = (bits & 0xFFFFFFFFFFFFFLL) | (1LL << 52);
-  const int sh = ex + shift_base;
-  long long V = 0;
-  if (sh >= 0) V = mant << sh;
-  else if (sh > -63) V = (mant + (1LL << (-sh - 1))) >> (-sh);
-  return bits < 0 ? -V : V;
+// One FP64 entry's balanced base-256 digits in one word: W = V + 128 *
+// sum_p 256^p, where V = round(x * 2^(8S - 1 - e)) is the fixed-point integer
+// of a row of scale 2^e, |V| <= 2^(8S-1) (zeros, subnormals, infinities and
+// NaNs give V = 0).  Digit p < S-1 is byte p of W minus 128 and the top digit
+// W >> 8(S-1) minus 128 -- the same digits as peeling them from the bottom.
+// shift_base = 8S - 1076 - e, so V = mantissa * 2^(exponent field + shift_base);
+// the shift left by 3 leaves only right shifts, and one bit more than V to
+// round by.  The integer pipe is what bounds the conversions (the products
+// that cut their digits themselves spend as long on this as on their MMAs), so
+// this and digit_pair are written for few of its instructions.
+template <int S>
+__device__ __forceinline__ unsigned long long digit_word(double x, int shift_base) {
+  constexpr unsigned long long BIAS = 0x8080808080808080ULL >> (8 * (8 - S));
+  const int hi = __double2hiint(x);
+  const unsigned lo = (unsigned)__double2loint(x);
+  const int ex = (hi >> 20) & 0x7FF;
+  unsigned r = (unsigned)(2 - shift_base - ex);
+  if ((unsigned)(ex - 1) >= 2046u || r > 63u) r = 63u;
+  const unsigned mh = ((unsigned)hi & 0xFFFFFu) | 0x100000u;
+  const unsigned long long m = ((unsigned long long)((mh << 3) | (lo >> 29)) << 32) | (lo << 3);
+  const unsigned long long v = ((m >> r) + 1ull) >> 1;
+  const long long neg = hi >> 31;
+  return (v ^ (unsigned long long)neg) + (BIAS - (unsigned long long)neg);
 }
 
-// The same digit times 2^(-8s) for slice s, so that products carry their
-// level's weight: the FP32 pattern with exponent 23 - 8s and mantissa u is
-// 2^(23-8s) + u 2^(-8s) exactly, and subtracting 2^(23-8s) + 128 2^(-8s)
-// (exact in FP32) leaves (u - 128) 2^(-8s) in one add.
-__device__ __forceinline__ uint32_t digit_scaled(uint32_t u, int s) {
-  const float base = __uint_as_float(((uint32_t)(150 - 8 * s) << 23) | u);
-  const float off = __uint_as_float(((uint32_t)(150 - 8 * s) << 23) | 128u);
-  return __float_as_uint(__fsub_rn(base, off));
+// Digits S-1-s of two words, times 2^(-8s), as a pair of BF16: the FP32
+// pattern with exponent 23 - 8s and mantissa u is 2^(23-8s) + u 2^(-8s)
+// exactly, and subtracting 2^(23-8s) + 128 2^(-8s) (exact in FP32) leaves
+// (u - 128) 2^(-8s), exact in BF16, in one byte permutation and one addition.
+template <int S>
+__device__ __forceinline__ uint32_t digit_pair(unsigned long long w0, unsigned long long w1,
+                                               int s) {
+  const int p = S - 1 - s;
+  const uint32_t base = (uint32_t)(150 - 8 * s) << 23;  // only its top byte is set
+  uint32_t f0, f1;
+  if (s == 0) {  // the top digit: up to 9 bits
+    f0 = base | (uint32_t)(w0 >> (8 * p));
+    f1 = base | (uint32_t)(w1 >> (8 * p));
+  } else {
+    f0 = __byte_perm((uint32_t)(w0 >> (32 * (p / 4))), base, 0x7540 | (p & 3));
+    f1 = __byte_perm((uint32_t)(w1 >> (32 * (p / 4))), base, 0x7540 | (p & 3));
+  }
+  const float off = __uint_as_float(base | 128u);
+  const uint32_t d0 = __float_as_uint(__fsub_rn(__uint_as_float(f0), off));
+  const uint32_t d1 = __float_as_uint(__fsub_rn(__uint_as_float(f1), off));
+  return __byte_perm(d0, d1, 0x7632);
+}
+
+// The S digits of entries 8 ch .. 8 ch + 7 of row r, one 16-byte store each,
+// in the tile layout.
+template <int S>
+__device__ __forceinline__ void put_digits(const unsigned long long (&W)[8], uint8_t* tiles, int r,
+                                           int ch, int TR, int KB) {
+  const int rt = r / TR, ri = r - rt * TR;
+  uint8_t* base = tiles + ((long long)rt * KB + (ch >> 2)) * (S * TR * (TK * 2)) + ri * (TK * 2) +
+                  (((ch & 3) ^ ((ri >> 1) & 3)) << 4);
+#pragma unroll
+  for (int s = 0; s < S; ++s)
+    *reinterpret_cast<uint4*>(base + s * (TR * (TK * 2))) =
+        make_uint4(digit_pair<S>(W[0], W[1], s), digit_pair<S>(W[2], W[3], s),
+                   digit_pair<S>(W[4], W[5], s), digit_pair<S>(W[6], W[7], s));
 }
 
 // Rows r < R of X (element (r, k) at X[r*rs + k*ks], k < K) -> S digit tiles.
 // One warp per row; each lane takes 8-element chunks (one 16-byte group of a
 // tile row), so every digit is written with one 16-byte store.  Rows
-// R..RT*TR-1 and k >= K are written as zeros.  Balanced base-256 digits come
-// from W = V + 128 * sum_p 256^p: digit p < S-1 is byte p of W minus 128, the
-// top digit W >> 8(S-1) minus 128 (the same digits as peeling them from the
-// bottom); slice s holds digit p = S-1-s, the most significant first.
+// R..RT*TR-1 and k >= K are written as zeros.  Slice s holds digit p = S-1-s,
+// the most significant first.
 template <int S>
 __global__ void ozk_split_kernel(const double* __restrict__ X, long long rs, long long ks, int R,
                                  int K, int TR, int KB, int rows_total,
                                  uint8_t* __restrict__ tiles, int* __restrict__ exps) {
   HQ_PDL_WAIT();
-  constexpr unsigned long long BIAS = 0x8080808080808080ULL >> (8 * (8 - S));
   const int lane = threadIdx.x & 31;
   const int warps = blockDim.x >> 5;
   const int nchunk = KB * (TK / 8);
-  const long long kp = (long long)KB * TK;
-  const long long slice_bytes = (long long)rows_total * kp * 2;
   for (int r = blockIdx.x * warps + (threadIdx.x >> 5); r < rows_total;
        r += gridDim.x * warps) {
     const bool live = r < R;
@@ -141,31 +175,9 @@ __global__ void ozk_split_kernel(const double* __restrict__ X, long long rs, lon
       unsigned long long W[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        const long long V =
-            (live && k0 + j < K) ? fixed_point(xr[(long long)(k0 + j) * ks], shift_base) : 0;
-        W[j] = (unsigned long long)V + BIAS;
+        W[j] = digit_word<S>((live && k0 + j < K) ? xr[(long long)(k0 + j) * ks] : 0.0, shift_base);
       }
-      uint8_t* base = tiles + ((long long)r * kp + k0) * 2;
-#pragma unroll
-      for (int s = 0; s < S; ++s) {
-        // Slice s holds digit position p = S-1-s (slice 0 the most significant).
-        const int p = S - 1 - s;
-        uint32_t w[4];
-#pragma unroll
-        for (int j = 0; j < 8; j += 2) {
-          uint32_t u0, u1;
-          if (p == S - 1) {
-            u0 = (uint32_t)(W[j] >> (8 * p));
-            u1 = (uint32_t)(W[j + 1] >> (8 * p));
-          } else {
-            u0 = (uint32_t)(W[j] >> (8 * p)) & 255u;
-            u1 = (uint32_t)(W[j + 1] >> (8 * p)) & 255u;
-          }
-          w[j >> 1] = __byte_perm(digit_scaled(u0, s), digit_scaled(u1, s), 0x7632);
-        }
-        *reinterpret_cast<uint4*>(base + (long long)s * slice_bytes) =
-            make_uint4(w[0], w[1], w[2], w[3]);
-      }
+      put_digits<S>(W, tiles, r, ch, TR, KB);
     }
   }
 }
@@ -175,21 +187,18 @@ __global__ void ozk_split_kernel(const double* __restrict__ X, long long rs, lon
 // per entry, so a CTA first stages 32 consecutive rows x K in shared memory
 // with coalesced loads (one warp load = 32 consecutive rows of one column),
 // then splits each row exactly as ozk_split_kernel does (same digits and
-// exponents), one warp per row.
+// exponents), the maxima one warp per row, the digits four lanes a tile row.
 constexpr int CM_KMAX = 128;
 template <int S>
 __global__ void __launch_bounds__(256) ozk_split_cm_kernel(const double* __restrict__ X,
-                                                           long long ks, int R, int K, int KB,
-                                                           int rows_total,
+                                                           long long ks, int R, int K, int TR,
+                                                           int KB, int rows_total,
                                                            uint8_t* __restrict__ tiles,
                                                            int* __restrict__ exps) {
   HQ_PDL_WAIT();
-  constexpr unsigned long long BIAS = 0x8080808080808080ULL >> (8 * (8 - S));
   __shared__ double tile[CM_KMAX][33];
+  __shared__ int s_e[32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nchunk = KB * (TK / 8);
-  const long long kp = (long long)KB * TK;
-  const long long slice_bytes = (long long)rows_total * kp * 2;
   const int r0 = blockIdx.x * 32;
   for (int k = warp; k < K; k += 8) {
     const int r = r0 + lane;
@@ -199,57 +208,36 @@ __global__ void __launch_bounds__(256) ozk_split_cm_kernel(const double* __restr
   for (int rr = warp; rr < 32; rr += 8) {
     const int r = r0 + rr;
     if (r >= rows_total) break;
-    const bool live = r < R;
     long long mb = 0;
-    if (live)
-      for (int k = lane; k < K; k += 32) {
-        const long long bb = __double_as_longlong(tile[k][rr]) & 0x7FFFFFFFFFFFFFFFLL;
-        mb = bb > mb ? bb : mb;
-      }
+    for (int k = lane; k < K; k += 32) {
+      const long long bb = __double_as_longlong(tile[k][rr]) & 0x7FFFFFFFFFFFFFFFLL;
+      mb = bb > mb ? bb : mb;
+    }
     for (int o = 16; o > 0; o >>= 1) {
       const long long ob = __shfl_xor_sync(0xffffffffu, mb, o);
       mb = ob > mb ? ob : mb;
     }
     const int bexp = (int)(mb >> 52);
     const int e = bexp == 0 ? 0 : bexp - 1022;
-    if (lane == 0) exps[r] = e;
-    const int shift_base = 8 * S - 1076 - e;
-    for (int ch = lane; ch < nchunk; ch += 32) {
-      const int k0 = ch * 8;
-      unsigned long long W[8];
+    if (lane == 0) exps[r] = s_e[rr] = e;
+  }
+  __syncthreads();
+  for (int it = threadIdx.x; it < KB * 128; it += 256) {
+    const int rr = (it >> 2) & 31, ch = (it >> 7) * 4 + (it & 3), r = r0 + rr;
+    if (r >= rows_total) continue;
+    const int shift_base = 8 * S - 1076 - s_e[rr];
+    unsigned long long W[8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const long long V = (live && k0 + j < K) ? fixed_point(tile[k0 + j][rr], shift_base) : 0;
-        W[j] = (unsigned long long)V + BIAS;
-      }
-      uint8_t* base = tiles + ((long long)r * kp + k0) * 2;
-#pragma unroll
-      for (int s = 0; s < S; ++s) {
-        const int p = S - 1 - s;
-        uint32_t w[4];
-#pragma unroll
-        for (int j = 0; j < 8; j += 2) {
-          uint32_t u0, u1;
-          if (p == S - 1) {
-            u0 = (uint32_t)(W[j] >> (8 * p));
-            u1 = (uint32_t)(W[j + 1] >> (8 * p));
-          } else {
-            u0 = (uint32_t)(W[j] >> (8 * p)) & 255u;
-            u1 = (uint32_t)(W[j + 1] >> (8 * p)) & 255u;
-          }
-          w[j >> 1] = __byte_perm(digit_scaled(u0, s), digit_scaled(u1, s), 0x7632);
-        }
-        *reinterpret_cast<uint4*>(base + (long long)s * slice_bytes) =
-            make_uint4(w[0], w[1], w[2], w[3]);
-      }
-    }
+    for (int j = 0; j < 8; ++j)
+      W[j] = digit_word<S>(ch * 8 + j < K ? tile[ch * 8 + j][rr] : 0.0, shift_base);
+    put_digits<S>(W, tiles, r, ch, TR, KB);
   }
 }
 
 // Largest exponent field of each row, several CTAs per row (ROWMAX_SPAN
 // entries each, eight loads in flight per thread) raising raw[r] -- zeroed
-// before -- with an integer atomicMax: the first pass of the two-pass split
-// for few long rows, which one CTA per row left latency-bound.
+// before -- with an integer atomicMax: the first pass of the split of long
+// rows.
 constexpr int ROWMAX_SPAN = 2048;
 __global__ void __launch_bounds__(256) ozk_rowmax_atomic_kernel(const double* __restrict__ X,
                                                                 long long rs, long long ks, int K,
@@ -281,157 +269,55 @@ __global__ void __launch_bounds__(256) ozk_rowmax_atomic_kernel(const double* __
   }
 }
 
-// One-pass variant for long rows (4096 <= K <= 16384 with 512 threads): one
-// CTA per row holds the row in registers (CPT chunks of 8 per thread), takes
-// the block maximum and writes the digits, so every entry is read from
-// memory once (the two-pass kernel above re-reads each row, which misses L2
-// when many long rows are in flight).  Same output as the kernel above.
-template <int S, int CPT>
-__global__ void __launch_bounds__(512) ozk_split_row_kernel(
-    const double* __restrict__ X, long long rs, long long ks, int R, int K, int TR, int KB,
-    int rows_total, uint8_t* __restrict__ tiles, int* __restrict__ exps) {
+// The same for column-major operands (row stride 1): 32 rows a CTA, a row a
+// lane, so that a warp's loads are contiguous.
+constexpr int ROWMAX_CM_SPAN = 512;
+__global__ void __launch_bounds__(256) ozk_rowmax_cm_kernel(const double* __restrict__ X,
+                                                            long long ks, int R, int K,
+                                                            int* __restrict__ raw) {
   HQ_PDL_WAIT();
-  constexpr unsigned long long BIAS = 0x8080808080808080ULL >> (8 * (8 - S));
-  constexpr int NTH = 512;
-  __shared__ long long s_max[NTH / 32];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int nchunk = KB * (TK / 8);
-  const long long kp = (long long)KB * TK;
-  const long long slice_bytes = (long long)rows_total * kp * 2;
-  for (int r = blockIdx.x; r < rows_total; r += gridDim.x) {
-    const bool live = r < R;
-    const double* xr = X + (live ? (long long)r * rs : 0);
-    double v[CPT][8];
-    long long mb = 0;
-    // Contiguous, 16-byte aligned rows are read with 16-byte loads.
-    const bool vec = ks == 1 && ((reinterpret_cast<uintptr_t>(xr) & 15) == 0);
+  __shared__ int s_max[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int r = blockIdx.x * 32 + lane;
+  const int k1 = min(K, (int)(blockIdx.y + 1) * ROWMAX_CM_SPAN);
+  int m = 0;
+  if (r < R) {
+    const int* xr = reinterpret_cast<const int*>(X + r) + 1;  // the upper word
+#pragma unroll 8
+    for (int k = blockIdx.y * ROWMAX_CM_SPAN + warp; k < k1; k += 8)
+      m = max(m, (xr[(long long)k * ks * 2] >> 20) & 0x7FF);
+  }
+  s_max[warp][lane] = m;
+  __syncthreads();
+  if (warp == 0 && r < R) {
 #pragma unroll
-    for (int i = 0; i < CPT; ++i) {
-      const int k0 = (tid + i * NTH) * 8;
-      if (vec && live && k0 + 8 <= K) {
-        const double2* p2 = reinterpret_cast<const double2*>(xr + k0);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const double2 d = p2[j];
-          v[i][2 * j] = d.x;
-          v[i][2 * j + 1] = d.y;
-        }
-      } else {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[i][j] = (live && k0 + j < K) ? xr[(long long)(k0 + j) * ks] : 0.0;
-      }
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const long long bb = __double_as_longlong(v[i][j]) & 0x7FFFFFFFFFFFFFFFLL;
-        mb = bb > mb ? bb : mb;
-      }
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      const long long ob = __shfl_xor_sync(0xffffffffu, mb, o);
-      mb = ob > mb ? ob : mb;
-    }
-    if (lane == 0) s_max[warp] = mb;
-    __syncthreads();
-    mb = s_max[0];
-#pragma unroll
-    for (int w = 1; w < NTH / 32; ++w) mb = s_max[w] > mb ? s_max[w] : mb;
-    __syncthreads();  // s_max is rewritten for the next row
-    const int bexp = (int)(mb >> 52);
-    const int e = bexp == 0 ? 0 : bexp - 1022;
-    if (tid == 0) exps[r] = e;
-    const int shift_base = 8 * S - 1076 - e;
-#pragma unroll
-    for (int i = 0; i < CPT; ++i) {
-      const int ch = tid + i * NTH;
-      if (ch >= nchunk) continue;
-      unsigned long long W[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) W[j] = (unsigned long long)fixed_point(v[i][j], shift_base) + BIAS;
-      const int k0 = ch * 8;
-      uint8_t* base = tiles + ((long long)r * kp + k0) * 2;
-#pragma unroll
-      for (int s = 0; s < S; ++s) {
-        const int p = S - 1 - s;
-        uint32_t w[4];
-#pragma unroll
-        for (int j = 0; j < 8; j += 2) {
-          uint32_t u0, u1;
-          if (p == S - 1) {
-            u0 = (uint32_t)(W[j] >> (8 * p));
-            u1 = (uint32_t)(W[j + 1] >> (8 * p));
-          } else {
-            u0 = (uint32_t)(W[j] >> (8 * p)) & 255u;
-            u1 = (uint32_t)(W[j + 1] >> (8 * p)) & 255u;
-          }
-          w[j >> 1] = __byte_perm(digit_scaled(u0, s), digit_scaled(u1, s), 0x7632);
-        }
-        *reinterpret_cast<uint4*>(base + (long long)s * slice_bytes) =
-            make_uint4(w[0], w[1], w[2], w[3]);
-      }
-    }
+    for (int w = 1; w < 8; ++w) m = max(m, s_max[w][lane]);
+    if (m != 0) atomicMax(raw + r, m);
   }
 }
 
-// Long rows (K > 16384): the row does not fit the registers of one CTA, so
-// the split takes two streaming passes -- the per-row scale exponent first,
-// then every 8-element chunk of every row independently (consecutive threads
-// take consecutive chunks of a row: coalesced 64-byte loads, 512-byte digit
-// stores per warp and slice).  Same output as the kernels above.
-__global__ void __launch_bounds__(256) ozk_rowmax_kernel(const double* __restrict__ X,
-                                                         long long rs, long long ks, int R, int K,
-                                                         int rows_total, int* __restrict__ exps) {
-  HQ_PDL_WAIT();
-  __shared__ long long s_max[8];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int r = blockIdx.x; r < rows_total; r += gridDim.x) {
-    long long mb = 0;
-    if (r < R) {
-      const double* xr = X + (long long)r * rs;
-      for (int k = tid; k < K; k += 256) {
-        const long long bb = __double_as_longlong(xr[(long long)k * ks]) & 0x7FFFFFFFFFFFFFFFLL;
-        mb = bb > mb ? bb : mb;
-      }
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      const long long ob = __shfl_xor_sync(0xffffffffu, mb, o);
-      mb = ob > mb ? ob : mb;
-    }
-    if (lane == 0) s_max[warp] = mb;
-    __syncthreads();
-    if (tid == 0) {
-      for (int w = 1; w < 8; ++w) mb = s_max[w] > mb ? s_max[w] : mb;
-      mb = s_max[0] > mb ? s_max[0] : mb;
-      const int bexp = (int)(mb >> 52);
-      exps[r] = bexp == 0 ? 0 : bexp - 1022;
-    }
-    __syncthreads();
-  }
-}
-
+// Long rows: with the rows' largest exponent fields known (from the kernels
+// above, or from the epilogue of the update that wrote X), every 8-element
+// chunk independently -- a warp takes a K block of 8 rows: 256-byte loads (64
+// down a column), 512-byte digit stores per slice.
 template <int S>
 __global__ void __launch_bounds__(256) ozk_split_chunk_kernel(
-    const double* __restrict__ X, long long rs, long long ks, int R, int K, int KB, int rows_total,
-    uint8_t* __restrict__ tiles, int* __restrict__ exps, const int* __restrict__ raw) {
+    const double* __restrict__ X, long long rs, long long ks, int R, int K, int TR, int KB,
+    int rows_total, uint8_t* __restrict__ tiles, int* __restrict__ exps,
+    const int* __restrict__ raw) {
   HQ_PDL_WAIT();
-  constexpr unsigned long long BIAS = 0x8080808080808080ULL >> (8 * (8 - S));
-  const int nchunk = KB * (TK / 8);
-  const long long kp = (long long)KB * TK;
-  const long long slice_bytes = (long long)rows_total * kp * 2;
-  const long long total = (long long)rows_total * nchunk;
+  static_assert(TK == 32, "four chunks a K block");
+  const long long total = (long long)rows_total * KB * (TK / 8);
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
-    const int r = (int)(idx / nchunk), ch = (int)(idx % nchunk);
-    const int k0 = ch * 8;
+    const long long grp = idx >> 5;  // K block kb of 8 rows
+    const int kb = (int)(grp % KB), r = (int)(grp / KB) * 8 + (((int)idx >> 2) & 7);
+    const int ch = kb * 4 + ((int)idx & 3), k0 = ch * 8;
     const bool live = r < R;
     const double* xr = X + (live ? (long long)r * rs : 0);
-    int e;
-    if (raw != nullptr) {  // the rows' largest exponent fields, known in advance
-      const int bexp = live ? raw[r] : 0;
-      e = bexp == 0 ? 0 : bexp - 1022;
-      if (ch == 0) exps[r] = e;
-    } else {
-      e = exps[r];
-    }
+    const int bexp = live ? raw[r] : 0;
+    const int e = bexp == 0 ? 0 : bexp - 1022;
+    if (ch == 0) exps[r] = e;
     const int shift_base = 8 * S - 1076 - e;
     double v[8];
     if (live && ks == 1 && k0 + 8 <= K && ((reinterpret_cast<uintptr_t>(xr + k0) & 15) == 0)) {
@@ -448,26 +334,8 @@ __global__ void __launch_bounds__(256) ozk_split_chunk_kernel(
     }
     unsigned long long W[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) W[j] = (unsigned long long)fixed_point(v[j], shift_base) + BIAS;
-    uint8_t* base = tiles + ((long long)r * kp + k0) * 2;
-#pragma unroll
-    for (int s = 0; s < S; ++s) {
-      const int p = S - 1 - s;
-      uint32_t w[4];
-#pragma unroll
-      for (int j = 0; j < 8; j += 2) {
-        uint32_t u0, u1;
-        if (p == S - 1) {
-          u0 = (uint32_t)(W[j] >> (8 * p));
-          u1 = (uint32_t)(W[j + 1] >> (8 * p));
-        } else {
-          u0 = (uint32_t)(W[j] >> (8 * p)) & 255u;
-          u1 = (uint32_t)(W[j + 1] >> (8 * p)) & 255u;
-        }
-        w[j >> 1] = __byte_perm(digit_scaled(u0, s), digit_scaled(u1, s), 0x7632);
-      }
-      *reinterpret_cast<uint4*>(base + (long long)s * slice_bytes) = make_uint4(w[0], w[1], w[2], w[3]);
-    }
+    for (int j = 0; j < 8; ++j) W[j] = digit_word<S>(v[j], shift_base);
+    put_digits<S>(W, tiles, r, ch, TR, KB);
   }
 }
 
@@ -475,8 +343,8 @@ __global__ void __launch_bounds__(256) ozk_split_chunk_kernel(
 // GEMM
 
 struct OzkArgs {
-  const uint8_t* A;  // M-side tiles [MT][KB][S][TM x TK]
-  const uint8_t* B;  // N-side tiles [NTL][KB][S][TN x TK]
+  const uint8_t* A;  // M-side tiles [MT][KB][S][TM x TK], 16-byte aligned
+  const uint8_t* B;  // N-side tiles [NTL][KB][S][TN x TK], 16-byte aligned
   const int* ea;
   const int* eb;
   int M, N, S, KB;
@@ -526,6 +394,17 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* b) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(b)) : "memory");
 }
 
+// mbar_wait by a whole warp, with one outcome.
+__device__ __forceinline__ bool warp_wait(uint64_t* b, unsigned parity, unsigned limit,
+                                          volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, mbar_wait(b, parity, limit, abort_flag));
+}
+
+// The warp's index, known to be the same in all its lanes.
+__device__ __forceinline__ int uniform_warp() {
+  return __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0);
+}
+
 // One arrival for the warp, after all its lanes.
 __device__ __forceinline__ void warp_arrive(uint64_t* b, int lane) {
   __syncwarp();
@@ -538,14 +417,14 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* b, unsigned bytes) {
                : "memory");
 }
 
-// One box of a 3-D tensor map (k, row, digit) into shared memory, completing
-// on the mbarrier; x = k must be a multiple of 8 (16 bytes of BF16).
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z,
-                                            uint64_t* bar) {
+// bytes (a multiple of 16, both addresses 16-byte aligned) into shared memory,
+// completing on the mbarrier.
+__device__ __forceinline__ void bulk_load(void* dst, const uint8_t* src, unsigned bytes,
+                                          uint64_t* bar) {
   asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+          smem_u32(dst)),
+      "l"(src), "r"(bytes), "r"(smem_u32(bar))
       : "memory");
 }
 
@@ -559,19 +438,25 @@ __device__ __forceinline__ uint64_t sw64_desc(uint32_t saddr) {
   return d;
 }
 
+// The MMA warp runs as a whole and elects the thread that issues (always the
+// same one): its operands are then known to be uniform.  One thread on its own
+// took 3200 clocks to issue a K block's MMAs beside busy converting warps,
+// which take 2650.
 __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t ad, uint64_t bd, uint32_t idesc,
                                          uint32_t acc) {
   asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d_tmem),
+      "{\n .reg .pred p, q;\n setp.ne.b32 p, %4, 0;\n elect.sync _|q, 0xffffffff;\n"
+      " @q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d_tmem),
       "l"(ad), "l"(bd), "r"(idesc), "r"(acc)
       : "memory");
 }
 
 __device__ __forceinline__ void mma_commit(uint64_t* b) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   smem_u32(b))
-               : "memory");
+  asm volatile(
+      "{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n"
+      " @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}" ::"r"(
+          smem_u32(b))
+      : "memory");
 }
 
 // (hi, lo) += x in FP32 pairs (TwoSum, then renormalise).
@@ -646,8 +531,7 @@ __device__ __forceinline__ bool drain_levels(uint32_t tacc, int nacc, Handover h
     const int g = q / ACC_GROUP;
     if (q % ACC_GROUP == 0) {
       // One outcome per warp: TMEM loads are warp-wide.
-      if (!__all_sync(0xffffffffu, mbar_wait(&h.full[g], round & 1, lim, abort_flag)))
-        return false;
+      if (!warp_wait(&h.full[g], round & 1, lim, abort_flag)) return false;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     }
     float v[16];
@@ -692,75 +576,115 @@ struct ExactSums {
 #pragma unroll
     for (int c = 0; c < EPI_COLS; ++c) sum[c] = 0;
   }
-  __device__ __forceinline__ void add(int q, const float* v) {  // q: a constant once unrolled
+  // q: a constant once unrolled.  Levels 0 and 1 only touch the upper word;
+  // the others are wide multiply-adds, off the integer pipe.
+  __device__ __forceinline__ void add(int q, const float* v) {
     const float unit = __uint_as_float((uint32_t)(127 + 8 * q) << 23);
 #pragma unroll
-    for (int c = 0; c < EPI_COLS; ++c)
-      sum[c] += (long long)__float2int_rn(v[c] * unit) * (1LL << (40 - 8 * q));
+    for (int c = 0; c < EPI_COLS; ++c) {
+      const int i = __float2int_rn(v[c] * unit);
+      if (q < 2)
+        sum[c] += (long long)((unsigned long long)(unsigned)(q == 0 ? i * 256 : i) << 32);
+      else
+        asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(sum[c]) : "r"(i), "r"(1 << (40 - 8 * q)));
+    }
   }
   // sign * sum * 2^(ek - 40), rounded to FP64 (half away from zero); results
   // below the FP64 normal range give 0.
   __device__ __forceinline__ double value(int c, int ek, unsigned neg) const {
     const long long v = sum[c];
     const unsigned long long u = (unsigned long long)(v < 0 ? -v : v);
-    const int z = __clzll((long long)u);
-    const unsigned long long m = u << (z & 63);
-    const unsigned long long mant = (m >> 11) + ((m >> 10) & 1ull);
-    const int e = 63 - z + ek - 40 + 1023;  // of the leading bit, biased
-    unsigned long long bits = ((unsigned long long)(unsigned)(e - 1) << 52) + mant;
-    if (e >= 2047) bits = 0x7FFull << 52;
-    bits |= (unsigned long long)((unsigned)(v < 0) ^ neg) << 63;
-    return (u == 0ull || e <= 0) ? 0.0 : __longlong_as_double((long long)bits);
+    unsigned h = (unsigned)(u >> 32), l = (unsigned)u;
+    int e = ek + 1045;  // biased exponent - 1 of a leading bit 63
+    const bool low = h == 0u;
+    h = low ? l : h;
+    l = low ? 0u : l;
+    e -= low ? 32 : 0;
+    const int z = __clz((int)h);
+    h = __funnelshift_l(l, h, z);
+    l <<= z & 31;
+    e -= z;
+    const unsigned sign = ((unsigned)((unsigned long long)v >> 32) ^ (neg << 31)) & 0x80000000u;
+    const unsigned ml = __funnelshift_r(l, h, 11);
+    // The mantissa's leading bit (bit 20 of h >> 11) adds the 1 to e.
+    const unsigned long long bits =
+        (((unsigned long long)((h >> 11) + (unsigned)e * 0x100000u + sign) << 32) | ml) +
+        ((l >> 10) & 1u);
+    // No bit set, or below or above FP64's normal range.
+    const bool none = (int)h >= 0 || e < 0, inf = e >= 2046;
+    const unsigned bh = none ? 0u : (inf ? sign | 0x7FF00000u : (unsigned)(bits >> 32));
+    return __hiloint2double((int)bh, none || inf ? 0 : (int)(unsigned)bits);
   }
 };
 
+// Raises colexp[n0 + c], c < EPI_COLS, to the largest exponent field over the
+// warp's rows: w[i] holds columns 2i and 2i+1, each exponent field at bits
+// 4..14 of its half.  Halving the columns with each exchange takes 9 shuffles
+// and one atomic instruction where a reduction a column took 16 of each.
+__device__ __forceinline__ void raise_exponents(uint32_t (&w)[EPI_COLS / 2], int* colexp, int n0,
+                                                int N, int lane) {
+#pragma unroll
+  for (int h = EPI_COLS / 4; h >= 1; h >>= 1) {
+    const int o = 4 * h;
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int i = 0; i < h; ++i) {
+      const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? w[i] : w[i + h], o);
+      w[i] = __vmaxu2(up ? w[i + h] : w[i], got);
+    }
+  }
+  w[0] = __vmaxu2(w[0], __shfl_xor_sync(0xffffffffu, w[0], 2));
+  w[0] = __vmaxu2(w[0], __shfl_xor_sync(0xffffffffu, w[0], 1));
+  const int n = n0 + 2 * (lane >> 2) + (lane & 1);
+  const int m = (int)(((lane & 1) ? w[0] >> 16 : w[0] & 0xFFFFu) >> 4);
+  if ((lane & 2) == 0 && n < N && m != 0) atomicMax(colexp + n, m);
+}
+
 // Output of one row's EPI_COLS columns: out = sign * sum * 2^(ea + eb - 14)
-// (mode 0) or C += that (mode 1).  In update mode the row's C entries are
-// first prefetched into L2 (no registers held), then read in batches of 8
-// with every load of a batch issued before its stores.
+// (mode 0) or C += that (mode 1), C's entries loaded LOAD_BATCH ahead.  FULL: all of the columns are there.
+template <bool FULL, typename Sums>
+__device__ __forceinline__ void write_cols(const OzkArgs& a, int r, int n0, double* crow,
+                                           const Sums& sums, bool live) {
+  static_assert(EPI_COLS == 16, "two columns a word, eight words for 32 lanes");
+  const unsigned neg = a.sign < 0.0 ? 1u : 0u;
+  const int er = live ? a.ea[r] - 14 : 0;
+  double* p = crow + (long long)n0 * a.ccs;
+  constexpr int LOAD_BATCH = 8;
+  double cv[LOAD_BATCH];
+  const uint32_t counted = live && r >= a.row_lo ? 0x7FF07FF0u : 0u;
+  uint32_t ex[EPI_COLS / 2];
+#pragma unroll
+  for (int j = 0; j < EPI_COLS; ++j) {
+    if (j % LOAD_BATCH == 0) {
+#pragma unroll
+      for (int i = 0; i < LOAD_BATCH; ++i)
+        cv[i] = (a.mode == 1 && live && (FULL || n0 + j + i < a.N)) ? p[(long long)(j + i) * a.ccs]
+                                                                    : 0.0;
+    }
+    const int n = n0 + j;
+    double out = 0.0;
+    if (FULL || n < a.N) {
+      const int ek = er + (a.eb_raw ? scale_of_raw(a.eb_raw[n]) : a.eb[n]);
+      const double v = sums.value(j, ek, neg);
+      out = a.mode == 0 ? v : cv[j % LOAD_BATCH] + v;
+      if (live) p[(long long)j * a.ccs] = out;
+    }
+    if (j & 1)
+      ex[j / 2] = __byte_perm(ex[j / 2], (uint32_t)__double2hiint(out), 0x7632) & counted;
+    else
+      ex[j / 2] = (uint32_t)__double2hiint(out);
+  }
+  if (a.colexp != nullptr)  // kernel-uniform; every lane of the warp is here
+    raise_exponents(ex, a.colexp, n0, a.N, threadIdx.x & 31);
+}
+
 template <typename Sums>
 __device__ __forceinline__ void write_row(const OzkArgs& a, int r, int n0, double* crow,
                                           const Sums& sums, bool live) {
-  const unsigned neg = a.sign < 0.0 ? 1u : 0u;
-  const int er = live ? a.ea[r] - 14 : 0;
-  const bool counted = live && r >= a.row_lo;
-  if (a.mode == 1 && live) {
-#pragma unroll
-    for (int j = 0; j < EPI_COLS; ++j)
-      if (n0 + j < a.N)
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(crow + (long long)(n0 + j) * a.ccs));
-  }
-#pragma unroll
-  for (int c8 = 0; c8 < EPI_COLS; c8 += 8) {
-    double cv[8];
-    int ek[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int n = n0 + c8 + j;
-      ek[j] = (live && n < a.N) ? er + (a.eb_raw ? scale_of_raw(a.eb_raw[n]) : a.eb[n]) : 0;
-      cv[j] = (a.mode == 1 && live && n < a.N) ? crow[(long long)n * a.ccs] : 0.0;
-    }
-    unsigned fx[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int n = n0 + c8 + j;
-      fx[j] = 0u;
-      if (live && n < a.N) {
-        const double v = sums.value(c8 + j, ek[j], neg);
-        const double out = a.mode == 0 ? v : cv[j] + v;
-        crow[(long long)n * a.ccs] = out;
-        if (counted) fx[j] = (unsigned)((__double_as_longlong(out) >> 52) & 0x7FF);
-      }
-    }
-    if (a.colexp != nullptr) {  // kernel-uniform; every lane of the warp is here
-      const int lane = threadIdx.x & 31;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const unsigned m = __reduce_max_sync(0xffffffffu, fx[j]);
-        if (lane == j && m != 0u) atomicMax(a.colexp + n0 + c8 + j, (int)m);
-      }
-    }
-  }
+  if (n0 + EPI_COLS <= a.N)
+    write_cols<true>(a, r, n0, crow, sums, live);
+  else
+    write_cols<false>(a, r, n0, crow, sums, live);
 }
 
 // Digit-pair MMAs of one K block into the accumulators at tb: pair (s, t) into
@@ -787,7 +711,7 @@ __device__ __forceinline__ bool issue_pairs(uint32_t tb, uint64_t da0, uint64_t 
     const int hi = lo + ACC_GROUP < nacc ? lo + ACC_GROUP : nacc;
     if (lo >= nacc) continue;
     if (FIRST) {
-      if (!mbar_wait(&h.empty[g], (round & 1) ^ 1, lim, abort_flag)) return false;
+      if (!warp_wait(&h.empty[g], (round & 1) ^ 1, lim, abort_flag)) return false;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     }
 #pragma unroll
@@ -822,16 +746,14 @@ __device__ __forceinline__ bool issue_block(uint32_t tb, uint64_t da0, uint64_t 
                : issue_pairs<0, false>(tb, da0, db0, S, idesc, last, h, round, lim, abort_flag);
 }
 
-__global__ void __launch_bounds__(NT, 1) ozk_gemm_kernel(OzkArgs a,
-                                                        const __grid_constant__ CUtensorMap tmA,
-                                                        const __grid_constant__ CUtensorMap tmB) {
+__global__ void __launch_bounds__(NT, 1) ozk_gemm_kernel(OzkArgs a) {
   HQ_PDL_WAIT();
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[MAX_STAGES], empty_bar[MAX_STAGES];
   __shared__ __align__(8) uint64_t acc_full[MAX_GROUPS], acc_empty[MAX_GROUPS], done_bar;
   __shared__ uint32_t tmem_base;
   __shared__ volatile int s_abort;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
   const int S = a.S;
   const int a_stage = S * A_TILE, b_stage = S * B_TILE;
   const int nacc = n_acc(S);
@@ -882,36 +804,35 @@ __global__ void __launch_bounds__(NT, 1) ozk_gemm_kernel(OzkArgs a,
           break;
         }
         mbar_expect_tx(&full_bar[st], (unsigned)(a_stage + b_stage));
-        const int k0 = (kb0 + i) * TK;
-        tma_load_3d(sA + st * a_stage, &tmA, k0, mt * TM, 0, &full_bar[st]);
-        tma_load_3d(sB + st * b_stage, &tmB, k0, nt * TN, 0, &full_bar[st]);
+        bulk_load(sA + st * a_stage, a.A + ((long long)mt * a.KB + kb0 + i) * a_stage, a_stage,
+                  &full_bar[st]);
+        bulk_load(sB + st * b_stage, a.B + ((long long)nt * a.KB + kb0 + i) * b_stage, b_stage,
+                  &full_bar[st]);
         ++copies_issued;
       }
     }
   } else if (warp == MMA_WARP) {
-    if (lane == 0) {
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TM >> 4) << 24);
-      for (int i = 0; i < nkb; ++i) {
-        const int st = i % STAGES;
-        if (!mbar_wait(&full_bar[st], (i / STAGES) & 1, lim, &s_abort)) {
-          s_abort = 1;
-          break;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        // Every accumulator restarts after a drain, every KB_PER_DRAIN blocks.
-        if (!issue_block(tbase, sw64_desc(smem_u32(sA + st * a_stage)),
-                         sw64_desc(smem_u32(sB + st * b_stage)), S, idesc, i % KB_PER_DRAIN == 0,
-                         (i + 1) % KB_PER_DRAIN == 0 || i + 1 == nkb, hand, i / KB_PER_DRAIN, lim,
-                         &s_abort)) {
-          s_abort = 1;
-          break;
-        }
-        mma_commit(&empty_bar[st]);
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TM >> 4) << 24);
+    for (int i = 0; i < nkb; ++i) {
+      const int st = i % STAGES;
+      if (!warp_wait(&full_bar[st], (i / STAGES) & 1, lim, &s_abort)) {
+        s_abort = 1;
+        break;
       }
-      // Nothing of the tensor core's may arrive in shared memory after exit.
-      mma_commit(&done_bar);
-      if (!mbar_wait(&done_bar, 0, lim, nullptr)) s_abort = 1;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      // Every accumulator restarts after a drain, every KB_PER_DRAIN blocks.
+      if (!issue_block(tbase, sw64_desc(smem_u32(sA + st * a_stage)),
+                       sw64_desc(smem_u32(sB + st * b_stage)), S, idesc, i % KB_PER_DRAIN == 0,
+                       (i + 1) % KB_PER_DRAIN == 0 || i + 1 == nkb, hand, i / KB_PER_DRAIN, lim,
+                       &s_abort)) {
+        s_abort = 1;
+        break;
+      }
+      mma_commit(&empty_bar[st]);
     }
+    // Nothing of the tensor core's may arrive in shared memory after exit.
+    mma_commit(&done_bar);
+    if (!warp_wait(&done_bar, 0, lim, nullptr)) s_abort = 1;
   } else {
     // Epilogue warps 0-19: TMEM lanes 32*(warp&3).. = tile rows, columns
     // (warp>>2)*EPI_COLS.. of the tile.
@@ -963,11 +884,15 @@ __global__ void __launch_bounds__(NT, 1) ozk_gemm_kernel(OzkArgs a,
 // recorded by the epilogue of the update that wrote C), so nothing is read
 // twice: the trailing matrix is read once as FP64 instead of being split to
 // 14 bytes of digits per entry and read back.  The digits are those
-// ozk_split_chunk_kernel writes.  A conversion barrier per stage orders the
-// digit writes (generic proxy, fenced to the async proxy) before the MMAs.
+// ozk_split_chunk_kernel writes.  The writes (generic proxy) are
+// fenced to the async proxy before the MMAs.
 // K <= 256 takes the sums that the short-K kernel takes (the last blocks of a
 // factorization), so both routes give the same bits there too.
 constexpr int C64_TILE = TN * TK * 8;  // 20 KB of FP64 per stage
+// The FP64 tiles have a producer warp of their own: two lanes of one warp that
+// wait for different barriers hold each other up.
+constexpr int C64_PRODUCER_WARP = 22;
+constexpr int NT_C64 = NT + 32;
 
 // One thread's share of a block's conversion: 4 consecutive K entries (h-th
 // quarter of the 32) of tile column c, read as two 16-byte loads, written as
@@ -975,33 +900,18 @@ constexpr int C64_TILE = TN * TK * 8;  // 20 KB of FP64 per stage
 template <int S>
 __device__ __forceinline__ void convert_quarter(const double* __restrict__ sC, uint8_t* sBst, int c,
                                                 int h, int shift_base) {
-  constexpr unsigned long long BIAS = 0x8080808080808080ULL >> (8 * (8 - S));
   const double2* x2 = reinterpret_cast<const double2*>(sC + c * TK + h * 4);
   const double2 p0 = x2[0], p1 = x2[1];
-  const double x[4] = {p0.x, p0.y, p1.x, p1.y};
-  unsigned long long W[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) W[j] = (unsigned long long)fixed_point(x[j], shift_base) + BIAS;
+  const unsigned long long w0 = digit_word<S>(p0.x, shift_base);
+  const unsigned long long w1 = digit_word<S>(p0.y, shift_base);
+  const unsigned long long w2 = digit_word<S>(p1.x, shift_base);
+  const unsigned long long w3 = digit_word<S>(p1.y, shift_base);
   const int phys = (h >> 1) ^ ((c >> 1) & 3);  // 64-byte swizzle of the 16-byte chunk
   uint8_t* dst = sBst + c * (TK * 2) + phys * 16 + (h & 1) * 8;
 #pragma unroll
-  for (int s = 0; s < S; ++s) {
-    const int p = S - 1 - s;
-    uint32_t w[2];
-#pragma unroll
-    for (int j = 0; j < 4; j += 2) {
-      uint32_t u0, u1;
-      if (p == S - 1) {
-        u0 = (uint32_t)(W[j] >> (8 * p));
-        u1 = (uint32_t)(W[j + 1] >> (8 * p));
-      } else {
-        u0 = (uint32_t)(W[j] >> (8 * p)) & 255u;
-        u1 = (uint32_t)(W[j + 1] >> (8 * p)) & 255u;
-      }
-      w[j >> 1] = __byte_perm(digit_scaled(u0, s), digit_scaled(u1, s), 0x7632);
-    }
-    *reinterpret_cast<uint2*>(dst + s * B_TILE) = make_uint2(w[0], w[1]);
-  }
+  for (int s = 0; s < S; ++s)
+    *reinterpret_cast<uint2*>(dst + s * B_TILE) =
+        make_uint2(digit_pair<S>(w0, w1, s), digit_pair<S>(w2, w3, s));
 }
 
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y,
@@ -1014,22 +924,22 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
 }
 
 template <typename Sums>
-__global__ void __launch_bounds__(NT, 1) ozk_gemm_c64_kernel(
-    OzkArgs a, const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmC) {
+__global__ void __launch_bounds__(NT_C64, 1) ozk_gemm_c64_kernel(
+    OzkArgs a, const __grid_constant__ CUtensorMap tmC) {
   HQ_PDL_WAIT();
   constexpr int S = 7;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  // a_full: the M side's digits of a block landed; c_full: its FP64 N-side
-  // tile landed; c_empty: the converters are done with that FP64 tile;
-  // conv_bar: its digits are in the B stage; empty_bar: the MMAs are done
-  // with the A and B stages.  The FP64 tile of block i is fetched as soon as
-  // block i - 2's was converted, so its load never waits for the MMAs.
-  __shared__ __align__(8) uint64_t a_full[MAX_STAGES], c_full[MAX_STAGES], c_empty[MAX_STAGES],
-      empty_bar[MAX_STAGES], conv_bar[MAX_STAGES];
+  // full_bar: the M side's digits of a block landed and those of the N side
+  // are cut; c_full: its FP64 N-side tile landed; c_empty: the converters are
+  // done with that FP64 tile; empty_bar: the MMAs are done with the A and B
+  // stages.  The FP64 tile of block i is fetched as soon as block i - 2's was
+  // converted, so its load never waits for the MMAs.
+  __shared__ __align__(8) uint64_t full_bar[MAX_STAGES], c_full[MAX_STAGES], c_empty[MAX_STAGES],
+      empty_bar[MAX_STAGES];
   __shared__ __align__(8) uint64_t acc_full[MAX_GROUPS], acc_empty[MAX_GROUPS], done_bar;
   __shared__ uint32_t tmem_base;
   __shared__ volatile int s_abort;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
   const int a_stage = S * A_TILE, b_stage = S * B_TILE;
   const int nacc = n_acc(S);
   const uint32_t tmem_cols = tmem_pow2((uint32_t)(nacc * TN));
@@ -1044,11 +954,10 @@ __global__ void __launch_bounds__(NT, 1) ozk_gemm_c64_kernel(
 
   if (tid == 0) {
     for (int i = 0; i < STAGES; ++i) {
-      mbar_init(&a_full[i], 1);
+      mbar_init(&full_bar[i], 1 + NEPI / 32);
       mbar_init(&c_full[i], 1);
       mbar_init(&c_empty[i], NEPI / 32);
       mbar_init(&empty_bar[i], 1);
-      mbar_init(&conv_bar[i], NEPI / 32);
     }
     for (int g = 0; g < MAX_GROUPS; ++g) {
       mbar_init(&acc_full[g], 1);
@@ -1070,7 +979,7 @@ __global__ void __launch_bounds__(NT, 1) ozk_gemm_c64_kernel(
   const uint32_t tbase = tmem_base;
   const unsigned lim = a.spin_limit;
   const Handover hand = {acc_full, acc_empty};
-  int a_issued = 0, c_issued = 0;  // producer lanes 0 and 1
+  int a_issued = 0, c_issued = 0;  // the two producers
 
   if (warp == PRODUCER_WARP) {
     if (lane == 0) {  // the M side's digit tiles, as the MMAs free the stages
@@ -1080,11 +989,14 @@ __global__ void __launch_bounds__(NT, 1) ozk_gemm_c64_kernel(
           s_abort = 1;
           break;
         }
-        mbar_expect_tx(&a_full[st], (unsigned)a_stage);
-        tma_load_3d(sA + st * a_stage, &tmA, (kb0 + i) * TK, mt * TM, 0, &a_full[st]);
+        mbar_expect_tx(&full_bar[st], (unsigned)a_stage);
+        bulk_load(sA + st * a_stage, a.A + ((long long)mt * a.KB + kb0 + i) * a_stage, a_stage,
+                  &full_bar[st]);
         ++a_issued;
       }
-    } else if (lane == 1) {  // the FP64 tiles, as the converters free them
+    }
+  } else if (warp == C64_PRODUCER_WARP) {
+    if (lane == 0) {  // the FP64 tiles, as the converters free them
       for (int i = 0; i < nkb; ++i) {
         const int st = i % STAGES;
         if (!mbar_wait(&c_empty[st], ((i / STAGES) & 1) ^ 1, lim, &s_abort)) {
@@ -1097,29 +1009,26 @@ __global__ void __launch_bounds__(NT, 1) ozk_gemm_c64_kernel(
       }
     }
   } else if (warp == MMA_WARP) {
-    if (lane == 0) {
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TM >> 4) << 24);
-      for (int i = 0; i < nkb; ++i) {
-        const int st = i % STAGES;
-        if (!mbar_wait(&a_full[st], (i / STAGES) & 1, lim, &s_abort) ||
-            !mbar_wait(&conv_bar[st], (i / STAGES) & 1, lim, &s_abort)) {
-          s_abort = 1;
-          break;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (!issue_block(tbase, sw64_desc(smem_u32(sA + st * a_stage)),
-                         sw64_desc(smem_u32(sB + st * b_stage)), S, idesc, i % KB_PER_DRAIN == 0,
-                         (i + 1) % KB_PER_DRAIN == 0 || i + 1 == nkb, hand, i / KB_PER_DRAIN, lim,
-                         &s_abort)) {
-          s_abort = 1;
-          break;
-        }
-        mma_commit(&empty_bar[st]);
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TM >> 4) << 24);
+    for (int i = 0; i < nkb; ++i) {
+      const int st = i % STAGES;
+      if (!warp_wait(&full_bar[st], (i / STAGES) & 1, lim, &s_abort)) {
+        s_abort = 1;
+        break;
       }
-      // Nothing of the tensor core's may arrive in shared memory after exit.
-      mma_commit(&done_bar);
-      if (!mbar_wait(&done_bar, 0, lim, nullptr)) s_abort = 1;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (!issue_block(tbase, sw64_desc(smem_u32(sA + st * a_stage)),
+                       sw64_desc(smem_u32(sB + st * b_stage)), S, idesc, i % KB_PER_DRAIN == 0,
+                       (i + 1) % KB_PER_DRAIN == 0 || i + 1 == nkb, hand, i / KB_PER_DRAIN, lim,
+                       &s_abort)) {
+        s_abort = 1;
+        break;
+      }
+      mma_commit(&empty_bar[st]);
     }
+    // Nothing of the tensor core's may arrive in shared memory after exit.
+    mma_commit(&done_bar);
+    if (!warp_wait(&done_bar, 0, lim, nullptr)) s_abort = 1;
   } else {
     // Epilogue warps 0-19: convert every K block, drain every 256 K, write.
     Sums sums;
@@ -1153,7 +1062,7 @@ __global__ void __launch_bounds__(NT, 1) ozk_gemm_c64_kernel(
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0) {
-        mbar_arrive(&conv_bar[st]);
+        mbar_arrive(&full_bar[st]);
         mbar_arrive(&c_empty[st]);
       }
       // The drain of the K blocks before this one, after this one's digits are
@@ -1177,9 +1086,9 @@ __global__ void __launch_bounds__(NT, 1) ozk_gemm_c64_kernel(
     if (tid == 0) atomicCAS(a.err, 0, HQ_ERR_BARRIER_TIMEOUT);
     if (warp == PRODUCER_WARP && lane == 0) {
       for (int i = a_issued > STAGES ? a_issued - STAGES : 0; i < a_issued; ++i)
-        mbar_wait(&a_full[i % STAGES], (i / STAGES) & 1, lim, nullptr);
+        mbar_wait(&full_bar[i % STAGES], (i / STAGES) & 1, lim, nullptr);
     }
-    if (warp == PRODUCER_WARP && lane == 1) {
+    if (warp == C64_PRODUCER_WARP && lane == 0) {
       for (int i = c_issued > STAGES ? c_issued - STAGES : 0; i < c_issued; ++i)
         mbar_wait(&c_full[i % STAGES], (i / STAGES) & 1, lim, nullptr);
     }
@@ -1194,21 +1103,21 @@ __global__ void __launch_bounds__(NT, 1) ozk_gemm_c64_kernel(
 }
 
 // Persistent variant for short products (K <= 256, so no intermediate drain
-// of the exact levels): one CTA per SM walks the output tiles (TM x TN), and
+// of the exact levels): one CTA per SM walks the output tiles (TM x TN), down
+// the columns (what the CTAs update at one time is then contiguous), and
 // the producer streams operand stages ahead across tile boundaries.  The
 // epilogue warps first drain a tile's accumulators into registers and hand
 // the TMEM back, then do the FP64 output (the part bound by the FP64 pipe and
 // by C's memory traffic) while the MMAs of the next tile run.  Mode 1
 // (C += sign * A B^T) or 0 (C = sign * A B^T), no grid.z split.
-__global__ void __launch_bounds__(NT, 1) ozk_gemm_short_kernel(
-    OzkArgs a, const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB) {
+__global__ void __launch_bounds__(NT, 1) ozk_gemm_short_kernel(OzkArgs a) {
   HQ_PDL_WAIT();
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[MAX_STAGES], empty_bar[MAX_STAGES];
   __shared__ __align__(8) uint64_t acc_full[MAX_GROUPS], acc_empty[MAX_GROUPS], done_bar;
   __shared__ uint32_t tmem_base;
   __shared__ volatile int s_abort;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
   const int S = a.S;
   const int a_stage = S * A_TILE, b_stage = S * B_TILE;
   const int nacc = n_acc(S);
@@ -1251,7 +1160,7 @@ __global__ void __launch_bounds__(NT, 1) ozk_gemm_short_kernel(
     if (lane == 0) {
       int i = 0;  // stage counter across tiles
       for (int t = blockIdx.x; t < ntiles && !s_abort; t += gridDim.x) {
-        const int mt = t / NTL, nt = t % NTL;
+        const int mt = t % MT, nt = t / MT;
         for (int kb = 0; kb < nkb; ++kb, ++i) {
           const int st = i % STAGES;
           if (!mbar_wait(&empty_bar[st], ((i / STAGES) & 1) ^ 1, lim, &s_abort)) {
@@ -1259,37 +1168,37 @@ __global__ void __launch_bounds__(NT, 1) ozk_gemm_short_kernel(
             break;
           }
           mbar_expect_tx(&full_bar[st], (unsigned)(a_stage + b_stage));
-          tma_load_3d(sA + st * a_stage, &tmA, kb * TK, mt * TM, 0, &full_bar[st]);
-          tma_load_3d(sB + st * b_stage, &tmB, kb * TK, nt * TN, 0, &full_bar[st]);
+          bulk_load(sA + st * a_stage, a.A + ((long long)mt * nkb + kb) * a_stage, a_stage,
+                    &full_bar[st]);
+          bulk_load(sB + st * b_stage, a.B + ((long long)nt * nkb + kb) * b_stage, b_stage,
+                    &full_bar[st]);
           ++copies_issued;
         }
       }
     }
   } else if (warp == MMA_WARP) {
-    if (lane == 0) {
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TM >> 4) << 24);
-      int i = 0, lt = 0;
-      for (int t = blockIdx.x; t < ntiles && !s_abort; t += gridDim.x, ++lt) {
-        bool ok = true;
-        for (int kb = 0; kb < nkb && ok; ++kb, ++i) {
-          const int st = i % STAGES;
-          ok = mbar_wait(&full_bar[st], (i / STAGES) & 1, lim, &s_abort);
-          if (!ok) break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          ok = issue_block(tbase, sw64_desc(smem_u32(sA + st * a_stage)),
-                           sw64_desc(smem_u32(sB + st * b_stage)), S, idesc, kb == 0,
-                           kb + 1 == nkb, hand, lt, lim, &s_abort);
-          if (ok) mma_commit(&empty_bar[st]);
-        }
-        if (!ok) {
-          s_abort = 1;
-          break;
-        }
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TM >> 4) << 24);
+    int i = 0, lt = 0;
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++lt) {
+      bool ok = true;
+      for (int kb = 0; kb < nkb && ok; ++kb, ++i) {
+        const int st = i % STAGES;
+        ok = warp_wait(&full_bar[st], (i / STAGES) & 1, lim, &s_abort);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        ok = issue_block(tbase, sw64_desc(smem_u32(sA + st * a_stage)),
+                         sw64_desc(smem_u32(sB + st * b_stage)), S, idesc, kb == 0,
+                         kb + 1 == nkb, hand, lt, lim, &s_abort);
+        if (ok) mma_commit(&empty_bar[st]);
       }
-      // Nothing of the tensor core's may arrive in shared memory after exit.
-      mma_commit(&done_bar);
-      if (!mbar_wait(&done_bar, 0, lim, nullptr)) s_abort = 1;
+      if (!ok) {
+        s_abort = 1;
+        break;
+      }
     }
+    // Nothing of the tensor core's may arrive in shared memory after exit.
+    mma_commit(&done_bar);
+    if (!warp_wait(&done_bar, 0, lim, nullptr)) s_abort = 1;
   } else {
     const int col0 = (warp >> 2) * EPI_COLS;
     const uint32_t tacc = tbase + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)col0;
@@ -1304,7 +1213,7 @@ __global__ void __launch_bounds__(NT, 1) ozk_gemm_short_kernel(
         s_abort = 1;
         break;
       }
-      const int mt = t / NTL, nt = t % NTL;
+      const int mt = t % MT, nt = t / MT;
       const int r = mt * TM + (warp & 3) * 32 + lane;
       // Every lane takes part (the column-exponent reduction is warp-wide);
       // rows past M only skip their loads and stores.
@@ -1359,8 +1268,13 @@ extern "C" int hq_ozk_rowmax_raw(cudaStream_t stream, const double* X, long long
   if (R <= 0 || K <= 0) return 0;
   const int e = hq_zero_words(stream, raw, (size_t)rows_total, nullptr, 0);
   if (e) return e;
-  hq_launch(ozk_rowmax_atomic_kernel, dim3(R, (K + ROWMAX_SPAN - 1) / ROWMAX_SPAN), 256, 0, stream,
-      X, rs, ks, K, raw);
+  if (rs == 1 && ks != 1)
+    hq_launch(ozk_rowmax_cm_kernel,
+              dim3((R + 31) / 32, (K + ROWMAX_CM_SPAN - 1) / ROWMAX_CM_SPAN), 256, 0, stream, X, ks,
+              R, K, raw);
+  else
+    hq_launch(ozk_rowmax_atomic_kernel, dim3(R, (K + ROWMAX_SPAN - 1) / ROWMAX_SPAN), 256, 0,
+              stream, X, rs, ks, K, raw);
   hq_count_launches(1);
   return (int)cudaGetLastError();
 }
@@ -1380,49 +1294,25 @@ extern "C" int hq_ozk_split(cudaStream_t stream, const double* X, long long rs, 
   int blocks = (rows_total + 7) / 8;
   if (blocks > 4096) blocks = 4096;
   uint8_t* t = static_cast<uint8_t*>(tiles);
-  constexpr int ROW_CPT = 4;
-  // Long rows (K > 16384), or fewer than FEW_ROWS rows of 512 or more (the
-  // one-pass kernel's 8-row CTAs would then number fewer than a GB300's 152
-  // SMs, each warp walking a long row), take the two-pass split, which
-  // spreads every row over CTAs.
-  constexpr int FEW_ROWS = 8 * 152;
-  if (S == 7 && (K > 512 * 8 * ROW_CPT || (K >= 512 && rows_total < FEW_ROWS))) {
-    const long long chunks = (long long)rows_total * KB * (TK / 8);
-    long long cblocks = (chunks + 255) / 256;
-    if (cblocks > 65536) cblocks = 65536;
-    if (raw != nullptr) {  // row maxima with several CTAs per row (scratch given)
-      const int e = hq_ozk_rowmax_raw(stream, X, rs, ks, R, K, rows_total, raw);
-      if (e) return e;
-      hq_launch(ozk_split_chunk_kernel<7>, (unsigned)cblocks, 256, 0, stream, X, rs, ks, R, K, KB,
-                                                                        rows_total, t, exps, raw);
-      hq_count_launches(1);
-      return (int)cudaGetLastError();
-    }
-    int mblocks = rows_total < 8192 ? rows_total : 8192;
-    hq_launch(ozk_rowmax_kernel, mblocks, 256, 0, stream, X, rs, ks, R, K, rows_total, exps);
-    hq_launch(ozk_split_chunk_kernel<7>, (unsigned)cblocks, 256, 0, stream, X, rs, ks, R, K, KB,
-                                                                      rows_total, t, exps, nullptr);
-    hq_count_launches(2);
-    return (int)cudaGetLastError();
+  // Rows of 512 or more take two passes, spread over CTAs (4000 x 4000: the
+  // exponents in 34 us, then the digits in 54; one CTA a row that held the row in
+  // registers took 133, its one pass bound by latency).
+  if (S == 7 && K >= 512) {
+    if (raw == nullptr) return (int)cudaErrorInvalidValue;
+    const int e = hq_ozk_rowmax_raw(stream, X, rs, ks, R, K, rows_total, raw);
+    return e ? e : hq_ozk_split_raw(stream, X, rs, ks, R, K, S, side, tiles, exps, raw);
   }
   if (rs == 1 && ks != 1 && K <= CM_KMAX) {  // column-major rows of a short operand
     const int cb = (rows_total + 31) / 32;
     switch (S) {
 #define HQ_SPLIT_CM_CASE(SS)                                                            \
   case SS:                                                                              \
-    hq_launch(ozk_split_cm_kernel<SS>, cb, 256, 0, stream, X, ks, R, K, KB, rows_total, t, exps); \
+    hq_launch(ozk_split_cm_kernel<SS>, cb, 256, 0, stream, X, ks, R, K, TR, KB, rows_total, t, exps); \
     break;
       HQ_SPLIT_CM_CASE(1) HQ_SPLIT_CM_CASE(2) HQ_SPLIT_CM_CASE(3) HQ_SPLIT_CM_CASE(4)
       HQ_SPLIT_CM_CASE(5) HQ_SPLIT_CM_CASE(6) HQ_SPLIT_CM_CASE(7)
 #undef HQ_SPLIT_CM_CASE
     }
-    hq_count_launches(1);
-    return (int)cudaGetLastError();
-  }
-  if (K >= 4096 && K <= 512 * 8 * ROW_CPT && S == 7) {
-    int rblocks = rows_total < 16384 ? rows_total : 16384;
-    hq_launch(ozk_split_row_kernel<7, ROW_CPT>, rblocks, 512, 0, stream, X, rs, ks, R, K, TR, KB,
-                                                                 rows_total, t, exps);
     hq_count_launches(1);
     return (int)cudaGetLastError();
   }
@@ -1456,36 +1346,9 @@ extern "C" int hq_ozk_split_raw(cudaStream_t stream, const double* X, long long 
   long long cblocks = (chunks + 255) / 256;
   if (cblocks > 65536) cblocks = 65536;
   hq_launch(ozk_split_chunk_kernel<7>, (unsigned)cblocks, 256, 0, stream,
-      X, rs, ks, R, K, KB, rows_total, static_cast<uint8_t*>(tiles), exps, raw);
+      X, rs, ks, R, K, TR, KB, rows_total, static_cast<uint8_t*>(tiles), exps, raw);
   hq_count_launches(1);
   return (int)cudaGetLastError();
-}
-
-// Tensor map of a split operand: D[s][row][k], BF16, dims (k, row, digit) =
-// (kp, rows_p, S); box 32 x tile_rows x S, 64-byte swizzle.
-static int make_digit_map(CUtensorMap* map, const void* tiles, int rows, int K, int S,
-                          int tile_rows) {
-  static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
-  if (encode == nullptr) {
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    cudaError_t e = cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000,
-                                                     cudaEnableDefault, &q);
-    if (e != cudaSuccess || q != cudaDriverEntryPointSuccess || fn == nullptr)
-      return (int)cudaErrorNotSupported;
-    encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
-  }
-  const cuuint64_t rp = (cuuint64_t)((rows + tile_rows - 1) / tile_rows) * tile_rows;
-  const cuuint64_t kp = (cuuint64_t)((K + TK - 1) / TK) * TK;
-  const cuuint64_t dims[3] = {kp, rp, (cuuint64_t)S};
-  const cuuint64_t strides[2] = {kp * 2, rp * kp * 2};  // bytes, dims 1 and 2
-  const cuuint32_t box[3] = {(cuuint32_t)TK, (cuuint32_t)tile_rows, (cuuint32_t)S};
-  const cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(tiles), dims,
-                      strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                      CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
 }
 
 // Split K of the long products (one CTA per SM): the time is about (waves)
@@ -1565,14 +1428,10 @@ extern "C" int hq_ozk_gemm(cudaStream_t stream, const hq_device_info* dev, int M
   }
   if (smem > dev->smem_optin) return (int)cudaErrorInvalidValue;
   a.stages = stages;
-  CUtensorMap tmA, tmB;
-  int rc = make_digit_map(&tmA, Atiles, M, K, S, TM);
-  if (rc == 0) rc = make_digit_map(&tmB, Btiles, N, K, S, TN);
-  if (rc) return rc;
   cudaError_t e =
       cudaFuncSetAttribute(ozk_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  hq_launch(ozk_gemm_kernel, dim3(MT, NTL, Z), NT, smem, stream, a, tmA, tmB);
+  hq_launch(ozk_gemm_kernel, dim3(MT, NTL, Z), NT, smem, stream, a);
   hq_count_launches(1);
   if (Z > 1) {
     long long total = (long long)M * N;
@@ -1636,9 +1495,7 @@ extern "C" int hq_ozk_gemm_c64(cudaStream_t stream, const hq_device_info* dev, i
     a.ccs = ccs;
     a.zstride = 0;
   }
-  CUtensorMap tmA, tmC;
-  int rc = make_digit_map(&tmA, Atiles, M, K, S, TM);
-  if (rc) return rc;
+  CUtensorMap tmC;
   {
     static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
     if (encode == nullptr) {
@@ -1665,7 +1522,7 @@ extern "C" int hq_ozk_gemm_c64(cudaStream_t stream, const hq_device_info* dev, i
   cudaError_t e =
       cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  hq_launch(kernel, dim3(MT, NTL, Z), NT, smem, stream, a, tmA, tmC);
+  hq_launch(kernel, dim3(MT, NTL, Z), NT_C64, smem, stream, a, tmC);
   hq_count_launches(1);
   if (Z > 1) {
     long long total = (long long)M * N;
@@ -1716,16 +1573,12 @@ extern "C" int hq_ozk_gemm_short(cudaStream_t stream, const hq_device_info* dev,
   const size_t smem = (size_t)stages * per_stage + 1024;
   if (smem > dev->smem_optin) return (int)cudaErrorInvalidValue;
   a.stages = stages;
-  CUtensorMap tmA, tmB;
-  int rc = make_digit_map(&tmA, Atiles, M, K, S, TM);
-  if (rc == 0) rc = make_digit_map(&tmB, Btiles, N, K, S, TNV);
-  if (rc) return rc;
   cudaError_t e = cudaFuncSetAttribute(ozk_gemm_short_kernel,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
   const long long tiles = (long long)((M + TM - 1) / TM) * ((N + TNV - 1) / TNV);
   const int grid = (int)(tiles < dev->num_sms ? tiles : dev->num_sms);
-  hq_launch(ozk_gemm_short_kernel, grid, NT, smem, stream, a, tmA, tmB);
+  hq_launch(ozk_gemm_short_kernel, grid, NT, smem, stream, a);
   hq_count_launches(1);
   return (int)cudaGetLastError();
 }
