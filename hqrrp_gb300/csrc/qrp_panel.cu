@@ -625,86 +625,59 @@ int panel_grid(const hq_device_info* dev, int mp, int nc) {
   return g < 1 ? 1 : g;
 }
 
-// DLARFT (Forward, Columnwise) from the Gram matrix Z = U^T U: for each i,
-// T[0:i, i] = -tau_i T[0:i, 0:i] Z[0:i, i] and T[i, i] = tau_i (T[0:i, i] = 0
-// when tau_i = 0).  One CTA; the columns are a sequential recurrence, so each
-// step's triangular matrix-vector product is spread over the CTA with eight
-// lanes per row (short FP64 dependency chains), combined by shuffles.  T is
-// built in shared memory with an odd leading dimension (no bank conflicts
-// between the eight lanes of a row) when it fits.
-__global__ void larft_kernel(int k, const double* __restrict__ Z, int ldz,
-                             const double* __restrict__ tau, double* __restrict__ T, int ldt,
-                             int use_smem) {
-  extern __shared__ double sT[];
-  __shared__ double tmp[HQ_MAX_MY];
-  double* Tm = use_smem ? sT : T;
-  const int ld = use_smem ? (k | 1) : ldt;
-  const int tid = threadIdx.x, nt = blockDim.x;
-  const int g = tid & 7, rows_per_pass = nt >> 3;
-  for (int e = tid; e < k * k; e += nt) Tm[(e % k) + (size_t)(e / k) * ld] = 0.0;
-  __syncthreads();
-  for (int i = 0; i < k; ++i) {
-    const double ti = tau[i];
-    for (int r = tid; r < i; r += nt) tmp[r] = -ti * Z[r + (size_t)i * ldz];
-    __syncthreads();
-    if (ti != 0.0) {
-      for (int r0 = 0; r0 < i; r0 += rows_per_pass) {
-        const int r = r0 + (tid >> 3);
-        double acc = 0.0;
-        if (r < i)
-          for (int c = r + g; c < i; c += 8) acc = fma(Tm[r + (size_t)c * ld], tmp[c], acc);
-        acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-        acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-        acc += __shfl_xor_sync(0xffffffffu, acc, 4);
-        if (g == 0 && r < i) Tm[r + (size_t)i * ld] = acc;
-      }
-    }
-    if (tid == 0) Tm[i + (size_t)i * ld] = ti;
-    __syncthreads();
-  }
-  if (use_smem)
-    for (int e = tid; e < k * k; e += nt)
-      T[(e % k) + (size_t)(e / k) * ldt] = sT[(e % k) + (size_t)(e / k) * ld];
-}
-
-// The same T, one CTA per row.  Row r of T only involves row r itself:
+// DLARFT (Forward, Columnwise) from the Gram matrix Z = U^T U, one CTA per row:
+// row r of T only involves row r itself,
 // T[r, i] = -tau_i * sum_{c = r}^{i-1} T[r, c] Z[c, i] for i > r, T[r, r] =
 // tau_r (zero when tau_i = 0), so the k rows are independent recurrences and
-// run side by side on k SMs instead of one SM's FP64 pipe doing all of them.
-// The CTA first stages the part of Z its row reads (Z[r:i, i], i > r: the
-// upper triangle from row r) in shared memory with all its threads, then one
-// warp runs the recurrence: per step a dot of length i - r over the lanes and
-// a shuffle reduction, with the row kept in shared memory.
-constexpr int LARFT_ROW_MAX = 128;  // k up to this: row and staged triangle fit (<= 66 KB)
-
-__global__ void __launch_bounds__(128) larft_rows_kernel(int k, const double* __restrict__ Z,
-                                                         int ldz, const double* __restrict__ tau,
-                                                         double* __restrict__ T, int ldt) {
-  extern __shared__ double lsm[];
-  double* sT = lsm;      // [k] the row, from column r on
-  double* sZ = lsm + k;  // [k (k - 1) / 2] the staged triangle
-  const int r = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
-  // Column i > r of the staged triangle holds Z[r:i, i] at offset
-  // off(i) = (i - r - 1)(i - r) / 2.
-  for (int i = r + 1; i < k; ++i) {
-    const int off = (i - r - 1) * (i - r) / 2;
-    for (int c = r + tid; c < i; c += blockDim.x) sZ[off + (c - r)] = Z[c + (size_t)i * ldz];
-  }
-  __syncthreads();
-  if (tid < 32) {
-    if (lane == 0) sT[0] = tau[r];
-    __syncwarp();
-    for (int i = r + 1; i < k; ++i) {
-      const double ti = tau[i];
-      const int off = (i - r - 1) * (i - r) / 2;
-      double acc = 0.0;
-      for (int c = lane; c < i - r; c += 32) acc = fma(sT[c], sZ[off + c], acc);
-      acc = hq_warp_sum(acc);
-      if (lane == 0) sT[i - r] = ti != 0.0 ? -ti * acc : 0.0;
-      __syncwarp();
+// run side by side on the SMs instead of one SM's FP64 pipe doing all of them.
+// A thread holds one entry of the row and a warp 32: the warps before it hand
+// theirs over in shared memory, and within the warp each entry, once known,
+// is broadcast and added to the ones after it with the factors -tau_i Z[c, i]
+// ready in registers -- a shuffle and a fused multiply-add a step.  (A dot
+// product and a warp sum a step took 60 us for k = 64; this takes 9.)
+__global__ void __launch_bounds__(HQ_MAX_MY) larft_rows_kernel(
+    int k, const double* __restrict__ Z, int ldz, const double* __restrict__ tau,
+    double* __restrict__ T, int ldt) {
+  __shared__ double sx[HQ_MAX_MY];
+  const int r = blockIdx.x, c = threadIdx.x, lane = c & 31, warp = c >> 5;
+  const int n = k - r;  // T[r, r + c], c < n
+  const bool live = c < n;
+  const double t = live ? tau[r + c] : 0.0;
+  const double* zc = Z + r + (size_t)(r + (live ? c : 0)) * ldz;
+  double z[32];
+#pragma unroll
+  for (int d = 0; d < 32; ++d) z[d] = live && d < lane ? -t * zc[warp * 32 + d] : 0.0;
+  double acc = 0.0, x = 0.0;
+  const int nw = (n + 31) >> 5;
+  for (int b = 0; b < nw; ++b) {
+    double zb[32];
+    if (warp > b && live) {
+#pragma unroll
+      for (int d = 0; d < 32; ++d) zb[d] = zc[32 * b + d];
     }
-    for (int i = lane; i < k; i += 32) T[r + (size_t)i * ldt] = i < r ? 0.0 : sT[i - r];
+    if (warp == b) {
+      const bool on = t != 0.0;
+      x = c == 0 ? t : (on ? -t * acc : 0.0);
+#pragma unroll
+      for (int d = 0; d < 31; ++d) {
+        const double xd = __shfl_sync(0xffffffffu, x, d);
+        if (on && lane > d) x = fma(xd, z[d], x);
+      }
+      sx[c] = x;
+    }
+    __syncthreads();
+    if (warp > b && live) {
+      double acc2 = 0.0;
+#pragma unroll
+      for (int d = 0; d < 32; d += 2) {
+        acc = fma(sx[32 * b + d], zb[d], acc);
+        acc2 = fma(sx[32 * b + d + 1], zb[d + 1], acc2);
+      }
+      acc += acc2;
+    }
   }
+  if (live) T[r + (size_t)(r + c) * ldt] = x;
+  for (int i = c; i < r; i += blockDim.x) T[r + (size_t)i * ldt] = 0.0;
 }
 
 }  // namespace
@@ -787,24 +760,7 @@ extern "C" int hq_larft_from_gram(cudaStream_t stream, int k, const double* Z, i
                                   const double* tau, double* T, int ldt) {
   if (k <= 0) return 0;
   if (k > HQ_MAX_MY) return (int)cudaErrorInvalidValue;
-  if (k <= LARFT_ROW_MAX) {
-    const size_t rsm = sizeof(double) * ((size_t)k + (size_t)k * (k - 1) / 2);
-    cudaError_t e = cudaFuncSetAttribute(larft_rows_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rsm);
-    if (e != cudaSuccess) return (int)e;
-    larft_rows_kernel<<<k, 128, rsm, stream>>>(k, Z, ldz, tau, T, ldt);
-    hq_count_launches(1);
-    return (int)cudaGetLastError();
-  }
-  const size_t smem = sizeof(double) * (size_t)k * (k | 1);
-  if (smem <= 160 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(larft_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    larft_kernel<<<1, 256, smem, stream>>>(k, Z, ldz, tau, T, ldt, 1);
-  } else {
-    larft_kernel<<<1, 256, 0, stream>>>(k, Z, ldz, tau, T, ldt, 0);
-  }
+  larft_rows_kernel<<<k, (k + 31) / 32 * 32, 0, stream>>>(k, Z, ldz, tau, T, ldt);
   hq_count_launches(1);
   return (int)cudaGetLastError();
 }
