@@ -1756,9 +1756,11 @@ HQ_API int hqrrp_gb300_hqrrp_truncated_device(int m, int n, int k, double* dA, i
 /* C (m x nc, ldc) := Q C (trans 'N') or Q^T C (trans 'T'), Q = H_0 ... H_{k-1}
  * the product of the first k reflectors stored in F.  The reflector blocks
  * of nb columns are rebuilt (U, Gram, T) from F and applied one at a time:
- * from the last block to the first for Q C, first to last for Q^T C. */
+ * from the last block to the first for Q C, first to last for Q^T C.  unit:
+ * C is [I_k; 0] and trans 'N', so block j leaves the columns before j alone (they
+ * are zero in its rows), which halves the work. */
 static int apply_qk(hq_ws* w, char trans, int m, int nc, int k, int nb, const double* F, int ldf,
-                    const double* tau, double* C, int ldc) {
+                    const double* tau, double* C, int ldc, int unit) {
   const hq_device_info* dev = &w->ds->dev;
   const int nblk = (k + nb - 1) / nb;
   const int tr = trans == 'T' || trans == 't';
@@ -1769,9 +1771,11 @@ static int apply_qk(hq_ws* w, char trans, int m, int nc, int k, int nb, const do
     DGRAM(b, mp);
     CK(hq_larft_from_gram(w->st, b, w->Z, w->ldz, tau + j, w->T, w->ldt));
     /* C[j:, :] -= U op(T) U^T C[j:, :] */
-    DG('T', 'N', b, nc, mp, 1.0, w->U, w->ldu, C + j, ldc, 0.0, w->W1, w->ldw);
-    DG(tr ? 'T' : 'N', 'N', b, nc, b, 1.0, w->T, w->ldt, w->W1, w->ldw, 0.0, w->W2, w->ldw);
-    DG('N', 'N', mp, nc, b, -1.0, w->U, w->ldu, w->W2, w->ldw, 1.0, C + j, ldc);
+    const int c0 = unit ? j : 0;
+    double* Cj = C + j + (size_t)c0 * ldc;
+    DG('T', 'N', b, nc - c0, mp, 1.0, w->U, w->ldu, Cj, ldc, 0.0, w->W1, w->ldw);
+    DG(tr ? 'T' : 'N', 'N', b, nc - c0, b, 1.0, w->T, w->ldt, w->W1, w->ldw, 0.0, w->W2, w->ldw);
+    DG('N', 'N', mp, nc - c0, b, -1.0, w->U, w->ldu, w->W2, w->ldw, 1.0, Cj, ldc);
   }
   return HQ_OK;
 }
@@ -1780,7 +1784,7 @@ static int apply_qk(hq_ws* w, char trans, int m, int nc, int k, int nb, const do
 static int form_qk(hq_ws* w, int m, int k, int nb, const double* F, int ldf, const double* tau,
                    double* Q, int ldq) {
   CK(hq_eye(w->st, m, k, Q, ldq));
-  return apply_qk(w, 'N', m, k, k, nb, F, ldf, tau, Q, ldq);
+  return apply_qk(w, 'N', m, k, k, nb, F, ldf, tau, Q, ldq, 1);
 }
 
 HQ_API int hqrrp_gb300_apply_q_device(char trans, int m, int nc, int k, const double* dF,
@@ -1797,7 +1801,7 @@ HQ_API int hqrrp_gb300_apply_q_device(char trans, int m, int nc, int k, const do
   int rc = ws_begin(&w, (cudaStream_t)stream, 1);
   if (rc) return rc;
   rc = ws_setup(&w, m, imax(nc, k), 0, 0, nb);
-  if (!rc) rc = apply_qk(&w, trans, m, nc, k, nb, dF, lddf, d_tau, dC, lddc);
+  if (!rc) rc = apply_qk(&w, trans, m, nc, k, nb, dF, lddf, d_tau, dC, lddc, 0);
   if (!rc) rc = ws_check(&w);
   ws_release(&w);
   if (!rc) {
@@ -1855,7 +1859,7 @@ HQ_API int hqrrp_gb300_hqrrp_adjoint_device(int m, int n, int k, const double* d
     if (!rc && hq_copyltu(w.st, k, Mp, k, -1.0)) rc = HQ_E_CUDA;
     if (!rc) DGW('N', 'N', m, k, k, 1.0, Q, ldq, Mp, k, 1.0, GQ, ldq);
     /* Abar_1 = X R11^-T */
-    if (!rc && hq_trsm_rt(w.st, m, k, dF, lddf, GQ, ldq)) rc = HQ_E_CUDA;
+    if (!rc && hq_trsm_rt(w.st, dev, m, k, dF, lddf, GQ, ldq, w.ws, w.ws_elems)) rc = HQ_E_CUDA;
     /* dG = Q N, then dG[:, P_1] += Abar_1 */
     if (!rc) DGW('N', 'N', m, n, k, 1.0, Q, ldq, Nk, k, 0.0, dG, lddg);
     if (!rc && hq_scatter_cols(w.st, m, k, GQ, ldq, d_jpvt, dG, lddg, 1)) rc = HQ_E_CUDA;
