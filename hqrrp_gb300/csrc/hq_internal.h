@@ -84,11 +84,11 @@ size_t hq_panel_part_elems(const hq_device_info* dev, int nc);
 /* ---- Gram panel (mixed path): the b x b kernels of qrp_gram.cu -----------
  * All matrices column-major, b <= HQ_GRAM_MAX.  Status bits go to *stat. */
 #define HQ_GRAM_MAX 128
-/* Pass 1: pivoted Cholesky of G (lower triangle read) scaled to unit
- * diagonal, in FP32: perm[k] = source column of position k, R (FP64, upper)
- * with R^T R ~ P^T G P; *stat := 0, or bit with R = I, perm = identity;
- * *alt, *emax := 0. */
-int hq_gram_pchol32(cudaStream_t stream, int n, const double* G, int ldg, double* R, int ldr,
+/* Pass 1: pivoted Cholesky of G scaled to unit diagonal, in FP32: perm[k] =
+ * source column of position k, R (FP64, upper) with R^T R ~ P^T G P; *stat :=
+ * 0, or bit with R = I, perm = identity; *alt, *emax := 0.  G is overwritten;
+ * ldg = ldr = HQ_GRAM_MAX. */
+int hq_gram_pchol32(cudaStream_t stream, int n, double* G, int ldg, double* R, int ldr,
                     int* perm, int* stat, int bit, int* alt, unsigned long long* emax);
 /* FP64 on a cluster of eight CTAs.  mode 0: Cholesky of the symmetric A
  * (lower triangle read), F := R upper.  mode 1: LU without pivoting of A - D

@@ -28,8 +28,8 @@
 // SM, so one SM is slow for them: the FP64 Cholesky and LU run on a cluster
 // of eight CTAs (each owns every eighth column; the pivot column travels
 // through distributed shared memory), the triangular inverses and products
-// with one CTA per column, and only the pivoted first pass on one SM, in
-// FP32.
+// and the first pass's scaling with one CTA per column, and only the pivoted
+// first pass itself on one SM, in FP32.
 //
 // A step that meets a panel it cannot factor accurately sets a bit in a
 // status word: a first-pass pivot below 1e-5 of the column's own squared
@@ -54,9 +54,9 @@ namespace {
 
 constexpr int GN = HQ_GRAM_MAX;  // widest panel
 constexpr int LDS = GN + 1;      // shared-memory column stride of the b x b kernels
-constexpr int CT = 512;          // threads of the one-SM kernels
+constexpr int CT = 256;          // threads of the one-SM kernel
 constexpr int CW = CT / 32;
-constexpr int TW = 4;            // warps per CTA of the triangular kernel (one column per CTA)
+constexpr int TW = 4;            // warps per CTA of the second pass's kernel (one column per CTA)
 constexpr float PIVOT32_REL_MIN = 1e-5f;  // first pass: scaled pivot floor
 constexpr double CHOL2_REL_MIN = 1e-10;   // cluster Cholesky: pivot floor, relative to the diagonal
 constexpr double NEARID_MAX = 2e-4;       // second pass: largest max|G2 - I| it converges from
@@ -67,175 +67,193 @@ constexpr int CLW = CLT / 32;
 constexpr int OWN = GN / CL;              // columns per CTA (column j lives in CTA j % CL)
 static_assert(OWN == 2 * CLW, "each warp of a cluster CTA updates two own columns");
 
-// Pass 1: pivoted Cholesky of the n x n Gram matrix G (ldg) scaled to unit
-// diagonal, in FP32 on one SM, the matrix held in registers.  Thread (warp
-// w, lane t) holds the 32 entries (i, j) with i = t + 32 a (a < 4) and
-// j = w + 16 c (c < 8) of the full symmetric matrix.  Columns are not moved:
-// step k picks the active column p with the largest residual norm (scaled
-// Schur diagonal times the column's original squared norm relative to the
-// largest; the lowest index among residuals equal to 2^-15), the warp holding column p publishes
-// l = S[:, p] / sqrt(S[p][p]) over the active rows (0 elsewhere), and every
-// thread updates its entries by S_ij -= l_i l_j -- a no-op on eliminated
-// rows and columns, so the update needs no masks.  Every warp finds the
-// pivot itself (one warp maximum), so a step takes two barriers.
-// Writes perm[k] (source column of position k) and R = Rs diag(sqrt(G_pp))
-// in FP64 (upper, zeros below), Rs the scaled factor; *stat = 0, or `bit`
-// with R = I and perm = identity when a scaled pivot is not above
-// PIVOT32_REL_MIN; *alt (the second pass's choice of method) and *emax
-// (its max|E|) := 0.
-__global__ void __launch_bounds__(CT, 1)
-    gram_pchol32_kernel(int n, const double* __restrict__ G, int ldg, double* __restrict__ R,
-                        int ldr, int* __restrict__ perm, int* __restrict__ stat, int bit,
-                        int* __restrict__ alt, unsigned long long* __restrict__ emax) {
-  HQ_PDL_WAIT();
-  extern __shared__ float s_Rp[];  // GN * GN: s_Rp[k * GN + i] = row k of Rs at source column i
-  __shared__ double s_sc[GN], s_rt[GN];
-  __shared__ float s_key[GN], s_d[GN], s_l[GN], s_r[GN], s_wmax[CW];
-  __shared__ int s_ord[GN];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  static_assert(CT == 512 && GN == 128, "register layout: 16 warps x 32 lanes, 4 x 8 entries");
-  for (int j = tid; j < GN; j += CT) {
-    double d = 0.0;
-    if (j < n) d = G[j + (size_t)j * ldg];
-    const int ok = j < n && d > 0.0 && d <= 1.7e308;
-    const double rt = ok ? sqrt(d) : 0.0;
-    s_rt[j] = rt;
-    s_sc[j] = ok ? 1.0 / rt : 0.0;
-    s_key[j] = ok ? (float)log2(d) : -4096.0f;  // squared norm, scaled below
-  }
-  __syncthreads();
-  if (warp == 0) {
-    float m = -4096.0f;
-    for (int j = lane; j < n; j += 32) m = fmaxf(m, s_key[j]);
-#pragma unroll
-    for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if (lane == 0) s_wmax[0] = m;
-  }
-  __syncthreads();
-  const float kmax = s_wmax[0];
-  for (int j = tid; j < n; j += CT) s_key[j] = exp2f(s_key[j] - kmax);  // d_j / max d
-  float S[4][8];
-#pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    const int j = warp + 16 * c;
-    double v[4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      const int i = lane + 32 * a;
-      v[a] = (i < n && j < n) ? G[i + (size_t)j * ldg] : 0.0;
-    }
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      const int i = lane + 32 * a;
-      S[a][c] = (i < n && j < n) ? (float)(v[a] * s_sc[i] * s_sc[j]) : 0.0f;
-      if (i == j) s_d[j] = S[a][c];
-    }
-  }
-  __syncthreads();
+// Pass 1: pivoted Cholesky of the n x n Gram matrix G scaled to unit diagonal,
+// in FP32 on one SM, the matrix held in registers.  The FP64 arithmetic around
+// it -- S_ij = G_ij / sqrt(G_ii G_jj) before, R = Rs diag(sqrt(G_pp)) after --
+// runs on one CTA per column (gram_scale_kernel, gram_unscale_kernel): on the
+// one SM it took 28 of 97 us.
+//
+// What the three kernels hand on, in the memory of R (in) and of G (out):
+struct PcholIn {
+  float S[GN * GN];  // scaled Gram matrix, column-major
+  double rt[GN];     // sqrt(G_jj)
+  float key[GN];     // G_jj relative to the largest
+};
+struct PcholOut {
+  float Rs[GN * GN];  // Rs[k * GN + i]: row k of the scaled factor at source column i
+  double rt[GN];
+  float r[GN];        // its diagonal
+  int ord[GN];        // source column of position k
+};
+static_assert(sizeof(PcholIn) <= sizeof(double) * GN * GN &&
+                  sizeof(PcholOut) <= sizeof(double) * GN * GN,
+              "they fit a GN x GN FP64 matrix");
 
-  // Per lane: the keys and active flags of columns lane + 32 q.
-  float keyr[4];
-  int actr[4];
+__global__ void __launch_bounds__(GN)
+    gram_scale_kernel(int n, const double* __restrict__ G, int ldg, PcholIn* __restrict__ in) {
+  HQ_PDL_WAIT();
+  __shared__ double s_scj;
+  __shared__ float s_max[GN / 32];
+  const int i = threadIdx.x, j = blockIdx.x;
+  const double d = i < n ? G[i + (size_t)i * ldg] : 0.0;
+  const double v = i < n && j < n ? G[i + (size_t)j * ldg] : 0.0;
+  const int ok = d > 0.0 && d <= 1.7e308;
+  const double rt = ok ? sqrt(d) : 0.0;
+  const double sc = ok ? 1.0 / rt : 0.0;
+  if (i == j) s_scj = sc;
+  __syncthreads();
+  in->S[i + j * GN] = (float)(v * sc * s_scj);
+  if (j != 0) return;
+  const float l = ok ? (float)log2(d) : -4096.0f;  // squared norm, scaled below
+  float m = l;
+#pragma unroll
+  for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((i & 31) == 0) s_max[i >> 5] = m;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < GN / 32; ++w) m = fmaxf(m, s_max[w]);
+  in->rt[i] = rt;
+  in->key[i] = exp2f(l - m);
+}
+
+// Thread (warp w, lane t) holds the 64 entries (i, j) with i = t + 32 a
+// (a < 4) and j = 16 w + c (c < 16) of the full symmetric matrix.  Columns are
+// not moved: step k picks the active column p with the largest residual norm
+// (scaled Schur diagonal times the column's original squared norm relative to
+// the largest; the lowest index among residuals equal to 2^-15), the warp
+// holding column p publishes it over the active rows (0 elsewhere), every warp
+// scales it to l = S[:, p] / sqrt(S[p][p]), and every thread updates its
+// entries by S_ij -= l_i l_j -- a no-op on eliminated rows and columns, so the
+// update needs no masks.  Every warp keeps the whole diagonal (four entries a
+// lane, updated as the matrix's) and finds the pivot itself with one warp
+// maximum, so a step takes one barrier, and only the diagonal stands between a
+// published column and the next pivot.  What every warp does for itself is
+// what the SM issues most: 8 warps.  (16 warps, the diagonal passed through
+// shared memory, the FP64 scaling on the same SM: 102 us for n = 128; the
+// three kernels now take 70.)
+// Sets *stat = 0, or `bit` when a scaled pivot is not above PIVOT32_REL_MIN;
+// *alt (the second pass's choice of method) and *emax (its max|E|) := 0.
+__global__ void __launch_bounds__(CT, 1)
+    gram_pchol32_kernel(int n, const PcholIn* __restrict__ in, PcholOut* __restrict__ out,
+                        int* __restrict__ stat, int bit, int* __restrict__ alt,
+                        unsigned long long* __restrict__ emax) {
+  HQ_PDL_WAIT();
+  __shared__ __align__(16) float s_l[2][GN];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr int CPW = GN / CW;  // columns a warp
+  static_assert(CPW == 16 && GN == 128, "register layout: 8 warps x 16 columns, 32 lanes x 4 rows");
+  float S[4][CPW];
+#pragma unroll
+  for (int c = 0; c < CPW; ++c)
+#pragma unroll
+    for (int a = 0; a < 4; ++a) S[a][c] = in->S[lane + 32 * a + (CPW * warp + c) * GN];
+  // Per lane: the keys (negative once eliminated) and diagonal entries of
+  // columns lane + 32 q.
+  float keyr[4], dq[4];
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     const int j = lane + 32 * q;
-    keyr[q] = j < n ? s_key[j] : 0.0f;
-    actr[q] = j < n;
+    keyr[q] = j < n ? in->key[j] : -1.0f;
+    dq[q] = in->S[j + j * GN];
   }
+  for (int j = tid; j < GN; j += CT) out->rt[j] = in->rt[j];
   int fail = 0;
   for (int k = 0; k < n; ++k) {
     // Every warp finds the pivot: one 32-bit key per column, the residual's
     // FP32 bits above the low 8 (positive floats order like their bits) and
     // 255 - j below them, so one warp maximum gives the largest residual
-    // and, among residuals equal to 2^-15, the lowest column.
-    float dq[4];
-    unsigned best = 0u;
+    // and, among residuals equal to 2^-15, the lowest column.  Residuals below
+    // zero and eliminated columns are negative; a NaN, the largest, fails.
+    int best = 0;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int j = lane + 32 * q;
-      dq[q] = s_d[j];
-      if (actr[q]) {
-        const float v = keyr[q] * dq[q];
-        const unsigned vb = v > 0.0f ? __float_as_uint(v) : 0u;  // NaN and v <= 0: lowest
-        best = max(best, (vb & ~255u) | (unsigned)(255 - j));
-      }
-    }
+    for (int q = 0; q < 4; ++q)
+      best = max(best, (__float_as_int(keyr[q] * dq[q]) & ~255) | (255 - (lane + 32 * q)));
     best = __reduce_max_sync(0xffffffffu, best);
-    const int p = best ? 255 - (int)(best & 255u) : 0;
-    const int pq = p >> 5;
+    const int p = 255 - (best & 255);
+    const int pq = (p >> 5) & 3;
     float dsel = dq[0];
 #pragma unroll
     for (int q = 1; q < 4; ++q)
       if (q == pq) dsel = dq[q];
     const float dp = __shfl_sync(0xffffffffu, dsel, p & 31);
-    if (best == 0u || !(dp > PIVOT32_REL_MIN)) {  // also NaN and a zero column
+    if (best == 0 || !(dp > PIVOT32_REL_MIN)) {  // also NaN and a zero column
       fail = 1;
       break;
     }
     if ((p & 31) == lane) {
 #pragma unroll
       for (int q = 0; q < 4; ++q)
-        if (q == pq) actr[q] = 0;
+        if (q == pq) keyr[q] = -1.0f;
     }
-    const float r = sqrtf(dp);
-    if (tid == 0) {
-      s_r[k] = r;
-      s_ord[k] = p;
-    }
-    // The warp holding column p publishes l over the active rows (row
-    // lane + 32 a is this lane's column slot a: its flag is actr[a]).
-    if (warp == (p & 15)) {
-      const int cp = p >> 4;
-      const float rinv = 1.0f / r;
+    // The warp holding column p publishes it over the active rows (row
+    // lane + 32 a is this lane's column slot a); every warp takes the root
+    // and the quotient meanwhile and scales for itself.
+    const bool owner = warp == p / CPW;
+    if (owner) {
+      const int cp = p % CPW;
 #pragma unroll
       for (int a = 0; a < 4; ++a) {
         float v = S[a][0];
 #pragma unroll
-        for (int c = 1; c < 8; ++c)
+        for (int c = 1; c < CPW; ++c)
           if (c == cp) v = S[a][c];
-        const int i = lane + 32 * a;
-        const float l = actr[a] ? v * rinv : 0.0f;
-        s_l[i] = l;
-        s_Rp[k * GN + i] = l;
+        s_l[k & 1][lane + 32 * a] = keyr[a] >= 0.0f ? v : 0.0f;
       }
     }
+    const float r = sqrtf(dp);
+    const float rinv = 1.0f / r;
     __syncthreads();
-    float li[4], lj[8];
+    float li[4], lj[CPW];
 #pragma unroll
-    for (int a = 0; a < 4; ++a) li[a] = s_l[lane + 32 * a];
+    for (int a = 0; a < 4; ++a) {
+      li[a] = s_l[k & 1][lane + 32 * a] * rinv;
+      dq[a] = fmaf(-li[a], li[a], dq[a]);
+    }
+    const float4* l4 = reinterpret_cast<const float4*>(&s_l[k & 1][CPW * warp]);
 #pragma unroll
-    for (int c = 0; c < 8; ++c) lj[c] = s_l[warp + 16 * c];
+    for (int c = 0; c < CPW; c += 4) {
+      const float4 f = l4[c / 4];
+      lj[c] = f.x * rinv;
+      lj[c + 1] = f.y * rinv;
+      lj[c + 2] = f.z * rinv;
+      lj[c + 3] = f.w * rinv;
+    }
 #pragma unroll
     for (int a = 0; a < 4; ++a)
 #pragma unroll
-      for (int c = 0; c < 8; ++c) S[a][c] = fmaf(-li[a], lj[c], S[a][c]);
-    // Diagonal entries: lane w + 16 h of warp w holds (i, i) for
-    // i = lane + 32 a in slot c = 2 a + h.
-    if ((lane & 15) == warp) {
-      const int h = lane >> 4;
+      for (int c = 0; c < CPW; ++c) S[a][c] = fmaf(-li[a], lj[c], S[a][c]);
+    if (owner) {
 #pragma unroll
-      for (int a = 0; a < 4; ++a) s_d[lane + 32 * a] = h ? S[a][2 * a + 1] : S[a][2 * a];
+      for (int a = 0; a < 4; ++a) out->Rs[k * GN + lane + 32 * a] = li[a];
+      if (lane == 0) {
+        out->r[k] = r;
+        out->ord[k] = p;
+      }
     }
-    __syncthreads();
   }
-  // R[k][m] = Rs[k][m] sqrt(G_pp), p = perm[m]: row k of Rs at source column p.
-  for (int m = warp; m < n; m += CW)
-    for (int k = lane; k < n; k += 32) {
-      double v;
-      if (fail)
-        v = k == m ? 1.0 : 0.0;
-      else if (k < m)
-        v = (double)s_Rp[k * GN + s_ord[m]] * s_rt[s_ord[m]];
-      else
-        v = k == m ? (double)s_r[m] * s_rt[s_ord[m]] : 0.0;
-      R[k + (size_t)m * ldr] = v;
-    }
-  for (int k = tid; k < n; k += CT) perm[k] = fail ? k : s_ord[k];
   if (tid == 0) {
     *stat = fail ? bit : 0;
     *alt = 0;
     *emax = 0ull;
   }
+}
+
+// perm[m] (source column of position m) and R = Rs diag(sqrt(G_pp)) in FP64
+// (upper, zeros below); R = I and perm the identity when *stat has `bit`.
+__global__ void __launch_bounds__(GN)
+    gram_unscale_kernel(int n, const PcholOut* __restrict__ out, const int* __restrict__ stat,
+                        int bit, double* __restrict__ R, int ldr, int* __restrict__ perm) {
+  HQ_PDL_WAIT();
+  const int k = threadIdx.x, m = blockIdx.x;
+  const int fail = *stat & bit;
+  const int p = fail ? m : out->ord[m];
+  if (k < n) {
+    double v = fail ? (k == m ? 1.0 : 0.0) : 0.0;
+    if (!fail && k <= m)
+      v = (double)(k < m ? out->Rs[k * GN + p] : out->r[m]) * out->rt[p];
+    R[k + (size_t)m * ldr] = v;
+  }
+  if (k == 0) perm[m] = p;
 }
 
 // Pivot scalars of a cluster factorization step, from the updated diagonal
@@ -423,13 +441,6 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CLT, 1)
   if (bad && rank == 0 && tid == 0) atomicOr(stat, bit);
 }
 
-// E_ij (i <= j) of G = I + E, read from G's upper triangle (column j is
-// contiguous: coalesced loads).
-__device__ __forceinline__ double e_upper(const double* __restrict__ G, int ldg, int i, int j) {
-  const double g = G[i + (size_t)j * ldg];
-  return i < j ? g : g - 1.0;
-}
-
 // Fixed-point steps the second pass needs from max|E|: the error of R^{-1}
 // after m steps is about max|E|^(m+1) (measured on FP32-preconditioned
 // panels), below 2^-53 after 2 steps up to 4e-6, 3 up to 5e-5, 4 up to
@@ -449,7 +460,9 @@ __device__ __forceinline__ int nearid_steps(double emax) {
 // panels with condition numbers 10 .. 300); fewer suffice for smaller
 // max|E| (nearid_steps), and the later launches then only copy.  Every product is a column of a
 // b x b product, so the pass needs no sequential factorization: one CTA per
-// column c stages X's columns 0..c and each thread accumulates one row.
+// column c stages X's columns 0..c (asynchronous copies, all in flight at once)
+// and each thread accumulates one row (13 us for n = 128; with
+// the copies through registers and an atomic maximum per entry 30).
 // Step 0: X, Z are Uh(E), -Uh(E) (Xin, Zin unused), and the CTA checks its
 // column of E against NEARID_MAX, setting *alt when it is exceeded (the
 // later steps then return at once and the cluster Cholesky and a triangular
@@ -478,46 +491,45 @@ __global__ void __launch_bounds__(TW * 32)
       return;
     }
   }
-  for (int j0 = 4 * warp; j0 <= c; j0 += 4 * TW) {
-    double v[4][4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int j = j0 + a, i = lane + 32 * q;
-        double x = 0.0;
-        if (j <= c && i <= j) {
-          if (first) {
-            const double e = e_upper(G, ldg, i, j);
-            x = i < j ? e : 0.5 * e;
-          } else {
-            x = Xin[i + (size_t)j * ld];
-          }
-        }
-        v[a][q] = x;
-      }
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
+  {
+    const double* src = first ? G : Xin;
+    const int lds = first ? ldg : ld;
+    for (int j = warp; j <= c; j += TW)
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const int j = j0 + a, i = lane + 32 * q;
-        if (j <= c && i <= j) sX[i + j * LDS] = v[a][q];
+        const int i = lane + 32 * q;
+        if (i <= j)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                           (unsigned)__cvta_generic_to_shared(sX + i + j * LDS)),
+                       "l"(src + i + (size_t)j * lds)
+                       : "memory");
       }
   }
-  for (int k = tid; k <= c; k += TW * 32) {
-    if (first) {
-      const double e = e_upper(G, ldg, k, c);
-      s_z[k] = -(k < c ? e : 0.5 * e);
-      const double ae = fabs(e);
-      if (!(ae <= NEARID_MAX)) atomicOr(alt, 1);  // also NaN
-      // non-negative doubles order like their bits
-      else atomicMax(emax, (unsigned long long)__double_as_longlong(ae));
-    } else {
-      s_z[k] = Zin[k + (size_t)c * ld];
-    }
-  }
+  static_assert(TW * 32 == GN, "one row a thread");
+  // E's entry of this row (diagonal: minus 1) and Z's.
+  const int i = tid;
+  const double gi = i <= c ? G[i + (size_t)c * ldg] : 0.0;
+  const double ei = i == c ? gi - 1.0 : gi;
+  const double zi = !first && i <= c ? Zin[i + (size_t)c * ld] : 0.0;
+  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
-  for (int i = tid; i < n; i += TW * 32) {
+  if (first) {
+    if (i <= c) sX[i + i * LDS] = 0.5 * (sX[i + i * LDS] - 1.0);
+    // The CTA's largest |E|; non-negative doubles order like their bits.
+    const double ae = fabs(ei);
+    const int ok = i > c || ae <= NEARID_MAX;  // not for NaN
+    unsigned long long m = ok && i <= c ? (unsigned long long)__double_as_longlong(ae) : 0ull;
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+      const unsigned long long om = __shfl_xor_sync(0xffffffffu, m, o);
+      m = om > m ? om : m;
+    }
+    if (lane == 0 && m != 0ull) atomicMax(emax, m);
+    if (__syncthreads_or(!ok) && tid == 0) atomicOr(alt, 1);
+  }
+  if (i <= c) s_z[i] = first ? -sX[i + c * LDS] : zi;
+  __syncthreads();
+  if (i < n) {
     double xn = 0.0, zn = 0.0;
     if (i <= c) {
       double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
@@ -529,8 +541,7 @@ __global__ void __launch_bounds__(TW * 32)
         a3 = fma(sX[k + 3 + i * LDS], sX[k + 3 + c * LDS], a3);
       }
       for (; k <= i; ++k) a0 = fma(sX[k + i * LDS], sX[k + c * LDS], a0);
-      const double e = e_upper(G, ldg, i, c);
-      const double r = e - ((a0 + a1) + (a2 + a3));
+      const double r = ei - ((a0 + a1) + (a2 + a3));
       xn = i < c ? r : 0.5 * r;
       double b0 = 0.0, b1 = 0.0, b2 = 0.0, b3 = 0.0;
       k = i;
@@ -567,102 +578,77 @@ struct TriJob {
 };
 
 // One CTA per column c of X (and per job: blocks [0, n) run j0, [n, 2n)
-// j1): its warps stage A's columns 0..c in shared memory, then warp 0
-// computes the column with its entries in four registers per lane (rows
-// lane + 32 q) -- the inverse as a back substitution of axpys, the product
-// as rank-1 column updates.  One column per SM keeps each SM's narrow FP64
-// pipe on one dependent chain.
-__global__ void __launch_bounds__(TW * 32)
+// j1), one thread per entry.  The inverse is a back substitution: a warp holds
+// 32 entries and, once the warps after it have handed theirs over in shared
+// memory, broadcasts each entry as it becomes known and adds it to the ones
+// before it with the factors -A_ik / A_ii ready in registers: a shuffle and a
+// multiply-add a step.  The product is a sum per entry.  (One warp walking
+// the column took 33 us for n = 128; this takes 17.)
+__global__ void __launch_bounds__(GN)
     tri_kernel(int n, TriJob j0, TriJob j1, const int* __restrict__ gate) {
   HQ_PDL_WAIT();
-  extern __shared__ double sA[];  // LDS * n
-  __shared__ double s_dinv[GN];
+  __shared__ double sx[GN];
   if (gate != nullptr && *gate == 0) return;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int i = threadIdx.x, lane = i & 31, warp = i >> 5;
   const TriJob J = blockIdx.x < (unsigned)n ? j0 : j1;
   const int c = (int)(blockIdx.x % (unsigned)n);
-  const int mode = J.mode, lda = J.lda, ldb = J.ldb, ldx = J.ldx;
-  const double* __restrict__ A = J.A;
-  const double* __restrict__ B = J.B;
-  const double* __restrict__ rs = J.rs;
-  double* __restrict__ X = J.X;
-  // Stage A's columns 0..c, four columns per warp at a time (16 loads in
-  // flight per lane).
-  for (int j0 = 4 * warp; j0 <= c; j0 += 4 * TW) {
-    double v[4][4];
+  const int lda = J.lda;
+  const double* __restrict__ Ai = J.A + i;  // row i
+  const bool live = i <= c;
+  double x = 0.0;
+  if (J.mode == 0) {
+    const double dinv = live ? 1.0 / Ai[(size_t)i * lda] : 0.0;
+    double z[32];
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+    for (int d = 0; d < 32; ++d) {
+      const int k = warp * 32 + d;
+      z[d] = (k > i && k <= c) ? -Ai[(size_t)k * lda] * dinv : 0.0;
+    }
+    double acc = i == c ? 1.0 : 0.0;
+    for (int b = c >> 5; b >= 0; --b) {
+      double zb[32];
+      if (warp < b) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int j = j0 + a, i = lane + 32 * q;
-        v[a][q] = (j <= c && i <= j) ? A[i + (size_t)j * lda] : 0.0;
+        for (int d = 0; d < 32; ++d) {
+          const int k = 32 * b + d;
+          zb[d] = k <= c ? Ai[(size_t)k * lda] : 0.0;
+        }
       }
+      if (warp == b) {
+        x = acc * dinv;
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int j = j0 + a, i = lane + 32 * q;
-        if (j <= c && i <= j) sA[i + j * LDS] = v[a][q];
+        for (int d = 31; d > 0; --d) {
+          const double xd = __shfl_sync(0xffffffffu, x, d);
+          if (lane < d && 32 * b + d <= c) x = fma(xd, z[d], x);
+        }
+        sx[i] = x;
       }
-  }
-  if (mode == 0)
-    for (int i = tid; i <= c; i += TW * 32) s_dinv[i] = 1.0 / A[i + (size_t)i * lda];
-  __syncthreads();
-  if (warp != 0) return;
-  double t[4];
-  if (mode == 0) {
+      __syncthreads();
+      if (warp < b) {
+        double a1 = 0.0;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) t[q] = (lane + 32 * q == c) ? 1.0 : 0.0;
-    for (int k = c; k >= 0; --k) {
-      const int sq = k >> 5, sl = k & 31;
-      double tk = t[0];
-#pragma unroll
-      for (int q = 1; q < 4; ++q)
-        if (q == sq) tk = t[q];
-      const double xk = __shfl_sync(0xffffffffu, tk, sl) * s_dinv[k];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int i = lane + 32 * q;
-        if (q == sq && lane == sl)
-          t[q] = xk;
-        else if (32 * q < k && i < k)
-          t[q] -= sA[i + k * LDS] * xk;
+        for (int d = 0; d < 32; d += 2) {
+          acc = fma(-zb[d], sx[32 * b + d], acc);
+          a1 = fma(-zb[d + 1], sx[32 * b + d + 1], a1);
+        }
+        acc += a1;
       }
     }
   } else {
-    double bc[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int i = lane + 32 * q;
-      bc[q] = (i <= c) ? B[i + (size_t)c * ldb] : 0.0;
-      t[q] = 0.0;
+    sx[i] = live ? J.B[i + (size_t)c * J.ldb] : 0.0;
+    __syncthreads();
+    double a1 = 0.0;
+    int k = i;
+#pragma unroll 4
+    for (; k < c; k += 2) {
+      x = fma(Ai[(size_t)k * lda], sx[k], x);
+      a1 = fma(Ai[(size_t)(k + 1) * lda], sx[k + 1], a1);
     }
-    for (int k = 0; k <= c; ++k) {
-      const int sq = k >> 5, sl = k & 31;
-      double bk = bc[0];
-#pragma unroll
-      for (int q = 1; q < 4; ++q)
-        if (q == sq) bk = bc[q];
-      bk = __shfl_sync(0xffffffffu, bk, sl);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int i = lane + 32 * q;
-        if (32 * q <= k && i <= k) t[q] += sA[i + k * LDS] * bk;
-      }
-    }
-    if (rs) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int i = lane + 32 * q;
-        if (i <= c) t[q] *= rs[i];
-      }
-    }
+    if (k == c) x = fma(Ai[(size_t)k * lda], sx[k], x);
+    x += a1;
+    if (J.rs && live) x *= J.rs[i];
   }
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int i = lane + 32 * q;
-    if (i < n) X[i + (size_t)c * ldx] = (i <= c) ? t[q] : 0.0;
-  }
+  if (i < n) J.X[i + (size_t)c * J.ldx] = live ? x : 0.0;
 }
 
 // When *stat == 0: the panel P (mp x n, ldp) gets R on and above the
@@ -711,17 +697,16 @@ __global__ void gram_commit_kernel(int mp, int n, double* __restrict__ P, int ld
 
 }  // namespace
 
-extern "C" int hq_gram_pchol32(cudaStream_t stream, int n, const double* G, int ldg, double* R,
+extern "C" int hq_gram_pchol32(cudaStream_t stream, int n, double* G, int ldg, double* R,
                                int ldr, int* perm, int* stat, int bit, int* alt,
                                unsigned long long* emax) {
-  if (n <= 0 || n > GN) return (int)cudaErrorInvalidValue;
-  const size_t smem = sizeof(float) * (size_t)GN * GN;
-  cudaError_t e = cudaFuncSetAttribute(gram_pchol32_kernel,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return (int)e;
-  hq_launch(gram_pchol32_kernel, 1, CT, smem, stream, n, G, ldg, R, ldr, perm, stat, bit, alt,
-                                                emax);
-  hq_count_launches(1);
+  if (n <= 0 || n > GN || ldg != GN || ldr != GN) return (int)cudaErrorInvalidValue;
+  PcholIn* in = reinterpret_cast<PcholIn*>(R);
+  PcholOut* out = reinterpret_cast<PcholOut*>(G);
+  hq_launch(gram_scale_kernel, GN, GN, 0, stream, n, G, ldg, in);
+  hq_launch(gram_pchol32_kernel, 1, CT, 0, stream, n, in, out, stat, bit, alt, emax);
+  hq_launch(gram_unscale_kernel, n, GN, 0, stream, n, out, stat, bit, R, ldr, perm);
+  hq_count_launches(3);
   return (int)cudaGetLastError();
 }
 
@@ -778,13 +763,9 @@ extern "C" int hq_tri2g(cudaStream_t stream, int n, int mode0, const double* A0,
   if (n <= 0) return 0;
   if (n > GN || mode0 < 0 || mode0 > 1 || mode1 < -1 || mode1 > 1)
     return (int)cudaErrorInvalidValue;
-  const size_t smem = sizeof(double) * (size_t)LDS * (size_t)n;
-  cudaError_t e =
-      cudaFuncSetAttribute(tri_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return (int)e;
   const TriJob j0 = {mode0, A0, lda0, B0, ldb0, rs0, X0, ldx0};
   const TriJob j1 = {mode1 < 0 ? 0 : mode1, A1, lda1, B1, ldb1, rs1, X1, ldx1};
-  hq_launch(tri_kernel, mode1 < 0 ? n : 2 * n, TW * 32, smem, stream, n, j0, j1, gate);
+  hq_launch(tri_kernel, mode1 < 0 ? n : 2 * n, GN, 0, stream, n, j0, j1, gate);
   hq_count_launches(1);
   return (int)cudaGetLastError();
 }
