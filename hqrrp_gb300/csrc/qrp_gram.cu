@@ -26,8 +26,8 @@
 // tensor-core products issued by the host driver; the b x b steps are the
 // kernels of this file.  FP64 runs at about two lanes per clock on a GB300
 // SM, so one SM is slow for them: the FP64 Cholesky and LU run on a cluster
-// of eight CTAs (each owns every eighth column; the pivot column travels
-// through distributed shared memory), the triangular inverses and products
+// of eight CTAs (each owns every eighth column, or group of four; the pivot
+// columns travel through distributed shared memory), the triangular inverses and products
 // and the first pass's scaling with one CTA per column, and only the pivoted
 // first pass itself on one SM, in FP32.
 //
@@ -43,6 +43,7 @@
 
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
+#include <limits.h>
 #include <math.h>
 
 #include "hq_common.cuh"
@@ -256,67 +257,55 @@ __global__ void __launch_bounds__(GN)
   if (k == 0) perm[m] = p;
 }
 
-// Pivot scalars of a cluster factorization step, from the updated diagonal
-// entry q of the pivot column (one thread): Cholesky (mode 0) r = sqrt(q),
-// bad when q <= 1e-10 d0; LU (mode 1) D = -1 if q >= 0 else +1, u = q - D,
-// bad when |u| is outside [0.5, 2.5].  A bad pivot is replaced by 1.
-__device__ __forceinline__ void cluster_scalars(int mode, double q, double d0, double* out) {
-  double piv, D = 0.0;
-  int bad;
-  if (mode == 0) {
-    bad = !(q > CHOL2_REL_MIN * d0);
-    piv = bad ? 1.0 : sqrt(q);
-  } else {
-    D = q >= 0.0 ? -1.0 : 1.0;
-    const double u = q - D;
-    const double au = fabs(u);
-    bad = !(au >= 0.5 && au <= 2.5);
-    piv = bad ? 1.0 : u;
-  }
-  out[0] = piv;
-  // 1 / piv: an FP32 quotient refined by two Newton steps y += y (1 - piv y)
-  // (2^-24 -> 2^-48 -> FP64 rounding), four dependent FMAs instead of the
-  // longer FP64 division sequence on this critical path; piv lies in
-  // [0.5, 2.5] (LU) or is a square root of a diagonal entry well inside
-  // FP32's range (Cholesky of a scaled Gram matrix).
-  double y = (double)(1.0f / (float)piv);
-  y = fma(y, fma(-piv, y, 1.0), y);
-  y = fma(y, fma(-piv, y, 1.0), y);
-  out[1] = y;
-  out[2] = D;
-  out[3] = bad ? 1.0 : 0.0;
+// An FP32 approximation of 1 / x as an FP64, for |x| well inside FP32's range
+// (LU: 0.5 .. 2.5; Cholesky: the root of a diagonal entry of a scaled Gram
+// matrix).  Both conversions take integer instructions: x's bits are cut to
+// FP32's, the quotient's widened.
+__device__ __forceinline__ double seed_inverse(double x) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const unsigned f =
+      (hi & 0x80000000u) | ((((hi & 0x7FFFFFFFu) - 0x38000000u) << 3) | (lo >> 29));
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__uint_as_float(f)));
+  const unsigned r = __float_as_uint(y);
+  return __hiloint2double((int)((r & 0x80000000u) | (((r & 0x7FFFFFFFu) >> 3) + 0x38000000u)),
+                          (int)(r << 29));
 }
 
-// Unpivoted FP64 factorization of an n x n matrix A (lda) on a cluster of CL
-// CTAs:
-//   mode 0: Cholesky of the symmetric A (lower triangle read); F := R (upper,
-//           zeros below) with R^T R = A;
-//   mode 1: LU of A - D, D_kk = -1 if the k-th Schur pivot is >= 0 else +1
-//           (Householder reconstruction); F := L strictly below the diagonal
-//           and U on and above it, dsgn := D, tau := -D U_kk.
-// Column j lives in the shared memory of CTA j % CL.  Step k: every CTA
-// updates its columns right of k from the published, scaled column k; the
-// owner of column k + 1 updates that column first, takes its pivot scalars,
-// scales it and writes it into every CTA's receive buffer (distributed
-// shared memory, double-buffered by the parity of the step).  One cluster
-// barrier per step, split into arrive and wait around the update of the
-// remaining own columns; it also orders the receive buffers' reuse.  A bad
-// pivot is recorded and replaced by 1, so every CTA takes the same barriers;
-// the output is then the identity (and tau 0) and `bit` is set in *stat.
+// 1 / x from that seed y and one third-order correction: with e = 1 - x y,
+// 1 / x = y (1 + e + e^2 + ...), so y + y (e + e^2) leaves e^3 ~ 2^-66: three
+// dependent FMAs instead of the longer FP64 division sequence.
+__device__ __forceinline__ double quick_inverse(double x) {
+  const double y = seed_inverse(x);
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+
+// Unpivoted FP64 Cholesky factorization of the symmetric n x n matrix A (lda,
+// lower triangle read) on a cluster of CL CTAs: F := R (upper, zeros below)
+// with R^T R = A.  Column j lives in the shared memory of CTA j % CL.  Step k:
+// every CTA updates its columns right of k from the published, scaled column k;
+// the owner of column k + 1 updates that column first, takes its root, scales
+// it and writes it into every CTA's receive buffer (distributed shared memory,
+// double-buffered by the parity of the step).  One cluster barrier per step,
+// split into arrive and wait around the update of the remaining own columns;
+// it also orders the receive buffers' reuse.  A pivot q <= 1e-10 d0 is recorded
+// and replaced by 1, so every CTA takes the same barriers; the output is then
+// the identity and `bit` is set in *stat.  (Only panels without pivoting, and
+// second passes far from the identity, come here.)
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CLT, 1)
-    cluster_fact_kernel(int n, int mode, const double* __restrict__ A, int lda,
-                        double* __restrict__ F, int ldf, double* __restrict__ dsgn,
-                        double* __restrict__ tau, int* __restrict__ stat, int bit,
-                        const int* __restrict__ gate) {
+    cluster_chol_kernel(int n, const double* __restrict__ A, int lda, double* __restrict__ F,
+                        int ldf, int* __restrict__ stat, int bit, const int* __restrict__ gate) {
   HQ_PDL_WAIT();
   if (gate != nullptr && *gate == 0) return;  // every CTA of the cluster reads the same word
   cg::cluster_group cl = cg::this_cluster();
   const int rank = (int)cl.block_rank();
   __shared__ double Xc[OWN * LDS];
   __shared__ double colbuf[2][GN];
-  __shared__ double scal[2][4];  // pivot, 1 / pivot, D, bad
-  __shared__ double s_pub[4];
-  __shared__ double s_d0[OWN], s_D[OWN];
+  __shared__ int s_bad[2];
+  __shared__ double s_pub[2];  // root, 1 / root
+  __shared__ int s_pubbad;
+  __shared__ double s_d0[OWN];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nown = rank < n ? (n - 1 - rank) / CL + 1 : 0;
   for (int c = warp; c < nown; c += CLW) {
@@ -325,7 +314,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CLT, 1)
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int i = lane + 32 * q;
-      v[q] = (i < n && (mode == 1 || i >= j)) ? A[i + (size_t)j * lda] : 0.0;
+      v[q] = (i < n && i >= j) ? A[i + (size_t)j * lda] : 0.0;
     }
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -336,16 +325,20 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CLT, 1)
   __syncthreads();
   for (int c = tid; c < nown; c += CLT) s_d0[c] = Xc[(rank + CL * c) + c * LDS];
 
-  // Publish own column kk (local c): scalars, final diagonal, scaled rows
-  // below it, into every CTA's buffers of parity par.  Thread 0 wrote the
-  // column's diagonal entry itself (it updates row kk), so it takes the
-  // scalars before the barrier that orders the other rows' updates.
+  // Publish own column kk (local c): root, final diagonal, scaled rows below
+  // it, into every CTA's buffers of parity par.  Thread 0 wrote the column's
+  // diagonal entry itself (it updates row kk), so it takes the root before
+  // the barrier that orders the other rows' updates.
   auto publish = [&](int kk, int par) {
     const int c = kk / CL;
     if (tid == 0) {
-      cluster_scalars(mode, Xc[kk + c * LDS], s_d0[c], s_pub);
-      Xc[kk + c * LDS] = s_pub[0];
-      s_D[c] = s_pub[2];
+      const double q = Xc[kk + c * LDS];
+      const int bad = !(q > CHOL2_REL_MIN * s_d0[c]);
+      const double piv = bad ? 1.0 : sqrt(q);
+      s_pub[0] = piv;
+      s_pub[1] = quick_inverse(piv);
+      s_pubbad = bad;
+      Xc[kk + c * LDS] = piv;
     }
     __syncthreads();
     const double inv = s_pub[1];
@@ -355,13 +348,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CLT, 1)
 #pragma unroll
       for (int r = 0; r < CL; ++r) *cl.map_shared_rank(&colbuf[par][i], r) = l;
     }
-    if (tid < CL) {
-      double* d = cl.map_shared_rank(&scal[par][0], tid);
-      d[0] = s_pub[0];
-      d[1] = s_pub[1];
-      d[2] = s_pub[2];
-      d[3] = s_pub[3];
-    }
+    if (tid < CL) *cl.map_shared_rank(&s_bad[par], tid) = s_pubbad;
   };
 
   if (rank == 0 && n > 0) publish(0, 0);
@@ -372,13 +359,8 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CLT, 1)
     const int nx = k + 1;
     if (nx < n && nx % CL == rank) {
       const int c1 = nx / CL;
-      if (mode == 1) {
-        const double ukj = Xc[k + c1 * LDS];
-        for (int i = k + 1 + tid; i < n; i += CLT) Xc[i + c1 * LDS] -= colbuf[b][i] * ukj;
-      } else {
-        const double lj = colbuf[b][nx];
-        for (int i = nx + tid; i < n; i += CLT) Xc[i + c1 * LDS] -= colbuf[b][i] * lj;
-      }
+      const double lj = colbuf[b][nx];
+      for (int i = nx + tid; i < n; i += CLT) Xc[i + c1 * LDS] -= colbuf[b][i] * lj;
       publish(nx, b ^ 1);
     }
     // The other own columns right of k: warp w takes local columns w and
@@ -393,8 +375,8 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CLT, 1)
       for (int u = 0; u < 2; ++u) {
         const int c = warp + CLW * u, j = rank + CL * c;
         act[u] = c < nown && j > k && j != nx;
-        mult[u] = act[u] ? (mode == 1 ? Xc[k + c * LDS] : colbuf[b][j]) : 0.0;
-        base[u] = mode == 1 ? k + 1 : j;
+        mult[u] = act[u] ? colbuf[b][j] : 0.0;
+        base[u] = j;
       }
 #pragma unroll
       for (int u = 0; u < 2; ++u)
@@ -405,7 +387,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CLT, 1)
           xa[u][q] = live ? Xc[i + c * LDS] : 0.0;
           lb[u][q] = live ? colbuf[b][i] : 0.0;
         }
-      bad |= scal[b][3] != 0.0;
+      bad |= s_bad[b];
       cl.barrier_arrive();
 #pragma unroll
       for (int u = 0; u < 2; ++u)
@@ -418,26 +400,239 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CLT, 1)
     __syncthreads();  // the CTA's own updates (after its arrive) before the next step reads them
     cl.barrier_wait();
   }
-  // Output of the own columns.
+  // R[g][i] = L[i][g]; R[i][g] = 0 below the diagonal
   for (int c = warp; c < nown; c += CLW) {
     const int g = rank + CL * c;
-    for (int i = lane; i < n; i += 32) {
-      const double x = Xc[i + c * LDS];
-      if (mode == 1) {
-        F[i + (size_t)g * ldf] = bad ? (i == g ? 1.0 : 0.0) : x;
-      } else if (i >= g) {
-        // R[g][i] = L[i][g]; R[i][g] = 0 below the diagonal
-        F[g + (size_t)i * ldf] = bad ? (i == g ? 1.0 : 0.0) : x;
-        if (i > g) F[i + (size_t)g * ldf] = 0.0;
-      }
+    for (int i = g + lane; i < n; i += 32) {
+      F[g + (size_t)i * ldf] = bad ? (i == g ? 1.0 : 0.0) : Xc[i + c * LDS];
+      if (i > g) F[i + (size_t)g * ldf] = 0.0;
     }
   }
-  if (mode == 1)
-    for (int c = tid; c < nown; c += CLT) {
-      const int g = rank + CL * c;
-      dsgn[g] = bad ? -1.0 : s_D[c];
-      tau[g] = bad ? 0.0 : -s_D[c] * Xc[g + c * LDS];
+  if (bad && rank == 0 && tid == 0) atomicOr(stat, bit);
+}
+
+// Unpivoted FP64 LU of A - D (n x n), D_kk = -1 if the k-th Schur pivot is >= 0
+// else +1 (Householder reconstruction), on a cluster of CL CTAs: F := L
+// strictly below the diagonal and U on and above it, dsgn := D, tau :=
+// -D U_kk.
+//
+// Columns go in groups of LUG: group g lives in the shared memory of CTA
+// g % CL.  Step g: the owner of group g + 1 brings it up to date with group g,
+// factors its diagonal block in one warp (registers and shuffles) while the
+// other warps update the rows below, solves those rows for L, and writes L's
+// four columns into every CTA's receive buffer (distributed shared memory);
+// the other columns are updated between the arrive and the wait of the step's
+// cluster barrier.  Three receive buffers: group g's is read until a CTA
+// arrives at step g + 1 and written again during step g + 2.  (A barrier and
+// an exchange per column instead of per group took 152 us for n = 128; this
+// takes 105, most of it the diagonal blocks' chains of a quotient, a product
+// and an update per column.)  A pivot |u| outside [0.5, 2.5] is recorded and
+// replaced by 1; the output is then the identity (and tau 0) and `bit` is set
+// in *stat.
+constexpr int LUG = 4;
+__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CLT, 1)
+    cluster_lu_kernel(int n, const double* __restrict__ A, int lda, double* __restrict__ F,
+                      int ldf, double* __restrict__ dsgn, double* __restrict__ tau,
+                      int* __restrict__ stat, int bit) {
+  HQ_PDL_WAIT();
+  cg::cluster_group cl = cg::this_cluster();
+  const int rank = (int)cl.block_rank();
+  __shared__ double Xc[OWN * LDS];
+  // Row i of the published group's L (zeros on and above the diagonal).
+  __shared__ __align__(16) double Lb[3][GN][LUG];
+  __shared__ int s_badb[3];
+  __shared__ __align__(16) double s_l44[LUG][LUG];
+  __shared__ double s_u44[LUG][LUG], s_inv[LUG], s_u[LUG][LUG], s_D[OWN];
+  __shared__ int s_bad;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  static_assert(OWN % LUG == 0 && OWN == 2 * CLW && CLT == 256, "layout");
+  const int ng = (n + LUG - 1) / LUG;
+  auto column = [&](int c) { return ((c / LUG) * CL + rank) * LUG + c % LUG; };
+  for (int c = warp; c < OWN; c += CLW) {
+    const int j = column(c);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int i = lane + 32 * q;
+      Xc[i + c * LDS] = (i < n && j < n) ? A[i + (size_t)j * lda] : 0.0;
     }
+  }
+  __syncthreads();
+
+  // U's entries x[k .. k + 3] of a column against group buffer L, k its first row.
+  auto solve4 = [&](const double (*L)[LUG], int k, const double* x, double (&u)[LUG]) {
+    u[0] = x[k];
+    u[1] = fma(-L[k + 1][0], u[0], x[k + 1]);
+    u[2] = fma(-L[k + 2][1], u[1], fma(-L[k + 2][0], u[0], x[k + 2]));
+    u[3] = fma(-L[k + 3][2], u[2],
+               fma(-L[k + 3][1], u[1], fma(-L[k + 3][0], u[0], x[k + 3])));
+  };
+
+  // Bring own group gg up to date with group gg - 1, factor and publish it.
+  auto factor = [&](int gg) {
+    const int k0 = LUG * gg, kp = k0 - LUG, lc = LUG * (gg / CL);
+    const double (*L)[LUG] = Lb[(gg + 2) % 3];
+    double* X = Xc + lc * LDS;
+    if (warp == 0) {
+      const int r = (lane >> 2) & 3, cc = lane & 3;
+      double v = X[min(k0 + r, GN - 1) + cc * LDS];
+      if (gg > 0) {
+        double u[LUG];
+        solve4(L, kp, X + cc * LDS, u);
+        const double* lr = L[min(k0 + r, GN - 1)];
+        v = fma(-lr[1], u[1], fma(-lr[0], u[0], v)) - fma(lr[3], u[3], lr[2] * u[2]);
+      }
+      int bad = 0;
+#pragma unroll
+      for (int kk = 0; kk < LUG; ++kk) {
+        if (k0 + kk >= n) break;
+        const double q = __shfl_sync(0xffffffffu, v, kk * 4 + kk);
+        const double a = __shfl_sync(0xffffffffu, v, r * 4 + kk);
+        const double uk = __shfl_sync(0xffffffffu, v, kk * 4 + cc);
+        // The comparisons are of the bits: an FP64 one holds the chain up.
+        const long long qb = __double_as_longlong(q);
+        const double D = qb >= 0 || qb == LLONG_MIN ? -1.0 : 1.0;
+        double piv = q - D;
+        const long long ub = __double_as_longlong(piv) & LLONG_MAX;
+        if (!(ub >= 0x3FE0000000000000LL && ub <= 0x4004000000000000LL)) {  // 0.5, 2.5
+          bad = 1;
+          piv = 1.0;
+        }
+        // quick_inverse, and a / piv beside it.
+        const double y = seed_inverse(piv);
+        const double e = fma(-piv, y, 1.0), ay = a * y;
+        const double t = fma(e, e, e);
+        const double l = fma(ay, t, ay);
+        if (r > kk && cc > kk) v = fma(-l, uk, v);
+        if (r > kk && cc == kk) v = l;
+        if (r == kk && cc == kk) v = piv;
+        if (lane == 0) {
+          s_inv[kk] = fma(y, t, y);
+          s_D[lc + kk] = D;
+        }
+      }
+      if (lane < 16) {
+        if (k0 + r < n) X[k0 + r + cc * LDS] = v;
+        s_l44[r][cc] = r > cc ? v : 0.0;
+        s_u44[r][cc] = v;
+      }
+      if (lane == 0) s_bad = bad;
+    } else if (gg > 0) {
+      if (warp == 1 && lane < LUG) {
+        double u[LUG];
+        solve4(L, kp, X + lane * LDS, u);
+#pragma unroll
+        for (int s = 0; s < LUG; ++s) s_u[lane][s] = u[s];
+      }
+      __syncwarp();
+      asm volatile("bar.sync 1, %0;" ::"n"(CLT - 32) : "memory");  // warps 1 on
+      // (Warp 4 would share its FP64 pipe with warp 0.)
+      for (int it = warp < 4 ? warp - 1 : warp == 4 ? 4 * LUG : warp - 2; it < 4 * LUG;
+           it += CLW - 2) {
+        const int cc = it & 3, i = k0 + LUG + lane + 32 * (it >> 2);
+        if (i < n) {
+          const double2 l01 = *reinterpret_cast<const double2*>(&L[i][0]);
+          const double2 l23 = *reinterpret_cast<const double2*>(&L[i][2]);
+          double x = X[i + cc * LDS];
+          x = fma(-l01.x, s_u[cc][0], x);
+          x = fma(-l01.y, s_u[cc][1], x);
+          x = fma(-l23.x, s_u[cc][2], x);
+          X[i + cc * LDS] = fma(-l23.y, s_u[cc][3], x);
+        }
+      }
+    }
+    __syncthreads();
+    const int par = gg % 3;
+    if (tid < GN) {
+      const int i = k0 + LUG + tid;
+      if (i < n) {  // then the group is full
+        double a0 = X[i], a1 = X[i + LDS], a2 = X[i + 2 * LDS], a3 = X[i + 3 * LDS];
+        double2 l01, l23;
+        l01.x = a0 * s_inv[0];
+        a1 = fma(-l01.x, s_u44[0][1], a1);
+        a2 = fma(-l01.x, s_u44[0][2], a2);
+        a3 = fma(-l01.x, s_u44[0][3], a3);
+        l01.y = a1 * s_inv[1];
+        a2 = fma(-l01.y, s_u44[1][2], a2);
+        a3 = fma(-l01.y, s_u44[1][3], a3);
+        l23.x = a2 * s_inv[2];
+        a3 = fma(-l23.x, s_u44[2][3], a3);
+        l23.y = a3 * s_inv[3];
+        X[i] = l01.x;
+        X[i + LDS] = l01.y;
+        X[i + 2 * LDS] = l23.x;
+        X[i + 3 * LDS] = l23.y;
+#pragma unroll
+        for (int d = 0; d < CL; ++d) {
+          double* p = cl.map_shared_rank(&Lb[par][i][0], d);
+          *reinterpret_cast<double2*>(p) = l01;
+          *reinterpret_cast<double2*>(p + 2) = l23;
+        }
+      }
+    } else if (warp == 4) {
+      const int d = lane >> 2, r = lane & 3;
+      if (k0 + r < n) {
+        double* p = cl.map_shared_rank(&Lb[par][k0 + r][0], d);
+        *reinterpret_cast<double2*>(p) = *reinterpret_cast<const double2*>(&s_l44[r][0]);
+        *reinterpret_cast<double2*>(p + 2) = *reinterpret_cast<const double2*>(&s_l44[r][2]);
+      }
+    } else if (warp == 5) {
+      if (lane < CL) *cl.map_shared_rank(&s_badb[par], lane) = s_bad;
+    } else if (warp == 6 && gg > 0 && lane < LUG * LUG) {
+      X[kp + (lane >> 2) + (lane & 3) * LDS] = s_u[lane & 3][lane >> 2];
+    }
+  };
+
+  if (rank == 0) factor(0);
+  cl.sync();
+  int bad = 0;
+  for (int g = 0; g < ng; ++g) {
+    const double (*L)[LUG] = Lb[g % 3];
+    const int k0 = LUG * g;
+    bad |= s_badb[g % 3];
+    if (g + 1 < ng && (g + 1) % CL == rank) factor(g + 1);
+    __syncwarp();
+    cl.barrier_arrive();
+    // The other own columns right of the group: warp w takes local columns w
+    // and w + CLW.
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int c = warp + CLW * h, gc = (c / LUG) * CL + rank;
+      if (gc <= g + (((g + 1) % CL) == rank ? 1 : 0) || column(c) >= n) continue;
+      double* x = Xc + c * LDS;
+      double u[LUG];
+      solve4(L, k0, x, u);
+      __syncwarp();
+      if (lane < LUG) x[k0 + lane] = lane == 0 ? u[0] : lane == 1 ? u[1] : lane == 2 ? u[2] : u[3];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int i = k0 + LUG + lane + 32 * q;
+        if (i < n) {
+          const double2 l01 = *reinterpret_cast<const double2*>(&L[i][0]);
+          const double2 l23 = *reinterpret_cast<const double2*>(&L[i][2]);
+          double v = x[i];
+          v = fma(-l01.x, u[0], v);
+          v = fma(-l01.y, u[1], v);
+          v = fma(-l23.x, u[2], v);
+          x[i] = fma(-l23.y, u[3], v);
+        }
+      }
+    }
+    __syncthreads();
+    cl.barrier_wait();
+  }
+  // Output of the own columns.
+  for (int c = warp; c < OWN; c += CLW) {
+    const int j = column(c);
+    if (j >= n) continue;
+    for (int i = lane; i < n; i += 32)
+      F[i + (size_t)j * ldf] = bad ? (i == j ? 1.0 : 0.0) : Xc[i + c * LDS];
+  }
+  for (int c = tid; c < OWN; c += CLT) {
+    const int j = column(c);
+    if (j >= n) continue;
+    dsgn[j] = bad ? -1.0 : s_D[c];
+    tau[j] = bad ? 0.0 : -s_D[c] * Xc[j + c * LDS];
+  }
   if (bad && rank == 0 && tid == 0) atomicOr(stat, bit);
 }
 
@@ -714,8 +909,10 @@ extern "C" int hq_cluster_fact(cudaStream_t stream, int n, int mode, const doubl
                                double* F, int ldf, double* dsgn, double* tau, int* stat, int bit,
                                const int* gate) {
   if (n <= 0 || n > GN || mode < 0 || mode > 1) return (int)cudaErrorInvalidValue;
-  hq_launch(cluster_fact_kernel, CL, CLT, 0, stream, n, mode, A, lda, F, ldf, dsgn, tau, stat, bit,
-                                              gate);
+  if (mode == 0)
+    hq_launch(cluster_chol_kernel, CL, CLT, 0, stream, n, A, lda, F, ldf, stat, bit, gate);
+  else
+    hq_launch(cluster_lu_kernel, CL, CLT, 0, stream, n, A, lda, F, ldf, dsgn, tau, stat, bit);
   hq_count_launches(1);
   return (int)cudaGetLastError();
 }
