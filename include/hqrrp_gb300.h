@@ -261,10 +261,10 @@ int hqrrp_gb300_profile_counts(int* counts, int n);
 /* Number of kernels this library has launched in this process. */
 unsigned long long hqrrp_gb300_launch_count(void);
 
-/* Number of device allocations this library has made from its memory pools
+/* Number of device buffers this library has drawn from its memory pools
  * in this process (every entry point except hqrrp_gb300_qrp_noalloc draws its
- * workspace from a pool).  Setting HQRRP_GB300_FAIL_ALLOC=k in the
- * environment makes the k-th allocation of every later call fail as if the
+ * workspace from a pool; small buffers share one allocation).  Setting HQRRP_GB300_FAIL_ALLOC=k in the
+ * environment makes the k-th buffer of every later call fail as if the
  * device were out of memory (return code 4, dgeqp4 info 1004): host-side
  * fault injection for testing callers' error paths. */
 unsigned long long hqrrp_gb300_pool_alloc_count(void);
