@@ -48,10 +48,9 @@ sys.path.insert(0, ROOT)
 
 METRIC = "dgeqp4 TFLOP/s at n=16384, mixed vs plain FP64 at equal residual; bwd ms"
 # DRAM bytes per algorithmic flop of the dominant kernels, from ncu captures at
-# m = n = 6144 (committed summaries under profiles/): the split-BF16 products
-# -- W1 = U'^T C reading C as FP64 (302.1 MB per 2.43e11 BF16 flops,
-# ozk_gemm_c64_n6144.md) and C -= U'W2 (556.1 MB per 2.649e11, ozk_gemm_n6144.md)
-# -- and the FP64 update GEMMs of the plain path (W1, C -= U W2).
+# m = n = 6144: the split-BF16 products -- W1 = U'^T C reading C as FP64
+# (302.1 MB per 2.43e11 BF16 flops) and C -= U'W2 (556.1 MB per 2.649e11) -- and
+# the FP64 update GEMMs of the plain path (W1, C -= U W2).
 TENSOR_BYTES_PER_FLOP = (302.1e6 + 556.1e6) / (2.43e11 + 2.649e11)
 FP64_UPDATE_BYTES_PER_FLOP = (314.4e6 + 546.3e6) / (2 * 9.462e9)
 

@@ -634,7 +634,8 @@ int panel_grid(const hq_device_info* dev, int mp, int nc) {
 // theirs over in shared memory, and within the warp each entry, once known,
 // is broadcast and added to the ones after it with the factors -tau_i Z[c, i]
 // ready in registers -- a shuffle and a fused multiply-add a step.  (A dot
-// product and a warp sum a step took 60 us for k = 64; this takes 9.)
+// product and a warp sum a step took 60 us for k = 64 and 132 for 128; this
+// takes 9 and 16.)
 __global__ void __launch_bounds__(HQ_MAX_MY) larft_rows_kernel(
     int k, const double* __restrict__ Z, int ldz, const double* __restrict__ tau,
     double* __restrict__ T, int ldt) {
