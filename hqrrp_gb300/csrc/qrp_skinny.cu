@@ -11,7 +11,9 @@
 // discarded and the swaps of A, Y and the labels are composed into one
 // permutation that a gather kernel applies afterwards.
 //
-// GB300 layout: the N columns are split into contiguous ranges, one range per
+// Two kernels: one keeps the columns in registers and exchanges tagged words
+// (skinny_qrp_reg_kernel, below); what does not fit it takes the one described
+// here.  The N columns are split into contiguous ranges, one range per
 // CTA (one CTA per SM), and a range stays in that CTA's shared memory for all
 // b stages (138 x 108 doubles = 119 KB at N = 16384, nb = 128), falling back
 // to an L2-resident global copy when it does not fit.  A column never changes
