@@ -281,7 +281,6 @@ __global__ void __launch_bounds__(NT, 1) panel_qrp_kernel(PnArgs a) {
   // become complete, and the reflector (built by one thread of every CTA from
   // the same inputs).  Returns false in every thread if a wait gave up.
   auto gather_sums = [&](int s) {
-    const double sep = se[s];
     const bool odd = s & 1;
     const unsigned long long tag = (unsigned long long)s + 1ull;
     unsigned long long w[EPT][R][3], xr[EPT], xt[EPT];
@@ -310,8 +309,10 @@ __global__ void __launch_bounds__(NT, 1) panel_qrp_kernel(PnArgs a) {
       const int k = tid + NT * j;
       if (k >= s && k < nc) load(j, k);
     }
-    // sw and srow, written below, are read until here by the pass before.
+    // sw and srow, written below, are read until here by the pass before, in
+    // which one thread rewrites the labels: se[s] is read from here on.
     __syncthreads();
+    const double sep = se[s];
     int bad = 0;
     unsigned it = 0;
 #pragma unroll
