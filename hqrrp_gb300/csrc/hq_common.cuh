@@ -261,3 +261,15 @@ __device__ __forceinline__ void hq_red_word(void* p, unsigned long long v) {
 
 // LAPACK's tol3z = sqrt(dlamch('Epsilon')) with eps = 2^-53.
 #define HQ_TOL3Z 1.0536712127723509e-08
+
+// Whether a downdated squared norm nd = d^2 - r^2 has lost its digits and is
+// recomputed: nd <= thr = tol3z e^2, e the norm when it was last computed in
+// full.  On the integer pipe: thr >= 0, and a negative difference orders below
+// it.  As in LAPACK's test, a NaN or an infinite norm is kept: computed again at
+// every later stage it would be no better, and each costs the stage a second
+// pass.
+__device__ __forceinline__ bool hq_norm_cancelled(double nd, double thr) {
+  const long long inf = 0x7ff0000000000000LL;
+  const long long nb = __double_as_longlong(nd), tb = __double_as_longlong(thr);
+  return nb <= tb && tb < inf && (nb & 0x7fffffffffffffffLL) <= inf;
+}

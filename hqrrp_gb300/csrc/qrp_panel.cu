@@ -451,11 +451,8 @@ __global__ void __launch_bounds__(NT, 1) panel_qrp_kernel(PnArgs a) {
         int flag = 0;
         double dk = sd[k];
         if (dk != 0.0) {
-          // On the integer pipe: the bound is >= 0, a negative difference
-          // orders below it, and a NaN is recomputed.
           const double nd = fma(-r, r, dk);
-          const long long nb = __double_as_longlong(nd);
-          if (nb <= __double_as_longlong(thr) || nb > 0x7ff0000000000000LL) {
+          if (hq_norm_cancelled(nd, thr)) {
             flag = 1;
           } else {
             dk = nd;

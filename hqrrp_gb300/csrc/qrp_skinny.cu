@@ -677,15 +677,13 @@ __global__ void __launch_bounds__(CNT + 32, 1) skinny_qrp_reg_kernel(RegArgs a) 
       }
     }
     __syncthreads();
-    // Norm downdate, one thread per column (LAWN 176 on squared norms, the
-    // comparison on the integer pipe: thr >= 0, and a negative difference
-    // orders below it); flagged norms are recomputed from the registers.
+    // Norm downdate, one thread per column (LAWN 176 on squared norms); flagged
+    // norms are recomputed from the registers.
     int flag = 0;
     if (dd && dpos > s && dn != 0.0) {
       const double r = F32 ? (double)srs[tid] * unscale : (double)srs[tid];
       const double nd = fma(-r, r, dn);
-      const long long nb = __double_as_longlong(nd);
-      if (nb <= __double_as_longlong(thr) || nb > 0x7ff0000000000000LL) flag = 1;
+      if (hq_norm_cancelled(nd, thr)) flag = 1;
       else dn = nd;
     }
     if (tid < NC) sflag[tid] = flag;

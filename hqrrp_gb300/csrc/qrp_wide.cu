@@ -279,8 +279,7 @@ __global__ void __launch_bounds__(WT, 1) wide_qrp_kernel(WdArgs a) {
       if (d != 0.0) {
         const double r = srs[q];
         const double nd = fma(-r, r, d);
-        const long long nb = __double_as_longlong(nd);
-        if (nb <= __double_as_longlong(sthr[q]) || nb > 0x7ff0000000000000LL) flag = 1;
+        if (hq_norm_cancelled(nd, sthr[q])) flag = 1;
         else sd[q] = nd;
       }
       if (flag) sd[q] = -1.0;

@@ -267,3 +267,5 @@ extern "C" int hq_test_panel(int m, int n, int pivoting, int smem_mode, int orde
   *barriers = emu::barriers;
   return ok ? err : -1;
 }
+
+extern "C" int hq_test_norm_cancelled(double nd, double thr) { return hq_norm_cancelled(nd, thr); }

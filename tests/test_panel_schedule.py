@@ -41,6 +41,7 @@ def panel(tmp_path_factory):
                               perm.ctypes.data, C.addressof(nbar))
         assert rc == 0
         return F, tau, perm, nbar.value
+    run.so = so
     return run
 
 
@@ -80,3 +81,27 @@ def test_any_order_with_recomputed_norms(panel, pivoting, smem_mode):
         v = np.concatenate([np.zeros(k), [1.0], F[k + 1:, k]])
         Q -= tau[k] * np.outer(v, v @ Q)
     assert np.linalg.norm(Q @ np.triu(F) - A[:, perm]) <= 1e-13 * np.linalg.norm(A)
+
+
+def test_a_norm_is_recomputed_only_when_it_has_cancelled(panel):
+    cancelled = panel.so.hq_test_norm_cancelled
+    cancelled.argtypes = [C.c_double] * 2
+    inf, nan = np.inf, np.nan
+    for nd, thr in ((0.5, 1.0), (1.0, 1.0), (0.0, 0.0), (-0.0, 1e-300), (-3.0, 1.0), (-inf, 1.0)):
+        assert cancelled(nd, thr)
+    for nd, thr in ((2.0, 1.0), (1e-300, 0.0), (inf, 1.0), (inf, inf), (nan, 1.0), (nan, nan),
+                    (-nan, 1.0), (-nan, nan), (-nan, -nan), (nan, inf)):
+        assert not cancelled(nd, thr)
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, 1e200])
+@pytest.mark.parametrize("smem_mode", [1, 0])
+def test_a_norm_that_is_not_finite_is_not_recomputed(panel, bad, smem_mode):
+    """Nor are the other columns': one grid barrier, for the initial norms."""
+    rng = np.random.default_rng(2)
+    m, n = 40, 24
+    A = np.asfortranarray(rng.standard_normal((m, n)))
+    A[7, 5] = bad
+    F, tau, perm, barriers = panel(A, 0, smem_mode=smem_mode)
+    assert barriers == 1 and sorted(perm) == list(range(n))
+    assert not np.all(np.isfinite(F))
