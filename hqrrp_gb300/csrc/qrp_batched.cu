@@ -142,13 +142,17 @@ __global__ void __launch_bounds__(NT, 512 / NT) qrp_batched_kernel(BatchArgs a) 
       item = (int)s_item[turn & 1][0];
       if (item < 0) break;
     }
-    const int T = teams ? T_all : 1, me = teams ? (int)rank : 0;
     const int m = a.m[item], n = a.n[item], lda = a.lda[item];
+    // The plan gives no matrix of more than TEAM_ROWS rows to a team; one that
+    // has them now is the first CTA's alone, the others go on to the next
+    // turn's barrier.
+    const bool alone = teams && m > TEAM_ROWS;
+    if (alone && rank != 0) continue;
+    const int T = teams && !alone ? T_all : 1, me = T > 1 ? (int)rank : 0;
     double* Ag = a.A[item];
     // A size the kernel cannot take (negative, lda < max(1, m), more than
     // max_n columns) is flagged and left untouched; an empty matrix is done.
-    // (The host gives no matrix of more than TEAM_ROWS rows to a team.)
-    const bool bad = m < 0 || n < 0 || n > a.max_n || lda < max(1, m) || (T > 1 && m > TEAM_ROWS);
+    const bool bad = m < 0 || n < 0 || n > a.max_n || lda < max(1, m);
     if (bad || m == 0 || n == 0) {
       if (tid == 0 && me == 0 && a.info) a.info[item] = bad ? HQ_ERR_BAD_SHAPE : 0;
       continue;

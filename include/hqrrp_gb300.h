@@ -200,8 +200,9 @@ int hqrrp_gb300_ozaki_dgemm(char transa, char transb, int m, int n, int k, doubl
  * (>= 0) or minus an error code.
  * run: all arrays on the device (d_A[i] column-major m[i] x n[i] with leading
  * dimension d_lda[i], d_jpvt[i] n[i] ints, d_tau[i] min(m,n) doubles, d_info
- * may be NULL); max_n bounds every n[i].  One persistent launch with a device
- * work queue; asynchronous on `stream`, allocates nothing and does not
+ * may be NULL); max_n bounds every n[i].  The sizes need not be the plan's:
+ * the schedule is the plan's then, and only the balance suffers.  One
+ * persistent launch with device work queues; asynchronous on `stream`, allocates nothing and does not
  * synchronise, so it can be captured in a CUDA graph.  Returns 0 or an error
  * code for the launch itself; d_info[i] != 0 flags a matrix it could not take. */
 size_t hqrrp_gb300_qrp_batched_workspace(int batch);

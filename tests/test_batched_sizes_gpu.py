@@ -1,0 +1,55 @@
+"""Batched QR: runs whose sizes are not the plan's."""
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-12
+
+
+def _team_counts(bq):
+    """How many of the schedule's first matrices go to teams, by CTAs per SM."""
+    import torch
+    return bq.work[:256].view(torch.int32)[9:16].cpu().tolist()
+
+
+def _factor(bq, shapes, seed):
+    import torch
+    As = [oracle.gaussian(m, n, seed + i) for i, (m, n) in enumerate(shapes)]
+    mats = [torch.from_numpy(np.ascontiguousarray(A.T)).cuda() for A in As]
+    bq.shapes = list(shapes)
+    sizes = np.array(shapes, np.int32)
+    bq.d_m.copy_(torch.from_numpy(sizes[:, 0].copy()))
+    bq.d_n.copy_(torch.from_numpy(sizes[:, 1].copy()))
+    bq.d_lda.copy_(torch.from_numpy(sizes[:, 0].copy()))
+    jp, tau, info = bq.run(mats)
+    torch.cuda.synchronize()
+    return As, [t.cpu().numpy().T for t in mats], jp, tau, info.cpu().numpy()
+
+
+def _check(oracle_lib, As, Fs, jps, taus, info):
+    assert not info.any(), [hex(i) for i in info]
+    for A, F, jp, tau in zip(As, Fs, jps, taus):
+        Ao, jo, to, _ = oracle_lib.dgeqp3(A)
+        k, n = min(A.shape), A.shape[1]
+        np.testing.assert_array_equal(jp.cpu().numpy()[:n], jo)
+        assert np.max(np.abs(tau.cpu().numpy()[:k] - to)) <= TOL
+        assert np.max(np.linalg.norm(F - Ao, axis=0) / np.linalg.norm(Ao, axis=0)) <= TOL
+
+
+@pytest.mark.parametrize("cfg", range(7))
+def test_sizes_that_are_not_the_plans(hq, oracle_lib, cfg):
+    """Planned for a team with up to 1024 rows, more than that when run; others
+    grow, shrink and vanish."""
+    plan = [(800, 300), (600, 200), (300, 200), (1500, 60), (20, 10), (40, 300)]
+    now = [(1300, 290), (1025, 120), (1024, 200), (700, 60), (200, 150), (1, 1)]
+    bq = hq.BatchedQRP(plan, autotune=False)
+    assert min(_team_counts(bq)) >= 2
+    # Outputs large enough for both.
+    import torch
+    bq.jpvt = [torch.zeros(300, dtype=torch.int32, device="cuda") for _ in plan]
+    bq.tau = [torch.zeros(300, dtype=torch.float64, device="cuda") for _ in plan]
+    bq.cfg = cfg
+    _check(oracle_lib, *_factor(bq, now, 70))
