@@ -1,4 +1,5 @@
-"""Batched QR: runs whose sizes are not the plan's."""
+"""Batched QR: which matrices the plan gives to teams of CTAs, at the limits of
+that rule, and runs whose sizes are not the plan's."""
 import numpy as np
 import pytest
 
@@ -37,6 +38,21 @@ def _check(oracle_lib, As, Fs, jps, taus, info):
         np.testing.assert_array_equal(jp.cpu().numpy()[:n], jo)
         assert np.max(np.abs(tau.cpu().numpy()[:k] - to)) <= TOL
         assert np.max(np.linalg.norm(F - Ao, axis=0) / np.linalg.norm(Ao, axis=0)) <= TOL
+
+
+# A team's smallest matrix, its most rows and one more, a matrix with fewer
+# columns than a team has warps; the counts hold for every number of CTAs per
+# SM here, each matrix being a large part of the batch.
+@pytest.mark.parametrize("shapes,count", [
+    ([(128, 128)], 1), ([(127, 129)], 0), ([(1024, 16)], 1), ([(1023, 16)], 0), ([(1024, 17)], 1),
+    ([(1025, 40)], 0), ([(700, 24), (128, 128)], 2), ([(16, 1024)], 1),
+    ([(1024, 60), (1025, 40), (128, 128)], 1)])
+@pytest.mark.parametrize("cfg", [3, 4, 5, 6])
+def test_team_limits(hq, oracle_lib, shapes, count, cfg):
+    bq = hq.BatchedQRP(shapes, autotune=False)
+    assert _team_counts(bq) == [count] * 7
+    bq.cfg = cfg
+    _check(oracle_lib, *_factor(bq, shapes, 40))
 
 
 @pytest.mark.parametrize("cfg", range(7))
