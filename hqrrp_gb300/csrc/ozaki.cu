@@ -546,13 +546,21 @@ __device__ __forceinline__ bool drain_levels(uint32_t tacc, int nacc, Handover h
 }
 
 // The running sums of a thread's 16 outputs.  Over any K: float-float pairs
-// (FloatSums).  Over K <= 256 (ExactSums): one 64-bit integer in units of 2^-40,
-// level 5's -- the accumulators of levels 0 to 4 are integers there, their
-// weighted sum stays below 2^63, and the shared accumulator of levels 5 and 6
-// is rounded to that unit.  That takes a few instructions an accumulator
-// instead of ten, makes the FP64 value on the integer pipe, which leaves
-// one FP64 addition an output instead of two, and errs less (1.9e-16 of the
-// product's norm against 5.9e-16, Gaussian operands, K = 64 to 256).
+// (FloatSums).  Over K <= 256 (ExactSums): integers in units of 2^-48, level
+// 6's -- the accumulators of levels 0 to 4 are integers in their own units, the
+// one that levels 5 and 6 share is a multiple of level 6's, and all of them
+// together stay below 2^71.  A 64-bit integer holds the sum down to 2^-40,
+// level 5's unit, and a byte the 8 bits below it, so nothing that the tensor
+// core hands over is dropped, however small the product is beside its row's and
+// column's scales; one rounding to FP64 is left.  That takes fewer instructions
+// an accumulator than a float-float addition, makes the FP64 value on the
+// integer pipe, which leaves one FP64 addition an output instead of two, and
+// errs no more: 1.8e-16 to 2.1e-16 of the product's norm against 6.0e-16 for
+// Gaussian operands of K = 64 to 256, and the same where the operands are graded
+// in opposite directions along K (K = 4 to 256), whose results are far below
+// their scales.  (Without the byte those erred up to 1.5 times as much; it takes
+// the 8192 x 8192 x 128 update from 0.398 to 0.420 ms -- 0.600 with
+// float-float sums and an MMA a level.)
 struct FloatSums {
   float hi[EPI_COLS], lo[EPI_COLS];
   __device__ __forceinline__ void clear() {
@@ -572,9 +580,12 @@ struct FloatSums {
 
 struct ExactSums {
   long long sum[EPI_COLS];
+  uint32_t rest[EPI_COLS / 4];  // a byte an output
   __device__ __forceinline__ void clear() {
 #pragma unroll
     for (int c = 0; c < EPI_COLS; ++c) sum[c] = 0;
+#pragma unroll
+    for (int c = 0; c < EPI_COLS / 4; ++c) rest[c] = 0u;
   }
   // q: a constant once unrolled.  Levels 0 and 1 only touch the upper word;
   // the others are wide multiply-adds, off the integer pipe.
@@ -582,7 +593,19 @@ struct ExactSums {
     const float unit = __uint_as_float((uint32_t)(127 + 8 * q) << 23);
 #pragma unroll
     for (int c = 0; c < EPI_COLS; ++c) {
-      const int i = __float2int_rn(v[c] * unit);
+      float t = v[c] * unit;
+      if (q == MAX_ACC - 1) {
+        // Rounded down; 256 times the rest is an integer below 256, and the
+        // lowest byte of that plus 2^23.
+        const float f = floorf(t);
+        const uint32_t r = __float_as_uint(fmaf(t - f, 256.f, 8388608.f));
+        rest[c / 4] = __byte_perm(rest[c / 4], r, c % 4 == 0   ? 0x3214
+                                                  : c % 4 == 1 ? 0x3240
+                                                  : c % 4 == 2 ? 0x3410
+                                                               : 0x4210);
+        t = f;
+      }
+      const int i = __float2int_rn(t);
       if (q < 2)
         sum[c] += (long long)((unsigned long long)(unsigned)(q == 0 ? i * 256 : i) << 32);
       else
@@ -592,10 +615,15 @@ struct ExactSums {
   // sign * sum * 2^(ek - 40), rounded to FP64 (half away from zero); results
   // below the FP64 normal range give 0.
   __device__ __forceinline__ double value(int c, int ek, unsigned neg) const {
-    const long long v = sum[c];
+    // The byte below is appended where the result is one word long with it, and
+    // rounded off where it is below a quarter of the result's last place.
+    const unsigned below = rest[c / 4] >> (8 * (c % 4)) & 0xFFu;
+    const bool fits = (unsigned)((int)(sum[c] >> 32) + 0x400000) < 0x800000u;  // |sum| < 2^54
+    const long long v = fits ? (long long)((unsigned long long)sum[c] << 8 | below)
+                             : sum[c] + (long long)(below >> 7);
     const unsigned long long u = (unsigned long long)(v < 0 ? -v : v);
     unsigned h = (unsigned)(u >> 32), l = (unsigned)u;
-    int e = ek + 1045;  // biased exponent - 1 of a leading bit 63
+    int e = ek + (fits ? 1037 : 1045);  // biased exponent - 1 of a leading bit 63
     const bool low = h == 0u;
     h = low ? l : h;
     l = low ? 0u : l;
