@@ -8,6 +8,7 @@
  * reflectors stay on the device, and the host waits once at the end.
  */
 #include <cuda_runtime_api.h>
+#include <math.h>
 #include <pthread.h>
 #include <stdarg.h>
 #include <stdio.h>
@@ -1571,6 +1572,17 @@ static double qr_cost(int m, int n) {
   return 2.0 * M * k * k - 2.0 * k * k * k / 3.0 + (double)m * n;
 }
 
+/* Microseconds that a matrix of this cost (k stages) takes one CTA of 256
+ * threads -- share: how many CTAs work on its SM -- or a team of four, two to an
+ * SM.  Fitted to batches of equal matrices from 64 x 64 to 1000 x 500; a stage's
+ * own time, then the FP64 work at an SM's 4 flops a clock (304 at once of 128 x
+ * 128, 300 x 300 and 1000 x 500, measured: single 1.73, 14.3 and 147 ms, teams
+ * 4.7, 25 and 185 in four rounds; the fit is within 15 % of these). */
+static double single_us(double cost, int k, double share) {
+  return 5.7 * k + 1.35 * share * cost / 7600.0;
+}
+static double team_us(double cost, int k) { return 6.8 * k + 1.62 * 0.5 * cost / 7600.0; }
+
 /* Time every launch shape on scratch matrices of the batch's sizes. */
 static int autotune_batched(hq_ws* w, int batch, const int* h_m, const int* h_n, int max_n,
                             void* d_work) {
@@ -1684,14 +1696,26 @@ HQ_API int hqrrp_gb300_qrp_batched_plan(int batch, const int* h_m, const int* h_
    * large enough (16384 entries) that a stage's FP64 work outweighs the team's
    * exchange. */
   int n_team[8] = {0};
+  double single_max = 0.0, single_sum = 0.0, mixed_max = 0.0, mixed_sum = 0.0;
   for (int i = 0; i < batch; ++i) {
-    const int id = ord[i].idx;
+    const int id = ord[i].idx, k = imin(h_m[id], h_n[id]);
     hord[i] = id;
     for (int c = 1; c < 8; ++c)
       if (n_team[c] == i && 4.0 * c * ord[i].cost * sms > total &&
           h_m[id] <= HQ_BATCHED_TEAM_ROWS && (double)h_m[id] * h_n[id] >= 16384.0)
         ++n_team[c];
+    /* What the batch takes with two CTAs an SM, without teams and with teams of
+     * four for the first n_team[2]. */
+    const double single = single_us(ord[i].cost, k, batch > sms ? 2.0 : 1.0);
+    const int team = n_team[2] == i + 1;
+    const double mixed = team ? team_us(ord[i].cost, k) : single;
+    single_sum += single;
+    mixed_sum += team ? 4.0 * mixed : mixed;
+    if (single > single_max) single_max = single;
+    if (mixed > mixed_max) mixed_max = mixed;
   }
+  const double single_us_all = fmax(single_max, single_sum / (2.0 * sms));
+  const double mixed_us_all = fmax(mixed_max, mixed_sum / (2.0 * sms));
   free(ord);
   hq_ws w;
   int rc = ws_begin(&w, (cudaStream_t)stream, 1);
@@ -1709,8 +1733,11 @@ HQ_API int hqrrp_gb300_qrp_batched_plan(int batch, const int* h_m, const int* h_
   }
   free(hord);
   if (rc) return -rc;
-  /* 256 threads, 32 KB staging, 2 CTAs per SM; teams of four where they have work. */
-  int cfg = n_team[2] > 0 ? 4 : 1;
+  /* 256 threads, 32 KB staging, 2 CTAs per SM; with teams of four where that is
+   * expected to end sooner: where a few matrices are long beside the rest of the
+   * batch.  (As many equal ones as CTAs, 304 of 128 x 128: 1.73 ms without teams,
+   * 4.7 with.) */
+  int cfg = mixed_us_all < single_us_all ? 4 : 1;
   if (autotune) {
     for (int i = 0; i < g_ntuned; ++i)
       if (g_tuned[i].batch == batch && g_tuned[i].max_n == max_n && g_tuned[i].cost == total)

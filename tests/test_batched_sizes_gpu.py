@@ -55,6 +55,16 @@ def test_team_limits(hq, oracle_lib, shapes, count, cfg):
     _check(oracle_lib, *_factor(bq, shapes, 40))
 
 
+# Teams of four (shape 4) by default only where a few matrices are long beside
+# the rest: alone, or before many small ones; not when as many equal matrices as
+# CTAs, or more, keep every CTA at work.
+@pytest.mark.parametrize("shapes,cfg", [
+    ([(128, 128)], 4), ([(128, 128)] * 304, 1), ([(128, 128)] * 1000, 1), ([(300, 300)] * 20, 4),
+    ([(300, 300)] * 304, 1), ([(1000, 500)] + [(40, 30)] * 500, 4), ([(60, 50)] * 10, 1)])
+def test_default_shape(hq, shapes, cfg):
+    assert hq.BatchedQRP(shapes, autotune=False).cfg == cfg
+
+
 @pytest.mark.parametrize("cfg", range(7))
 def test_sizes_that_are_not_the_plans(hq, oracle_lib, cfg):
     """Planned for a team with up to 1024 rows, more than that when run; others
