@@ -39,7 +39,8 @@ __device__ __forceinline__ double lanes_sum(const double (&d)[NY], int lane) {
 // y_c -= tau (v^T y_c) v over rows s..m-1 for NY columns y_c of one warp; the
 // new entries of row s go to rs[c].  CH > 0: CH steps of 32 rows cover them,
 // without a branch (so every load can be issued ahead), and the columns stay in
-// registers between the two uses; CH = 0: any number of rows, read twice.
+// registers between the two uses; CH = 0: any number of rows, read twice, eight
+// loads ahead (four or sixteen: 2 to 18 % slower batches).
 template <int NY, int CH>
 __device__ __forceinline__ void apply_warp(const double* __restrict__ v, double* const (&y)[NY],
                                            double tau, int s, int m, int lane, double* (&rs)[NY]) {
@@ -77,7 +78,7 @@ __device__ __forceinline__ void apply_warp(const double* __restrict__ v, double*
       }
     }
   } else {
-#pragma unroll 4
+#pragma unroll 8
     for (int i = s + lane; i < m; i += 32) {
       const double vi = v[i];
 #pragma unroll
@@ -87,7 +88,7 @@ __device__ __forceinline__ void apply_warp(const double* __restrict__ v, double*
     double w[NY];
 #pragma unroll
     for (int c = 0; c < NY; ++c) w[c] = __shfl_sync(0xffffffffu, t, 32 / NY * c);
-#pragma unroll 4
+#pragma unroll 8
     for (int i = s + lane; i < m; i += 32) {
       const double vi = v[i];
 #pragma unroll
@@ -108,12 +109,15 @@ struct Take {
 // Columns act[0..cnt) (local indices; colp gives a column's address) of a CTA
 // of NW warps: X[s:, k] -= tau v (v^T X[s:, k]), the new entries of row s to
 // row.  A warp takes four, two or one column together, as its registers hold
-// of this many rows (256, 512, 1024; longer columns are read twice).  More
-// together need fewer FP64 instructions -- with S steps of 32 rows 8 S + 7 for
-// four, 4 S + 6 for two, 2 S + 6 for one -- but spread over fewer quarters of
-// the SM, each of which issues one every 64 clocks: the choice is what the
-// busiest quarter issues.
-template <int NW, typename ColP>
+// of this many rows (256, 512, 1024).  More together need fewer FP64
+// instructions -- with S steps of 32 rows 8 S + 7 for four, 4 S + 6 for two, 2 S
+// + 6 for one -- but spread over fewer quarters of the SM, each of which issues
+// one every 64 clocks: the choice is what the busiest quarter issues.  Longer
+// columns are read twice, and one at a time: the second reading of one column a
+// warp still finds it in the L1 cache, of four it does not (400 matrices of 2000
+// x 64: 12.0 ms, with four a warp 16.6; 150 of 4000 x 40: 3.9 and 7.3).  LEAN:
+// few registers a thread, every column is read twice.
+template <int NW, bool LEAN = false, typename ColP>
 __device__ __forceinline__ void apply_columns(const double* v, double tau, int s, int m, int cnt,
                                               const int* act, double* row, ColP colp, int warp,
                                               int lane) {
@@ -139,14 +143,17 @@ __device__ __forceinline__ void apply_columns(const double* v, double tau, int s
       if (j < cnt) apply(single, j);
     }
   };
+  if constexpr (LEAN) {
+    apply_all(Take<1, 0>{}, Take<1, 0>{});
+    return;
+  }
 #define HQ_MANY(NY, CH) apply_all(Take<NY, CH>{}, Take<1, CH>{}); break;
   const int S = (m - s + 31) >> 5;
   const int t1 = ((cnt + 3) >> 2) * (2 * S + 6);
   const int t2 = S > 16 ? t1 : (((cnt >> 1) + (cnt & 1) + 3) >> 2) * (4 * S + 6);
   const int t4 = S > 8 ? t1 : (((cnt >> 2) + (cnt & 3) + 3) >> 2) * (8 * S + 7);
   if (S > 32) {
-    if (cnt >= 16) apply_all(Take<4, 0>{}, Take<1, 0>{});
-    else apply_all(Take<1, 0>{}, Take<1, 0>{});
+    apply_all(Take<1, 0>{}, Take<1, 0>{});
   } else if (t4 < t1 && t4 <= t2) {
     switch (S) {
       case 1: HQ_MANY(4, 1)
@@ -186,18 +193,17 @@ __device__ __forceinline__ void apply_columns(const double* v, double tau, int s
 #undef HQ_MANY
 }
 
-// Sum of squares of x over rows (s, m) by the ND threads t < ND of some warps:
-// each warp's part in every lane of it.
-template <int ND>
-__device__ __forceinline__ double tail_squares(const double* x, int s, int m, int t) {
+// Sum of squares of x over rows (s, m) by the threads t < nd of some warps: each
+// warp's part in every lane of it.
+__device__ __forceinline__ double tail_squares(const double* x, int s, int m, int t, int nd) {
   double sum = 0.0;
-  for (int i0 = s + 1 + t; i0 - t < m; i0 += 8 * ND) {
+  for (int i0 = s + 1 + t; i0 - t < m; i0 += 8 * nd) {
     double v[8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) v[k] = i0 + k * ND < m ? x[i0 + k * ND] : 0.0;
+    for (int k = 0; k < 8; ++k) v[k] = i0 + k * nd < m ? x[i0 + k * nd] : 0.0;
 #pragma unroll
     for (int k = 0; k < 8; ++k)
-      if (i0 - t + k * ND < m) sum = fma(v[k], v[k], sum);  // uniform
+      if (i0 - t + k * nd < m) sum = fma(v[k], v[k], sum);  // uniform
   }
   return hq_warp_sum(sum);
 }

@@ -1536,11 +1536,14 @@ typedef struct {
  * budget for a matrix (KB), CTAs per SM, team.  Small budgets: what shared
  * memory leaves of the 256 KB serves as L1 for the matrices worked on in
  * place, which are most of the work (4096 matrices of the benchmark, 256
- * threads, teams of two: 32 KB 106 ms, 64 KB 113, 96 KB 147). */
+ * threads, teams of two: 32 KB 106 ms, 64 KB 113, 96 KB 147).  From
+ * LONG_BATCHED_CFGS on: nothing staged and 1024 threads an SM, for long or narrow
+ * columns. */
 static const batched_cfg g_batched_cfgs[] = {
-    {128, 48, 4, 1}, {256, 32, 2, 1}, {512, 64, 1, 1}, {256, 32, 2, 2},
-    {256, 32, 2, 4}, {512, 64, 1, 2}, {256, 64, 2, 8},
+    {128, 48, 4, 1}, {256, 32, 2, 1}, {512, 64, 1, 1}, {256, 32, 2, 2}, {256, 32, 2, 4},
+    {512, 64, 1, 2}, {256, 64, 2, 8}, {256, 0, 4, 1},  {512, 0, 2, 1},
 };
+#define LONG_BATCHED_CFGS 7
 #define N_BATCHED_CFGS ((int)(sizeof g_batched_cfgs / sizeof g_batched_cfgs[0]))
 
 typedef struct {
@@ -1587,7 +1590,20 @@ static double team_us(double cost, int k) { return 6.8 * k + 1.62 * 0.5 * cost /
 static int autotune_batched(hq_ws* w, int batch, const int* h_m, const int* h_n, int max_n,
                             void* d_work) {
   size_t total = 0;
-  for (int i = 0; i < batch; ++i) total += (size_t)(h_m[i] > 0 ? h_m[i] : 1) * (h_n[i] > 0 ? h_n[i] : 1);
+  double cost = 0.0, cols = 0.0; /* cols: of the shorter side, by cost */
+  int rows = 0;
+  for (int i = 0; i < batch; ++i) {
+    const double c = qr_cost(h_m[i], h_n[i]);
+    total += (size_t)(h_m[i] > 0 ? h_m[i] : 1) * (h_n[i] > 0 ? h_n[i] : 1);
+    cost += c;
+    cols += c * imin(h_m[i], h_n[i]);
+    rows = imax(rows, h_m[i]);
+  }
+  /* The shapes for long or narrow columns where there are some (400 and 1200 equal
+   * matrices, the best shape without these and with them: 600 x 20 0.53 -> 0.37
+   * and 1.15 -> 0.88 ms, 600 x 48 2.18 -> 1.58 and 4.8 -> 4.2, 1000 x 40 2.4 -> 2.0
+   * and 5.5 -> 5.1 ms).  Others are spared the trials. */
+  const int use_long = rows > HQ_BATCHED_TEAM_ROWS || cols < 64.0 * cost;
   double* pool = ws_alloc(w, sizeof(double) * total);
   double** hA = malloc(sizeof(double*) * (size_t)batch);
   int** hJ = malloc(sizeof(int*) * (size_t)batch);
@@ -1624,7 +1640,7 @@ static int autotune_batched(hq_ws* w, int batch, const int* h_m, const int* h_n,
     cudaEvent_t e0, e1;
     ok = ok && cudaEventCreate(&e0) == 0 && cudaEventCreate(&e1) == 0;
     float best_ms = 1e30f;
-    for (int c = 0; ok && c < N_BATCHED_CFGS; ++c) {
+    for (int c = 0; ok && c < (use_long ? N_BATCHED_CFGS : LONG_BATCHED_CFGS); ++c) {
       const batched_cfg* k = &g_batched_cfgs[c];
       float ms = 0.f;
       int rc = hq_qrp_batched(w->st, &w->ds->dev, batch, dm, dn, (double* const*)dptr, dl,

@@ -91,8 +91,12 @@ __device__ __forceinline__ double cluster_ld(unsigned addr) {
   return v;
 }
 
-template <int NT>
-__global__ void __launch_bounds__(NT, 512 / NT) qrp_batched_kernel(BatchArgs a) {
+// LEAN: 1024 threads an SM and the registers that leaves each, for batches of
+// long or narrow columns, which wait for loads and stages more than for the FP64
+// pipe (batches of 1200, best launch shape without and with it: 600 x 20 1.15 ->
+// 0.88 ms, 1100 x 64 16.5 -> 13.0, 10000 x 30 61 -> 43).
+template <int NT, bool LEAN>
+__global__ void __launch_bounds__(NT, (LEAN ? 1024 : 512) / NT) qrp_batched_kernel(BatchArgs a) {
   extern __shared__ __align__(16) double smem[];
   constexpr int NW = NT / 32;
   // FP64 work that is one value per thread goes to four warps, one per quarter
@@ -100,7 +104,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) qrp_batched_kernel(BatchArgs a) 
   constexpr int ND = 128, NDW = ND / 32;
   __shared__ __align__(16) long long s_cand[2][T_MAX][2];  // the team's candidates, by stage parity
   __shared__ __align__(16) long long s_item[2][2];
-  __shared__ double s_red[NDW];
+  __shared__ double s_red[NW];
   __shared__ long long s_bk[NDW], s_at[NDW];
   __shared__ double s_tau, s_scale, s_beta;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -250,15 +254,17 @@ __global__ void __launch_bounds__(NT, 512 / NT) qrp_batched_kernel(BatchArgs a) 
             sv[i] = staged ? cluster_ld(r0 + 8u * (unsigned)i) : hq_ldcg(g + i);
           __syncthreads();
         }
-        if (tid < ND) {
-          const double t = tail_squares<ND>(v, s, m, tid);
+        // (All warps load a long column.)
+        const int nd = m > TEAM_ROWS ? NT : ND;
+        if (tid < nd) {
+          const double t = tail_squares(v, s, m, tid, nd);
           if (lane == 0) s_red[warp] = t;
         }
         __syncthreads();
         if (warp == 0) {
-          double q = s_red[lane & (NDW - 1)];
-#pragma unroll
-          for (int o = NDW / 2; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+          const int parts = nd / 32;  // a power of two
+          double q = s_red[lane & (parts - 1)];
+          for (int o = parts / 2; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
           if (lane == 0) {
             const HqReflector h = hq_make_reflector_sq(v[s], m - s > 1 ? q : 0.0);
             s_tau = h.tau;
@@ -286,7 +292,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) qrp_batched_kernel(BatchArgs a) 
       }
 
       // 3. X[s:, k] -= tau v (v^T X[s:, k]).
-      apply_columns<NW>(v, s_tau, s, m, cnt, sact, srs, colp, warp, lane);
+      apply_columns<NW, LEAN>(v, s_tau, s, m, cnt, sact, srs, colp, warp, lane);
       __syncthreads();
 
       // 4. LAWN 176 downdate of the squared norms, one thread per column; the
@@ -405,7 +411,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) qrp_batched_kernel(BatchArgs a) 
   }
 }
 
-template <int NT>
+template <int NT, bool LEAN = false>
 int launch_t(cudaStream_t st, const hq_device_info* dev, BatchArgs a, int ctas_per_sm,
              int team) {
   const size_t fixed = sizeof(double) * 4 * (size_t)a.max_n +
@@ -413,7 +419,7 @@ int launch_t(cudaStream_t st, const hq_device_info* dev, BatchArgs a, int ctas_p
   if (fixed > dev->smem_optin) return (int)cudaErrorInvalidValue;
   if ((size_t)a.stage_bytes > dev->smem_optin - fixed) a.stage_bytes = (int)(dev->smem_optin - fixed);
   const size_t smem = fixed + (size_t)a.stage_bytes;
-  auto kernel = qrp_batched_kernel<NT>;
+  auto kernel = qrp_batched_kernel<NT, LEAN>;
   cudaError_t e =
       cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
@@ -485,8 +491,12 @@ extern "C" int hq_qrp_batched(cudaStream_t stream, const hq_device_info* dev, in
   if (e != cudaSuccess) return (int)e;
   switch (threads) {
     case 128: return launch_t<128>(stream, dev, a, ctas_per_sm, team);
-    case 256: return launch_t<256>(stream, dev, a, ctas_per_sm, team);
-    case 512: return launch_t<512>(stream, dev, a, ctas_per_sm, team);
+    case 256:
+      return ctas_per_sm > 2 ? launch_t<256, true>(stream, dev, a, ctas_per_sm, team)
+                             : launch_t<256>(stream, dev, a, ctas_per_sm, team);
+    case 512:
+      return ctas_per_sm > 1 ? launch_t<512, true>(stream, dev, a, ctas_per_sm, team)
+                             : launch_t<512>(stream, dev, a, ctas_per_sm, team);
     default: return (int)cudaErrorInvalidValue;
   }
 }

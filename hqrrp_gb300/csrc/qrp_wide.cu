@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(WT, 1) wide_qrp_kernel(WdArgs a) {
       const double* x = colp(lq);
       const int wt = tid - 32;
       if (wt < ND) {
-        const double t = tail_squares<ND>(x, s, m, wt);
+        const double t = tail_squares(x, s, m, wt, ND);
         if (lane == 0) s_red[warp - 1] = t;
       }
       worker_barrier();

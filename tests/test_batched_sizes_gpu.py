@@ -65,7 +65,20 @@ def test_default_shape(hq, shapes, cfg):
     assert hq.BatchedQRP(shapes, autotune=False).cfg == cfg
 
 
-@pytest.mark.parametrize("cfg", range(7))
+# Columns on both sides of 1024 rows, where they no longer stay in registers,
+# and of the 32 rows that one step of a warp takes; narrow and wide ones.
+LONG = [(1024, 40), (1025, 40), (1055, 33), (1056, 1), (1057, 2), (2049, 20), (5000, 3), (1030, 129),
+        (31, 7), (32, 33), (33, 200), (1, 5)]
+
+
+@pytest.mark.parametrize("cfg", range(9))
+def test_long_columns(hq, oracle_lib, cfg):
+    bq = hq.BatchedQRP(LONG, autotune=False)
+    bq.cfg = cfg
+    _check(oracle_lib, *_factor(bq, LONG, 100))
+
+
+@pytest.mark.parametrize("cfg", range(9))
 def test_sizes_that_are_not_the_plans(hq, oracle_lib, cfg):
     """Planned for a team with up to 1024 rows, more than that when run; others
     grow, shrink and vanish."""
