@@ -62,6 +62,8 @@ namespace {
 constexpr int MAX_G = 160;          // CTAs (one per SM); partial loads per lane <= 5
 constexpr int CB = (MAX_G + 31) / 32;
 constexpr int QB = 8;               // columns reduced per warp per batch of loads
+constexpr int APART_COST = 16;      // FP64 instructions' time, 64 clocks each
+constexpr int APART_ROWS = 192;
 
 struct PnArgs {
   int mp, nc, ns, pivoting;
@@ -380,6 +382,33 @@ __global__ void __launch_bounds__(NT, 1) panel_qrp_kernel(PnArgs a) {
     return (bk == 0x7fffffff || bd < 0) ? k0 : bk;
   };
 
+  // The pivot among the warps' picks in s_bd, s_bk, or k0.
+  auto next_pivot = [&](int k0) {
+    if (!a.pivoting) return k0;
+    long long bd = s_bd[0];
+    int bk = s_bk[0];
+    for (int w = 1; w < NWARP; ++w) pick(s_bd[w], s_bk[w], bd, bk);
+    return bk != 0x7fffffff && bd >= 0 ? bk : k0;
+  };
+  // Whether update and dot products of na columns are made one after the other.
+  // Both are bound by the FP64 pipe when a slab is long, and the pass that does
+  // both deals columns out by a power of two of lanes, so some warps may have
+  // none (40 columns of 4 lanes: five warps of eight); the update alone takes any
+  // number of lanes.  Compared: the FP64 instructions that the busiest quarter of
+  // the SM issues, and APART_COST for the barrier and the second reading.  (One
+  // pass always -> this, us: 50000 x 80 1498 -> 1204, 100000 x 40 753 -> 610,
+  // 200000 x 20 403 -> 331.  In shorter slabs the comparison costs a stage up to
+  // 5 % and changes little; out of shared memory the second reading costs more.)
+  const bool long_slab = a.smem_mode && a.rloc_max > APART_ROWS;
+  auto apart = [&](int na) {
+    const int g = lanes_for(na);
+    const int warps = ((na * g > NT ? NT : na * g) + 127) >> 7;  // of a quarter
+    const int both = (a.rloc_max * warps + g - 1) / g;
+    const int groups = na < NT ? NT / na : 1;
+    const int update = (a.rloc_max * (NT >> 7) + groups - 1) / groups;
+    return both > update + APART_COST;
+  };
+
   // One thread: columns s and kp change places (labels, copied norms; se[s]
   // takes the pivot's own value, which bounds its stage sums -- position s's
   // norms are not read again otherwise).
@@ -470,10 +499,10 @@ __global__ void __launch_bounds__(NT, 1) panel_qrp_kernel(PnArgs a) {
     if (lane == 0) { s_bd[warp] = bd; s_bk[warp] = bk; }
     any = __syncthreads_or(any);
 
-    if (any || s + 1 == a.ns) {
-      // 3a. The last stage, or norms to be recomputed: update the slab,
-      //     X[i, k] -= v_i w_k for rows > s; the owner of row s stores its new
-      //     entries.
+    if (any || s + 1 == a.ns || (long_slab && apart(nc - s - 1))) {
+      // 3a. The last stage, norms to be recomputed, or a long slab: update the
+      //     slab, X[i, k] -= v_i w_k for rows > s; the owner of row s stores its
+      //     new entries.
       const int nt = nc - s - 1;
       if (nt >= NT) {
         for (int q = tid; q < nt; q += NT) {
@@ -491,6 +520,10 @@ __global__ void __launch_bounds__(NT, 1) panel_qrp_kernel(PnArgs a) {
       }
       __syncthreads();
       if (s + 1 == a.ns) break;
+      if (!any) {
+        begin_stage(s + 1, next_pivot(s + 1));
+        continue;
+      }
       slab_dots(-1, s, s, true, part_w(epoch + 1));
       ++epoch;
       if (!hq_grid_barrier(a.bar, a.err, epoch, a.spin_limit, &s_flag)) return;
@@ -509,13 +542,7 @@ __global__ void __launch_bounds__(NT, 1) panel_qrp_kernel(PnArgs a) {
     }
 
     // 3b. The next pivot's column, and its place.
-    int kp = s + 1;
-    if (a.pivoting) {
-      bd = s_bd[0];
-      bk = s_bk[0];
-      for (int w = 1; w < NWARP; ++w) pick(s_bd[w], s_bk[w], bd, bk);
-      if (bk != 0x7fffffff && bd >= 0) kp = bk;
-    }
+    const int kp = next_pivot(s + 1);
     // What positions s + 1 and kp hold before they change places: one thread
     // rewrites the labels during the pass below, which takes these two
     // positions from here.

@@ -46,7 +46,8 @@ def panel(tmp_path_factory):
 
 
 @pytest.mark.parametrize("smem_mode", [1, 0])
-@pytest.mark.parametrize("m,n", [(40, 24), (30, 40), (70, 128), (20, 130), (9, 33)])
+@pytest.mark.parametrize("m,n", [(40, 24), (30, 40), (70, 128), (20, 130), (9, 33), (200, 40),
+                                 (300, 140), (193, 60)])
 def test_any_order_of_the_warps(panel, m, n, smem_mode):
     import scipy.linalg as sl
     rng = np.random.default_rng(m + n)
