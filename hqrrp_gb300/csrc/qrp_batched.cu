@@ -43,6 +43,7 @@ namespace {
 
 constexpr int T_MAX = 8;        // CTAs per cluster (the portable limit)
 constexpr int TEAM_ROWS = HQ_BATCHED_TEAM_ROWS;  // rows of a matrix a team takes
+constexpr unsigned LAYER_NS = 4000;  // more than what CTAs of one layer start apart
 
 struct BatchArgs {
   int batch;
@@ -120,6 +121,17 @@ __global__ void __launch_bounds__(NT, (LEAN ? 1024 : 512) / NT) qrp_batched_kern
 
   // Every CTA of the cluster has started before its shared memory is written.
   if (T_all > 1) cluster_barrier();
+  // CTAs that share an SM take their first matrix one after the other, a layer
+  // of the whole GPU at a time: else the two largest, the next in the queue, often
+  // meet on one SM and take twice as long as they need (1024 matrices of up to
+  // 1024 x 512, two CTAs an SM, single / teams of two / of four: 115 / 58 / 31.4
+  // ms, so 71 / 42 / 28.5).  The warp's slot on the SM tells the layer; should it
+  // not, only the balance suffers.
+  if (tid == 0) {
+    unsigned slot;
+    asm volatile("mov.u32 %0, %%warpid;" : "=r"(slot));
+    __nanosleep(slot / NW * LAYER_NS);
+  }
   bool teams = T_all > 1;
   for (int turn = 0;; ++turn) {
     // The next matrix: of the teams' queue while it lasts, then of the CTAs'.
