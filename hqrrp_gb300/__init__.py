@@ -207,7 +207,7 @@ def gram_panel_counts():
 
 
 def pool_alloc_count():
-    """Device allocations the library has made from its memory pools."""
+    """Device buffers the library has drawn from its memory pools."""
     return int(load().hqrrp_gb300_pool_alloc_count())
 
 

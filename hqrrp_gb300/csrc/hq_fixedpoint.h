@@ -3,10 +3,11 @@
  * The pivoted panel kernel sums, per column and stage, one FP64 partial dot
  * product from every CTA.  Each partial t becomes the integer V = t / 2^ue
  * (truncated), split into three 48-bit limbs that are added to three signed
- * 64-bit words; the 16 spare bits of each word absorb the carries of up to
- * 2^15 addends.  Integer addition is associative, so the words end up the
- * same whatever order the addends arrive in, and the sum is exact up to the
- * truncation of each addend below 2^ue.
+ * 64-bit words.  The spare bits above a limb absorb the carries: up to 2^15
+ * addends of a whole word, 127 where its upper byte counts them, as the panel
+ * kernel's do (80 CTAs at most add to one of its words).  Integer addition is
+ * associative, so the words end up the same whatever order the addends arrive
+ * in, and the sum is exact up to the truncation of each addend below 2^ue.
  *
  * ue comes from a bound B on the sum's magnitude (for dot products, the two
  * columns' norms: Cauchy-Schwarz bounds every CTA's partial and their sum)

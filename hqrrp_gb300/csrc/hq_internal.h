@@ -199,8 +199,8 @@ int hq_ozk_gemm_c64(cudaStream_t stream, const hq_device_info* dev, int M, int N
                     const void* Atiles, const int* ea, const double* Y, long long yld,
                     const int* raw, double sign, double* C, long long crs, long long ccs,
                     double* ws, size_t ws_elems, int* err, unsigned spin_limit);
-/* K <= 256: persistent kernel with double-buffered TMEM; the N side must be
- * split with side 2 (32-row tiles).  Mode 1 with colexp: colexp[c] (zeroed
+/* K <= 256: persistent kernel whose accumulators change hands in two groups;
+ * the N side must be split with side 2 (tiles of 80 rows).  Mode 1 with colexp: colexp[c] (zeroed
  * before) receives the largest exponent field of the new C(r, c) over rows
  * r >= row_lo. */
 int hq_ozk_short_ok(int K);

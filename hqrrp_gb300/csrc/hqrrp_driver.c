@@ -533,7 +533,6 @@ static int ws_setup(hq_ws* w, int m, int n, int nb, int pp, int pw) {
   return HQ_OK;
 }
 
-/* Read the device error word; 0 if clean. */
 /* The call's outcome from its error word, read back after a synchronisation. */
 static int ws_result(hq_ws* w, int herr) {
   prof_finish(w);
@@ -545,6 +544,7 @@ static int ws_result(hq_ws* w, int herr) {
   return HQ_OK;
 }
 
+/* Read the device error word; 0 if clean. */
 static int ws_check(hq_ws* w) {
   int herr = 0;
   CK(cudaMemcpyAsync(&herr, w->err, sizeof(int), cudaMemcpyDeviceToHost, w->st));
@@ -775,7 +775,7 @@ static int block_reflector(hq_ws* w, int mp, int b, const double* tau, double* C
   } else {
     DGRAM(b, mp);
   }
-  /* T (one SM, a sequential recurrence) on the side stream, overlapped with
+  /* T (a CTA for each row's recurrence) on the side stream, overlapped with
    * W1 = U^T C, which does not need it; st waits for T before W2. */
   int rs = side_stream(w);
   if (rs) return rs;
@@ -1536,7 +1536,7 @@ typedef struct {
  * budget for a matrix (KB), CTAs per SM, team.  Small budgets: what shared
  * memory leaves of the 256 KB serves as L1 for the matrices worked on in
  * place, which are most of the work (4096 matrices of the benchmark, 256
- * threads, teams of two: 32 KB 106 ms, 64 KB 113, 96 KB 147).  From
+ * threads, teams of two: 32 KB 95 ms, 64 KB 98, 96 KB 123).  From
  * LONG_BATCHED_CFGS on: nothing staged and 1024 threads an SM, for long or narrow
  * columns. */
 static const batched_cfg g_batched_cfgs[] = {
@@ -1707,8 +1707,9 @@ HQ_API int hqrrp_gb300_qrp_batched_plan(int batch, const int* h_m, const int* h_
   qsort(ord, (size_t)batch, sizeof(cost_idx), cost_desc);
   /* The teams' share, by CTAs per SM (a CTA has that part of its SM's FP64
    * rate): the largest matrices, as long as a single CTA would take over a
-   * quarter of what the whole batch takes on all SMs (batches of 1024 and 4096
-   * from all to a quarter: 35 -> 30 and 126 -> 111 ms), and the matrix is
+   * quarter of what the whole batch takes on all SMs (the benchmark's batches of
+   * 1024 and 4096 with all of it, a half, a quarter: 31.0, 29.5, 28.9 ms and 94.1,
+   * 94.6, 95.2), and the matrix is
    * large enough (16384 entries) that a stage's FP64 work outweighs the team's
    * exchange. */
   int n_team[8] = {0};

@@ -31,8 +31,8 @@
 // The launch shape -- threads per CTA, the staging budget, T -- is chosen by
 // the host autotuner (hqrrp_driver.c) per batch signature.  Measured on GB300
 // against one CTA per matrix, swapped columns and a column per warp: 1024
-// matrices of the benchmark's sizes 90 -> 29 ms (FP64 alone: 16), 4096 of them
-// 139 -> 107 (63).
+// matrices of the benchmark's sizes 90 -> 28.5 ms (FP64 alone: 16), 4096 of them
+// 139 -> 95 (63).
 //
 // All columns are free (LAPACK jpvt = 0 input); on return jpvt[k] is the
 // 1-based original index of column k, tau[0..min(m,n)) the reflector scalars,

@@ -264,10 +264,10 @@ unsigned long long hqrrp_gb300_launch_count(void);
 
 /* Number of device buffers this library has drawn from its memory pools
  * in this process (every entry point except hqrrp_gb300_qrp_noalloc draws its
- * workspace from a pool; small buffers share one allocation).  Setting HQRRP_GB300_FAIL_ALLOC=k in the
- * environment makes the k-th buffer of every later call fail as if the
- * device were out of memory (return code 4, dgeqp4 info 1004): host-side
- * fault injection for testing callers' error paths. */
+ * workspace from a pool; small buffers share one allocation).  Setting
+ * HQRRP_GB300_FAIL_ALLOC=k in the environment makes the k-th buffer of every
+ * later call fail as if the device were out of memory (return code 4, dgeqp4
+ * info 1004): host-side fault injection for testing callers' error paths. */
 unsigned long long hqrrp_gb300_pool_alloc_count(void);
 
 /* Mixed precision's panels: of the last call that factored panels in mixed
