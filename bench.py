@@ -48,11 +48,12 @@ sys.path.insert(0, ROOT)
 
 METRIC = "dgeqp4 TFLOP/s at n=16384, mixed vs plain FP64 at equal residual; bwd ms"
 # DRAM bytes per algorithmic flop of the dominant kernels, from ncu captures at
-# m = n = 6144: the split-BF16 products -- W1 = U'^T C reading C as FP64
-# (302.1 MB per 2.43e11 BF16 flops) and C -= U'W2 (556.1 MB per 2.649e11) -- and
-# the FP64 update GEMMs of the plain path (W1, C -= U W2).
-TENSOR_BYTES_PER_FLOP = (302.1e6 + 556.1e6) / (2.43e11 + 2.649e11)
-FP64_UPDATE_BYTES_PER_FLOP = (314.4e6 + 546.3e6) / (2 * 9.462e9)
+# m = n = 6144 (profiles/split_products.md, profiles/dgemm_tile.md): the
+# split-BF16 products -- W1 = U'^T C reading C as FP64 (273.0 MB per 2.325e11
+# BF16 flops) and C -= U'W2 (554.8 MB per 2.649e11) -- and the FP64 update GEMMs
+# of the plain path (W1 306.8 MB, C -= U W2 547.0 MB, 9.462e9 flops each).
+TENSOR_BYTES_PER_FLOP = (273.0e6 + 554.8e6) / (2.325e11 + 2.649e11)
+FP64_UPDATE_BYTES_PER_FLOP = (306.8e6 + 547.0e6) / (2 * 9.462e9)
 
 
 def flops_qr(m, n):
